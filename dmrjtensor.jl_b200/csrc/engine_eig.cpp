@@ -24,11 +24,15 @@ void run_trid_eigvals(dmrg_ctx* c, double* base, int64_t nbase, const std::vecto
                       int slot) {
   check_trid(t, nbase, false);
   std::vector<TridTask> small, mid;
-  int ns = 0, nm = 0;
+  int ns = 0;
+  int64_t sum = 0;
   for (const TridTask& x : t) {
     if (x.n <= SYEVT_NMAX) { small.push_back(x); ns = std::max(ns, x.n); }
-    else { mid.push_back(x); nm = std::max(nm, x.n); }
+    else { mid.push_back(x); sum += x.n; }
   }
+  // the largest first: not all clusters of a long list are resident at once
+  std::stable_sort(mid.begin(), mid.end(),
+                   [](const TridTask& a, const TridTask& b) { return a.n > b.n; });
   if (small.empty() && mid.empty()) return;
   Upload u;
   const size_t o1 = u.put(small), o2 = u.put(mid);
@@ -37,8 +41,8 @@ void run_trid_eigvals(dmrg_ctx* c, double* base, int64_t nbase, const std::vecto
     launch_trid_eigvals(c->stream, base, reinterpret_cast<const TridTask*>(db + o1),
                         int(small.size()), ns);
   if (!mid.empty())
-    launch_trid_mid_eigvals(c->stream, base, reinterpret_cast<const TridTask*>(db + o2),
-                            int(mid.size()), nm);
+    launch_trid_cluster(c->stream, base, reinterpret_cast<const TridTask*>(db + o2),
+                        int(mid.size()), mid[0].n, sum);
   cuda_check(cudaGetLastError(), "tridiagonal eigenvalues");
 }
 

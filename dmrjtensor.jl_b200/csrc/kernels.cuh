@@ -67,7 +67,7 @@ struct EigTask {
 };
 
 // Tridiagonal eigensolver for density-matrix blocks with n <= SYEVT_NMAX (syevt.cu, shared
-// memory) and SYEVT_NMAX < n <= SYEVT_MID_NMAX (syevt_mid.cu, global memory + shared memory).
+// memory) and SYEVT_NMAX < n <= SYEVT_MID_NMAX (syevt_cluster.cu and syevt_mid.cu).
 constexpr int SYEVT_NMAX = 112;
 constexpr int SYEVT_MID_NMAX = 512;
 struct TridTask {
@@ -87,8 +87,10 @@ int64_t syevt_mid_workspace(int n, int k);
 // Largest kept count whose Gram matrix the mid-size vector kernel holds in shared memory for
 // blocks up to max_n (tasks above it take the global-memory path; launch them separately).
 int syevt_mid_gram_limit(int max_n);
-void launch_trid_mid_eigvals(cudaStream_t s, double* base, const TridTask* tasks, int ntasks,
-                             int max_n);
+// Tridiagonalisation by thread-block clusters and all eigenvalues (syevt_cluster.cu); sum_n: the
+// blocks' sizes added up.
+void launch_trid_cluster(cudaStream_t s, double* base, const TridTask* tasks, int ntasks,
+                         int max_n, int64_t sum_n);
 // xws: workspace base of the tasks' x_off
 void launch_trid_mid_vectors(cudaStream_t s, double* base, const TridTask* tasks, int ntasks,
                              int max_n, int max_k, double* xws);

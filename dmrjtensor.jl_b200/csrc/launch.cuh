@@ -44,4 +44,29 @@ inline void launch_k(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, c
   (void)cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 
+// The same with thread-block clusters of c CTAs (grid: a multiple of c). Above 8 CTAs the size is
+// not portable and has to be allowed first, once per kernel and device.
+inline void allow_wide_clusters(const void* func) {
+  (void)cudaFuncSetAttribute(func, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+}
+template <typename... P, typename... A>
+inline void launch_cluster_k(void (*kernel)(P...), int c, dim3 grid, dim3 block, size_t smem,
+                             cudaStream_t s, A&&... args) {
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = unsigned(c);
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  (void)cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
+
 }  // namespace dmrg

@@ -16,63 +16,55 @@ __device__ __forceinline__ double wsum(double v) {
   return v;
 }
 
-// Scales a pair by the power of two that brings the larger magnitude into [1, 2): exact, keeps
-// the signs, and needs only exponent-field arithmetic.
-__device__ __forceinline__ void rescale_pair(double& D, double& Dm1) {
-  const double mx = fmax(fabs(D), fabs(Dm1));
-  const int fld = (__double2hiint(mx) >> 20) & 0x7ff;
-  if (fld != 0 && fld != 0x7ff) {
-    const int ex = min(fld - 1023, 1022);
-    const double sc = __hiloint2double((1023 - ex) << 20, 0);
-    D *= sc;
-    Dm1 *= sc;
-  }
-}
-
 // Number of eigenvalues of T(d,e) strictly below x: sign changes of the leading minors
 // D_j = (d_j - x) D_{j-1} - e_{j-1}^2 D_{j-2}. The carried pair is (D_{j-1}, t_j) with
 // t_j = -e_{j-1}^2 D_{j-2}: each step is one FMA for D_j and one product t_{j+1} from D_{j-1}, two
-// independent operations, so only the FMA is on the dependent chain. Groups of 8 steps load
-// first, count signs after the group (an exact zero minor counts with the sign opposite to its
-// predecessor), then rescale the pair by a power of two.
+// independent operations, so only the FMA is on the dependent chain. Signs are counted on the high
+// words (an isolated exact zero gives the same count with either sign). After every 8 steps the
+// pair is rescaled by the power of two that brought its larger magnitude after the fourth of them
+// into [1, 2): the factor is ready before the chain needs it, and 12 steps stay far from
+// overflow and underflow. With the small blocks' kernel (85, 70 and 40 rows in one launch) the
+// lagged rescaling and the bit counts took 108 to 100 us.
 __device__ int sturm_below(const double* __restrict__ d, const double* __restrict__ e2, int n,
                            double x) {
   double D = d[0] - x;
   double t = -e2[0];                      // t_1 = -e_0^2 D_{-1}, D_{-1} = 1
-  bool neg = D < 0.0;
-  int c = neg ? 1 : 0;
+  int hp = __double2hiint(D);
+  unsigned c = unsigned(hp) >> 31;
   int j = 1;
   for (; j + 8 <= n; j += 8) {
-    double dx[8], ee[8], Ds[8];
+    double dx[8], ee[8];
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
       dx[q] = d[j + q] - x;
-      ee[q] = e2[j + q];                  // e2[n-1] = 0: the last product is unused
+      ee[q] = e2[j + q];
     }
+    double sc = 1.0;
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
       const double Dn = fma(dx[q], D, t);
       t = -ee[q] * D;
       D = Dn;
-      Ds[q] = Dn;
+      const int h = __double2hiint(Dn);
+      c += unsigned(h ^ hp) >> 31;
+      hp = h;
+      if (q == 3) {
+        const int fld = max(h & 0x7fffffff, __double2hiint(t) & 0x7fffffff) >> 20;
+        if (fld != 0 && fld != 0x7ff) sc = __hiloint2double((1023 - min(fld - 1023, 1022)) << 20, 0);
+      }
     }
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const bool ng = (Ds[q] == 0.0) ? !neg : (Ds[q] < 0.0);
-      c += (ng != neg) ? 1 : 0;
-      neg = ng;
-    }
-    rescale_pair(D, t);
+    D *= sc;
+    t *= sc;
   }
   for (; j < n; ++j) {
     const double Dn = fma(d[j] - x, D, t);
     t = -e2[j] * D;
     D = Dn;
-    const bool ng = (Dn == 0.0) ? !neg : (Dn < 0.0);
-    c += (ng != neg) ? 1 : 0;
-    neg = ng;
+    const int h = __double2hiint(Dn);
+    c += unsigned(h ^ hp) >> 31;
+    hp = h;
   }
-  return c;
+  return int(c);
 }
 
 // pseudo-random start vector entry (fixed: results are reproducible)
@@ -103,7 +95,10 @@ struct LUSlot {
   int stride;
 };
 
-// One thread: z <- (T - lam I)^{-1} z three times, z = column col of the row-major Z (leading
+// One thread: z <- (T - lam I)^{-1} z twice (with lam good to the last bits the first solve leaves
+// other eigenvectors at ~1e-16 ||T|| / gap and the second squares that; a third only turns the
+// vectors of equal eigenvalues towards each other: the worst residual of degenerate test blocks
+// fell from 5e-13 to 3e-14 without it), z = column col of the row-major Z (leading
 // dimension ldz). The solves run in groups of 8 steps whose loads are issued first, so that only
 // the arithmetic recurrence is on the dependent chain.
 __device__ void inverse_iteration(const double* __restrict__ d, const double* __restrict__ e, int n,
@@ -133,7 +128,7 @@ __device__ void inverse_iteration(const double* __restrict__ d, const double* __
   f.u0[(n - 1) * S] = 1.0 / ((dk == 0.0) ? pert : dk);
   f.u1[(n - 1) * S] = 0.0; f.u2[(n - 1) * S] = 0.0; f.piv[(n - 1) * S] = 0;
   double* z = Z + col;                        // z[r] at z[r * ldz]
-  for (int it = 0; it < 3; ++it) {
+  for (int it = 0; it < 2; ++it) {
     // solve P L y = z; z[k] is carried in a register. Loads of a group precede its stores, and
     // every store goes below the indices still to be loaded.
     double zk = z[0];

@@ -1,24 +1,12 @@
-// syevt_mid.cu -- density-matrix eigensolver for mid-size blocks, SYEVT_NMAX < n <= SYEVT_MID_NMAX:
-// the method of syevt.cu (Householder tridiagonalisation, multisection, inverse iteration,
-// Cholesky QR, blocked back-transformation), one CTA of 512 threads per block, for matrices that
-// do not fit in shared memory.
-//
-// Launch 1 (k_trid_mid_vals): the Householder steps run on the matrix in place in global memory
-// (L2-resident: a 512 x 512 block is 2 MB) until the trailing block's lower triangle fits in
-// shared memory in packed form (m <= mp, about 230 beside the vectors); it is then copied there
-// and the remaining steps run on the copy, which is written back at the end (its strictly lower
-// part holds the last reflectors). Global steps: the product p = tau B v by columns (B is
-// symmetric: p_j = tau B(:,j).v, one warp per column, four columns in flight), one block barrier,
-// then the rank-2 update B -= v w^T + w v^T by the other warps while warp 0 updates the next pivot
-// column first and builds the next reflector from it. Packed steps: the same with p by row pairs
-// (the stored part of row a along the diagonal direction and of column a below it).
-// Eigenvalues by trisection as in syevt.cu, in rounds of 256 eigenvalues.
-// Launch 2 (k_trid_mid_vectors): inverse iteration (one thread per kept vector, LU factors in a
+// syevt_mid.cu -- eigenvectors of mid-size density-matrix blocks, SYEVT_NMAX < n <= SYEVT_MID_NMAX
+// (their tridiagonal matrices and eigenvalues come from syevt_cluster.cu), one CTA of 512 threads
+// per block.
+// Launch 1 (k_trid_mid_vectors): inverse iteration (one thread per kept vector, LU factors in a
 // global workspace interleaved by thread so that every factor access of a warp is one line),
 // Cholesky QR (a second pass unless the Gram matrix is within 1e-3/k of the identity; classical
 // Gram-Schmidt with restarts if a pivot shows nearly dependent vectors); the vectors Z of the
 // tridiagonal matrix stay in the workspace.
-// Launch 3 (k_trid_mid_backtransform): U = H_0 ... H_{n-3} Z in blocks of 8 reflectors (compact
+// Launch 2 (k_trid_mid_backtransform): U = H_0 ... H_{n-3} Z in blocks of 8 reflectors (compact
 // WY), one CTA per slice of 32 kept vectors with its slice of Z in shared memory, the reflectors
 // read from the matrix in global memory (every slice is independent of the others).
 #include "kernels.cuh"
@@ -31,407 +19,7 @@ namespace {
 constexpr int MT = 512;             // threads per CTA
 constexpr int NW = MT / 32;         // warps
 constexpr int MID_BT_NB = 8;        // reflectors per back-transformation block
-// columns per warp and pass in the product p = tau B v and in the rank-2 update (fewer for the
-// 16-row variant, whose register budget under 512 threads is the same)
 constexpr size_t MID_SMEM_LIMIT = 227 * 1024 - 2048;
-
-// Householder reflector of x = col[0..m) (one warp): H x = beta e_1 with v[0] = 1,
-// H = I - tau v v^T. Writes v to vout and v[1..m) into col[1..m); returns beta and tau.
-__device__ void house_warp(double* __restrict__ col, int m, double* __restrict__ vout,
-                           double& beta_o, double& tau_o, int lane) {
-  double part = 0.0;
-  for (int i = 1 + lane; i < m; i += 32) part += col[i] * col[i];
-  const double xn2 = wsum(part);
-  const double alpha = col[0];
-  double t, sc, beta;
-  if (xn2 == 0.0) {
-    t = 0.0; sc = 0.0; beta = alpha;
-  } else {
-    beta = -copysign(sqrt(alpha * alpha + xn2), alpha);
-    t = (beta - alpha) / beta;
-    sc = 1.0 / (alpha - beta);
-  }
-  for (int i = lane; i < m; i += 32) {
-    const double vi = (i == 0) ? 1.0 : col[i] * sc;
-    vout[i] = vi;
-    if (i > 0) col[i] = vi;
-  }
-  beta_o = beta;
-  tau_o = t;
-}
-
-// Packed lower-triangular storage of the trailing block once it fits in shared memory: column j
-// (0-based, of the block of size m0 copied at the switch) holds rows j..m0-1 from offset pk(j).
-__device__ __forceinline__ int pk(int j, int m0) { return j * m0 - (j * (j - 1)) / 2; }
-
-// RM = register rows per lane: n <= 32 RM.
-template <int RM>
-__global__ void __launch_bounds__(MT, 1)
-k_trid_mid_vals(double* __restrict__ base, const TridTask* __restrict__ tasks, int mp) {
-  grid_entry();
-  constexpr int CW = RM >= 16 ? 2 : 4;
-  constexpr int CU = RM >= 16 ? 1 : 2;
-  const TridTask tk = tasks[blockIdx.x];
-  const int n = tk.n;
-  if (n < 3 || n > 32 * RM) return;
-  extern __shared__ double sm[];
-  double* vb = sm;                         // 2 x n: reflector of this step / of the next
-  double* p = vb + 2 * n;                  // n
-  double* d = p + n;                       // n
-  double* e = d + n;                       // n
-  double* e2 = e + n;                      // n
-  double* tau = e2 + n;                    // n
-  double* S = tau + n;                     // packed trailing block, mp (mp + 1) / 2
-  __shared__ double kw[NW];
-  __shared__ double s_lo, s_hi;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  double* Ag = base + tk.a_off;
-  double* B = Ag + n + 1;                  // trailing block of step 0, A[1:, 1:]
-  const int ld = n;
-  if (warp == 0) {
-    double be, ta;
-    house_warp(Ag + 1, n - 1, vb, be, ta, lane);
-    if (lane == 0) { d[0] = Ag[0]; e[0] = be; tau[0] = ta; }
-  }
-  __syncthreads();
-  // steps on the matrix in global memory while the trailing block is larger than mp
-  int k = 0;
-  for (; k + 2 < n && n - k - 1 > mp; ++k) {
-    const int m = n - k - 1;
-    const double* v = vb + (k & 1) * n;
-    double* vn = vb + ((k + 1) & 1) * n;
-    const double t = tau[k];
-    {   // p = t B v by columns, and this warp's share of K = p.v
-      double vr[RM];
-#pragma unroll
-      for (int r = 0; r < RM; ++r) {
-        const int i = lane + 32 * r;
-        vr[r] = (i < m) ? v[i] : 0.0;
-      }
-      // CW columns per warp at a time: their loads are independent, so a lane keeps CW * RM
-      // loads in flight instead of RM (the steps on the L2-resident matrix are latency-bound)
-      double kpart = 0.0;
-      for (int j0 = warp; j0 < m; j0 += CW * NW) {
-        double sc[CW];
-#pragma unroll
-        for (int c = 0; c < CW; ++c) {
-          const int j = j0 + c * NW;
-          double s0 = 0.0, s1 = 0.0;
-          if (j < m) {
-            const double* col = B + int64_t(j) * ld;
-#pragma unroll
-            for (int r = 0; r < RM; r += 2) {
-              const int i0 = lane + 32 * r, i1 = i0 + 32;
-              if (i0 < m) s0 += col[i0] * vr[r];
-              if (r + 1 < RM && i1 < m) s1 += col[i1] * vr[r + 1];
-            }
-          }
-          sc[c] = s0 + s1;
-        }
-#pragma unroll
-        for (int c = 0; c < CW; ++c) sc[c] = wsum(sc[c]);
-        if (lane == 0) {
-#pragma unroll
-          for (int c = 0; c < CW; ++c) {
-            const int j = j0 + c * NW;
-            if (j < m) {
-              const double pj = t * sc[c];
-              p[j] = pj;
-              kpart += pj * v[j];
-            }
-          }
-        }
-      }
-      if (lane == 0) kw[warp] = kpart;
-    }
-    __syncthreads();
-    double K = 0.0;
-#pragma unroll
-    for (int w = 0; w < NW; ++w) K += kw[w];
-    const double hk = 0.5 * t * K;
-    if (warp == 0) {
-      // pivot column (column 0 of B) with the update applied, then the next reflector from it
-      const double v0 = v[0];
-      const double w0 = p[0] - hk * v0;
-      double c[RM];
-#pragma unroll
-      for (int r = 0; r < RM; ++r) {
-        const int i = lane + 32 * r;
-        double vi = 0.0, pi = 0.0, bi = 0.0;
-        if (i < m) { vi = v[i]; pi = p[i]; bi = B[i]; }
-        const double wi = pi - hk * vi;
-        c[r] = bi - (vi * w0 + wi * v0);
-      }
-      if (k + 3 < n) {
-        double part = 0.0;
-#pragma unroll
-        for (int r = 0; r < RM; ++r) {
-          const int i = lane + 32 * r;
-          if (i >= 2 && i < m) part += c[r] * c[r];
-        }
-        const double xn2 = wsum(part);
-        const double alpha = __shfl_sync(FULL, c[0], 1);
-        double tn, sc, beta;
-        if (xn2 == 0.0) {
-          tn = 0.0; sc = 0.0; beta = alpha;
-        } else {
-          beta = -copysign(sqrt(alpha * alpha + xn2), alpha);
-          tn = (beta - alpha) / beta;
-          sc = 1.0 / (alpha - beta);
-        }
-#pragma unroll
-        for (int r = 0; r < RM; ++r) {
-          const int i = lane + 32 * r;
-          if (i >= 1 && i < m) {
-            const double vi = (i == 1) ? 1.0 : c[r] * sc;
-            vn[i - 1] = vi;
-            if (i >= 2) B[i] = vi;         // reflector tail, below the subdiagonal
-          }
-        }
-        if (lane == 0) {
-          d[k + 1] = c[0];
-          e[k + 1] = beta;
-          tau[k + 1] = tn;
-        }
-      } else {
-#pragma unroll
-        for (int r = 0; r < RM; ++r) {
-          const int i = lane + 32 * r;
-          if (i < m) B[i] = c[r];
-        }
-      }
-    } else {
-      // columns 1..m-1, rows 1..m-1 (row 0 of B is never read again); CU columns at a time
-      double vi[RM], wi[RM];
-#pragma unroll
-      for (int r = 0; r < RM; ++r) {
-        const int i = 1 + lane + 32 * r;
-        vi[r] = (i < m) ? v[i] : 0.0;
-        wi[r] = (i < m) ? p[i] - hk * vi[r] : 0.0;
-      }
-      for (int j0 = warp; j0 < m; j0 += CU * (NW - 1)) {
-        double cv[CU][RM];
-#pragma unroll
-        for (int c = 0; c < CU; ++c) {
-          const int j = j0 + c * (NW - 1);
-#pragma unroll
-          for (int r = 0; r < RM; ++r) {
-            const int i = 1 + lane + 32 * r;
-            cv[c][r] = (j < m && i < m) ? B[int64_t(j) * ld + i] : 0.0;
-          }
-        }
-#pragma unroll
-        for (int c = 0; c < CU; ++c) {
-          const int j = j0 + c * (NW - 1);
-          if (j < m) {
-            const double vj = v[j], wj = p[j] - hk * vj;
-            double* col = B + int64_t(j) * ld;
-#pragma unroll
-            for (int r = 0; r < RM; ++r) {
-              const int i = 1 + lane + 32 * r;
-              if (i < m) col[i] = cv[c][r] - (vi[r] * wj + wi[r] * vj);
-            }
-          }
-        }
-      }
-    }
-    __syncthreads();
-    B += ld + 1;
-  }
-
-  // the trailing block of step k_sw into shared memory (lower triangle, packed), then the
-  // remaining steps there: p = tau B v by row pairs (thread 2a sums row a's stored part b <= a
-  // along the diagonal direction, thread 2a+1 the column a part b > a), the rank-2 update by
-  // columns, warp 0 updating the pivot column first and building the next reflector from it
-  const int k_sw = k, m0 = n - k - 1;
-  for (int x = tid; x < m0 * m0; x += MT) {
-    const int i = x % m0, j = x / m0;
-    if (i >= j) S[pk(j, m0) + i - j] = B[i + int64_t(j) * ld];
-  }
-  __syncthreads();
-  for (; k + 2 < n; ++k) {
-    const int s0 = k - k_sw, m = n - k - 1;
-    const double* v = vb + (k & 1) * n;
-    double* vn = vb + ((k + 1) & 1) * n;
-    const double t = tau[k];
-    const int pks0 = pk(s0, m0);
-    {
-      const int a = tid >> 1, h = tid & 1;
-      double sa = 0.0, sb = 0.0;
-      if (a < m) {
-        if (h == 0) {                      // b = 0..a: element (a, b) in column s0 + b
-          int idx = pks0 + a;
-          int b = 0;
-          for (; b + 1 <= a; b += 2) {
-            sa += S[idx] * v[b];
-            idx += m - b - 1;
-            sb += S[idx] * v[b + 1];
-            idx += m - b - 2;
-          }
-          if (b <= a) sa += S[idx] * v[b];
-        } else {                           // b = a+1..m-1: element (b, a) in column s0 + a
-          const double* col = S + pk(s0 + a, m0) - a;
-          int b = a + 1;
-          for (; b + 2 <= m; b += 2) {
-            sa += col[b] * v[b];
-            sb += col[b + 1] * v[b + 1];
-          }
-          if (b < m) sa += col[b] * v[b];
-        }
-      }
-      double sum = sa + sb;
-      sum += __shfl_xor_sync(FULL, sum, 1);
-      double kpart = 0.0;
-      if (a < m && h == 0) {
-        const double pa = t * sum;
-        p[a] = pa;
-        kpart = pa * v[a];
-      }
-      kpart = wsum(kpart);
-      if (lane == 0) kw[warp] = kpart;
-    }
-    __syncthreads();
-    double K = 0.0;
-#pragma unroll
-    for (int w = 0; w < NW; ++w) K += kw[w];
-    const double hk = 0.5 * t * K;
-    if (warp == 0) {
-      double* B0 = S + pks0;               // pivot column: rows 0..m-1
-      const double v0 = v[0];
-      const double w0 = p[0] - hk * v0;
-      double c[RM];
-#pragma unroll
-      for (int r = 0; r < RM; ++r) {
-        const int i = lane + 32 * r;
-        double vi = 0.0, pi = 0.0, bi = 0.0;
-        if (i < m) { vi = v[i]; pi = p[i]; bi = B0[i]; }
-        const double wi = pi - hk * vi;
-        c[r] = bi - (vi * w0 + wi * v0);
-      }
-      if (k + 3 < n) {
-        double part = 0.0;
-#pragma unroll
-        for (int r = 0; r < RM; ++r) {
-          const int i = lane + 32 * r;
-          if (i >= 2 && i < m) part += c[r] * c[r];
-        }
-        const double xn2 = wsum(part);
-        const double alpha = __shfl_sync(FULL, c[0], 1);
-        double tn, sc, beta;
-        if (xn2 == 0.0) {
-          tn = 0.0; sc = 0.0; beta = alpha;
-        } else {
-          beta = -copysign(sqrt(alpha * alpha + xn2), alpha);
-          tn = (beta - alpha) / beta;
-          sc = 1.0 / (alpha - beta);
-        }
-#pragma unroll
-        for (int r = 0; r < RM; ++r) {
-          const int i = lane + 32 * r;
-          if (i >= 1 && i < m) {
-            const double vi = (i == 1) ? 1.0 : c[r] * sc;
-            vn[i - 1] = vi;
-            if (i >= 2) B0[i] = vi;        // reflector tail, below the subdiagonal
-          }
-        }
-        if (lane == 0) {
-          d[k + 1] = c[0];
-          e[k + 1] = beta;
-          tau[k + 1] = tn;
-        }
-      } else {
-#pragma unroll
-        for (int r = 0; r < RM; ++r) {
-          const int i = lane + 32 * r;
-          if (i < m) B0[i] = c[r];
-        }
-      }
-    } else {
-      for (int j = warp; j < m; j += NW - 1) {   // columns 1..m-1, rows j..m-1
-        const double vj = v[j], wj = p[j] - hk * vj;
-        double* col = S + pk(s0 + j, m0) - j;
-        for (int i = j + lane; i < m; i += 32) {
-          const double vi = v[i], wi = p[i] - hk * vi;
-          col[i] = col[i] - (vi * wj + wi * vj);
-        }
-      }
-    }
-    __syncthreads();
-  }
-  if (tid == 0) {   // the last 2 x 2 block: A[n-2.., n-2..] at packed column s0f - 1 and s0f
-    const int s0f = (n - 2) - k_sw;
-    d[n - 2] = S[pk(s0f - 1, m0)];
-    e[n - 2] = S[pk(s0f - 1, m0) + 1];
-    tau[n - 2] = 0.0;
-    d[n - 1] = S[pk(s0f, m0)];
-    e[n - 1] = 0.0;
-    tau[n - 1] = 0.0;
-  }
-  {   // the packed block back into the caller's matrix (its reflector tails)
-    double* G = Ag + int64_t(k_sw + 1) * n + (k_sw + 1);
-    for (int x = tid; x < m0 * m0; x += MT) {
-      const int i = x % m0, j = x / m0;
-      if (i >= j) G[i + int64_t(j) * n] = S[pk(j, m0) + i - j];
-    }
-  }
-  __syncthreads();
-  for (int i = tid; i < n; i += MT) e2[i] = e[i] * e[i];
-  double* ws = base + tk.ws_off;          // d | e | tau
-  for (int i = tid; i < n; i += MT) {
-    ws[i] = d[i];
-    ws[n + i] = e[i];
-    ws[2 * n + i] = tau[i];
-  }
-  if (warp == 0) {   // Gershgorin interval
-    double lo = 1e300, hi = -1e300;
-    for (int i = lane; i < n; i += 32) {
-      const double r = (i > 0 ? fabs(e[i - 1]) : 0.0) + (i + 1 < n ? fabs(e[i]) : 0.0);
-      lo = fmin(lo, d[i] - r);
-      hi = fmax(hi, d[i] + r);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      lo = fmin(lo, __shfl_xor_sync(FULL, lo, o));
-      hi = fmax(hi, __shfl_xor_sync(FULL, hi, o));
-    }
-    if (lane == 0) {
-      const double pad = 2.2e-16 * fmax(fabs(lo), fabs(hi)) + 1e-300;
-      s_lo = lo - pad;
-      s_hi = hi + pad;
-    }
-  }
-  __syncthreads();
-  // trisection, MT/2 eigenvalues per round: threads 2i, 2i+1 count at the interval's two
-  // interior points
-  const double tnm = fmax(fabs(s_lo), fabs(s_hi));
-  const double tol = 8.9e-16 * tnm;
-  for (int e0 = 0; e0 < n; e0 += MT / 2) {
-    const int ei = e0 + (tid >> 1), h = tid & 1;
-    const int target = n - 1 - ei;         // i-th largest = (n-1-i)-th smallest
-    bool done = ei >= n;
-    double a = s_lo, b = s_hi;
-    for (int it = 0; it < 200; ++it) {
-      if (__all_sync(FULL, done)) break;
-      double x0 = 0.0, x1 = 0.0;
-      bool below = false;
-      if (!done) {
-        const double w = b - a;
-        x0 = a + w * (1.0 / 3.0);
-        x1 = a + w * (2.0 / 3.0);
-        if (w <= tol || !(a < x0 && x0 < x1 && x1 < b)) done = true;
-        else below = sturm_below(d, e2, n, h ? x1 : x0) > target;
-      }
-      const bool other = __shfl_xor_sync(FULL, below, 1);
-      if (!done) {
-        const bool r0 = h ? other : below, r1 = h ? below : other;
-        if (r0) b = x0;
-        else if (r1) { a = x0; b = x1; }
-        else a = x1;
-      }
-    }
-    if (h == 0 && ei < n) base[tk.w_off + ei] = 0.5 * (a + b);
-  }
-}
 
 // Workspace of one task of k_trid_mid_vectors, in doubles from x_off: LU factors (4 n k),
 // pivots (n k ints), Z (n x (k|1), row-major), Gram matrix (k x k).
@@ -828,35 +416,10 @@ k_trid_mid_backtransform(double* __restrict__ base, const TridTask* __restrict__
   }
 }
 
-int mid_mp(int max_n) {
-  // largest trailing block whose packed lower triangle fits in shared memory beside the 7 n
-  // vectors (at least 2: the last steps always run there)
-  const size_t avail = MID_SMEM_LIMIT - sizeof(double) * 7 * size_t(max_n) - 64;
-  int mp = 2;
-  while (size_t(mp + 1) * (mp + 2) / 2 * sizeof(double) <= avail) ++mp;
-  return mp;
-}
-
-template <int RM>
-void launch_vals(cudaStream_t s, double* base, const TridTask* tasks, int ntasks, int max_n) {
-  const int mp = mid_mp(max_n);
-  const size_t sm = sizeof(double) * (size_t(mp) * (mp + 1) / 2 + 7 * size_t(max_n)) + 64;
-  raise_smem_limit(reinterpret_cast<const void*>(k_trid_mid_vals<RM>), sm);
-  launch_k(k_trid_mid_vals<RM>, ntasks, MT, sm, s, base, tasks, mp);
-  count_launch();
-}
-
 }  // namespace
 
 int64_t syevt_mid_workspace(int n, int k) { return mid_vec_workspace(n, k); }
 int syevt_mid_gram_limit(int max_n) { return mid_vec_kg(max_n); }
-
-void launch_trid_mid_eigvals(cudaStream_t s, double* base, const TridTask* tasks, int ntasks,
-                             int max_n) {
-  if (ntasks <= 0) return;
-  if (max_n <= 256) launch_vals<8>(s, base, tasks, ntasks, max_n);
-  else launch_vals<16>(s, base, tasks, ntasks, max_n);
-}
 
 void launch_trid_mid_vectors(cudaStream_t s, double* base, const TridTask* tasks, int ntasks,
                              int max_n, int max_k, double* xws) {
