@@ -84,9 +84,6 @@ void launch_trid_eigvals(cudaStream_t s, double* base, const TridTask* tasks, in
 void launch_trid_vectors(cudaStream_t s, double* base, const TridTask* tasks, int ntasks,
                          int max_n, int max_k);
 int64_t syevt_mid_workspace(int n, int k);
-// Largest kept count whose Gram matrix the mid-size vector kernel holds in shared memory for
-// blocks up to max_n (tasks above it take the global-memory path; launch them separately).
-int syevt_mid_gram_limit(int max_n);
 // Tridiagonalisation by thread-block clusters and all eigenvalues (syevt_cluster.cu); sum_n: the
 // blocks' sizes added up.
 void launch_trid_cluster(cudaStream_t s, double* base, const TridTask* tasks, int ntasks,

@@ -1,14 +1,23 @@
 // syevt_mid.cu -- eigenvectors of mid-size density-matrix blocks, SYEVT_NMAX < n <= SYEVT_MID_NMAX
-// (their tridiagonal matrices and eigenvalues come from syevt_cluster.cu), one CTA of 512 threads
-// per block.
-// Launch 1 (k_trid_mid_vectors): inverse iteration (one thread per kept vector, LU factors in a
-// global workspace interleaved by thread so that every factor access of a warp is one line),
-// Cholesky QR (a second pass unless the Gram matrix is within 1e-3/k of the identity; classical
-// Gram-Schmidt with restarts if a pivot shows nearly dependent vectors); the vectors Z of the
-// tridiagonal matrix stay in the workspace.
-// Launch 2 (k_trid_mid_backtransform): U = H_0 ... H_{n-3} Z in blocks of 8 reflectors (compact
-// WY), one CTA per slice of 32 kept vectors with its slice of Z in shared memory, the reflectors
-// read from the matrix in global memory (every slice is independent of the others).
+// (their tridiagonal matrices and eigenvalues come from syevt_cluster.cu). Every part runs on many
+// CTAs; one CTA per block for all of it took 1.6 + 0.54 ms at n = 345 with 200 kept vectors.
+//   * k_mid_invit: inverse iteration, one thread per kept vector, one warp per CTA; LU factors in
+//     a global workspace interleaved by thread, so that a warp's accesses to one factor element
+//     form one line. Bound by the latency of the recurrences.
+//   * k_mid_runs: vectors of (nearly) equal eigenvalues, which come out as independent but not
+//     orthogonal vectors of their common eigenspace, are orthonormalised among themselves.
+//   * up to three rounds of k_mid_gram and k_mid_apply: G = Z^T Z = I + E with a small E (vectors
+//     of separated eigenvalues are orthogonal to eps ||A|| / gap), then Z <- Z (I - E_up), E_up =
+//     the strict upper triangle and half the diagonal of E: the first-order Cholesky QR, which
+//     squares E each round and is two matrix products instead of an elimination of k dependent
+//     steps. A round whose predecessor left nothing to do returns at once.
+//   * k_mid_cholqr: blocks that round zero cannot treat (long runs of equal or numerically zero
+//     eigenvalues, nearly dependent vectors) take the Cholesky QR or Gram-Schmidt of one CTA; it
+//     returns at once for all others.
+//   * k_mid_back: U = H_0 ... H_{n-3} Z, two vectors per warp in registers, the reflectors read
+//     from the matrix in global memory two at a time, one pair ahead.
+#include <algorithm>
+
 #include "kernels.cuh"
 #include "launch.cuh"
 #include "syevt_common.cuh"
@@ -18,80 +27,272 @@ namespace {
 
 constexpr int MT = 512;             // threads per CTA
 constexpr int NW = MT / 32;         // warps
-constexpr int MID_BT_NB = 8;        // reflectors per back-transformation block
 constexpr size_t MID_SMEM_LIMIT = 227 * 1024 - 2048;
 
-// Workspace of one task of k_trid_mid_vectors, in doubles from x_off: LU factors (4 n k),
-// pivots (n k ints), Z (n x (k|1), row-major), Gram matrix (k x k).
+// Workspace of one task, in doubles from x_off: LU factors (4 n k), pivots (n k ints), Z (n x
+// (k|1), row-major), Gram matrix (k x k, row-major, upper triangle), control words.
+struct MidCtl {
+  unsigned long long emax[3];   // largest |E| of each round (bits of a non-negative double)
+  unsigned long long slow;      // set: the block goes to k_mid_cholqr
+};
+__host__ __device__ inline int64_t mid_z_off(int n, int k) {
+  return 4 * int64_t(n) * k + (int64_t(n) * k + 1) / 2;
+}
+__host__ __device__ inline int64_t mid_g_off(int n, int k) {
+  return mid_z_off(n, k) + int64_t(n) * (k | 1);
+}
 __host__ __device__ inline int64_t mid_vec_workspace(int n, int k) {
-  const int64_t ldz = k | 1;
-  return 4 * int64_t(n) * k + (int64_t(n) * k + 1) / 2 + int64_t(n) * ldz + int64_t(k) * k + 8;
+  return mid_g_off(n, k) + int64_t(k) * k + 8;
+}
+__device__ __forceinline__ MidCtl* mid_ctl(double* X, int n, int k) {
+  return reinterpret_cast<MidCtl*>(X + mid_g_off(n, k) + int64_t(k) * k);
+}
+
+// ---- inverse iteration: one warp per CTA, blockIdx.x = group of 32 vectors, blockIdx.y = task
+__global__ void __launch_bounds__(32)
+k_mid_invit(double* __restrict__ base, const TridTask* __restrict__ tasks,
+            double* __restrict__ xws) {
+  grid_entry();
+  const TridTask tk = tasks[blockIdx.y];
+  const int n = tk.n, kk = tk.keep, j = blockIdx.x * 32 + threadIdx.x;
+  if (int(blockIdx.x) * 32 >= kk) return;
+  extern __shared__ double sm[];
+  double* d = sm;
+  double* e = sm + n;
+  const double* ws = base + tk.ws_off;
+  const double* W = base + tk.w_off;
+  for (int i = threadIdx.x; i < n; i += 32) { d[i] = ws[i]; e[i] = ws[n + i]; }
+  __syncwarp();
+  if (j >= kk) return;
+  const double tn = fmax(fmax(fabs(W[0]), fabs(W[n - 1])), 1e-300);   // descending
+  double* X = xws + tk.x_off;
+  double* Z = X + mid_z_off(n, kk);
+  const int ldz = kk | 1;
+  LUSlot f{X + j, X + int64_t(n) * kk + j, X + 2 * int64_t(n) * kk + j,
+           X + 3 * int64_t(n) * kk + j, reinterpret_cast<int*>(X + 4 * int64_t(n) * kk) + j, kk};
+  for (int r = 0; r < n; ++r) Z[int64_t(r) * ldz + j] = prand(r, j);
+  // kept eigenvalues that are numerically zero keep the pseudo-random vector alone
+  if (W[j] > 1e-13 * tn) inverse_iteration(d, e, n, W[j], Z, ldz, j, tn, f);
+}
+
+// ---- runs of nearly equal eigenvalues (neighbours within 1e-12 ||T||): modified Gram-Schmidt
+// inside each run, twice, one warp per run. Runs longer than RUN_MAX go to k_mid_cholqr.
+constexpr int RUN_THREADS = 256, RUN_MAX = 32;
+__global__ void __launch_bounds__(RUN_THREADS)
+k_mid_runs(double* __restrict__ base, const TridTask* __restrict__ tasks,
+           double* __restrict__ xws) {
+  grid_entry();
+  const TridTask tk = tasks[blockIdx.x];
+  const int n = tk.n, kk = tk.keep;
+  if (n < 3 || kk <= 0) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const double* W = base + tk.w_off;
+  const double tol = 1e-12 * fmax(fmax(fabs(W[0]), fabs(W[n - 1])), 1e-300);
+  double* X = xws + tk.x_off;
+  double* Z = X + mid_z_off(n, kk);
+  MidCtl* ctl = mid_ctl(X, n, kk);
+  const int ldz = kk | 1;
+  if (threadIdx.x < 4) (threadIdx.x < 3 ? ctl->emax[threadIdx.x] : ctl->slow) = 0ull;
+  __syncthreads();
+  for (int j = warp; j < kk; j += RUN_THREADS / 32) {
+    if (j > 0 && !(W[j - 1] - W[j] > tol)) continue;       // not the first of its run
+    int len = 1;
+    while (j + len < kk && !(W[j + len - 1] - W[j + len] > tol)) ++len;
+    if (len > RUN_MAX) {
+      if (lane == 0) ctl->slow = 1ull;
+      continue;
+    }
+    for (int c = 0; c < len && len > 1; ++c) {
+      double* zc = Z + j + c;
+      for (int pass = 0; pass < 2; ++pass)
+        for (int p = 0; p < c; ++p) {
+          const double* zp = Z + j + p;
+          double s = 0.0;
+          for (int r = lane; r < n; r += 32) s += zp[int64_t(r) * ldz] * zc[int64_t(r) * ldz];
+          s = wsum(s);
+          for (int r = lane; r < n; r += 32) zc[int64_t(r) * ldz] -= s * zp[int64_t(r) * ldz];
+        }
+      double s = 0.0;
+      for (int r = lane; r < n; r += 32) s += zc[int64_t(r) * ldz] * zc[int64_t(r) * ldz];
+      s = sqrt(wsum(s));
+      if (!(s > 1e-4)) {                                    // nearly dependent
+        if (lane == 0) ctl->slow = 1ull;
+        break;
+      }
+      const double inv = 1.0 / s;
+      for (int r = lane; r < n; r += 32) zc[int64_t(r) * ldz] *= inv;
+    }
+  }
+}
+
+// Whether round `pass` has anything to do: not for a block handed to k_mid_cholqr, nor after a
+// round that found |E| < 1e-9 (its own correction leaves E^2).
+__device__ __forceinline__ bool round_active(const MidCtl* ctl, int pass) {
+  if (ctl->slow) return false;
+  return pass == 0 || __longlong_as_double(ctl->emax[pass - 1]) >= 1e-9;
+}
+
+// ---- G = Z^T Z, one 32 x 32 tile of its upper triangle per CTA (blockIdx.x; blockIdx.y = task),
+// rows of Z in chunks of 32 through shared memory, the next chunk on its way in registers
+constexpr int GT = 256;
+__global__ void __launch_bounds__(GT)
+k_mid_gram(double* __restrict__ base, const TridTask* __restrict__ tasks, double* __restrict__ xws,
+           int pass) {
+  grid_entry();
+  const TridTask tk = tasks[blockIdx.y];
+  const int n = tk.n, kk = tk.keep;
+  if (n < 3 || kk <= 0) return;
+  const int nt = (kk + 31) >> 5;
+  if (int(blockIdx.x) >= nt * (nt + 1) / 2) return;
+  int I = 0, x = blockIdx.x;
+  while (x >= nt - I) { x -= nt - I; ++I; }
+  const int J = I + x;
+  double* X = xws + tk.x_off;
+  MidCtl* ctl = mid_ctl(X, n, kk);
+  if (!round_active(ctl, pass)) return;
+  const double* Z = X + mid_z_off(n, kk);
+  double* G = X + mid_g_off(n, kk);
+  const int ldz = kk | 1;
+  __shared__ double sa[32][33], sb[32][33];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  double pa[4], pb[4];
+  auto fetch = [&](int r0) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int r = r0 + warp + 8 * u, ca = 32 * I + lane, cb = 32 * J + lane;
+      pa[u] = (r < n && ca < kk) ? Z[int64_t(r) * ldz + ca] : 0.0;
+      pb[u] = (r < n && cb < kk) ? Z[int64_t(r) * ldz + cb] : 0.0;
+    }
+  };
+  const int tp = 2 * (tid >> 4), tq = 2 * (tid & 15);
+  double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+  fetch(0);
+  for (int r0 = 0; r0 < n; r0 += 32) {
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      sa[warp + 8 * u][lane] = pa[u];
+      sb[warp + 8 * u][lane] = pb[u];
+    }
+    __syncthreads();
+    if (r0 + 32 < n) fetch(r0 + 32);
+#pragma unroll 8
+    for (int r = 0; r < 32; ++r) {
+      const double a0 = sa[r][tp], a1 = sa[r][tp + 1], b0 = sb[r][tq], b1 = sb[r][tq + 1];
+      acc[0][0] += a0 * b0;
+      acc[0][1] += a0 * b1;
+      acc[1][0] += a1 * b0;
+      acc[1][1] += a1 * b1;
+    }
+  }
+  double mx = 0.0;
+#pragma unroll
+  for (int u = 0; u < 2; ++u)
+#pragma unroll
+    for (int v = 0; v < 2; ++v) {
+      const int p = 32 * I + tp + u, q = 32 * J + tq + v;
+      if (p <= q && q < kk) {
+        G[int64_t(p) * kk + q] = acc[u][v];
+        const double ev = fabs(acc[u][v] - (p == q ? 1.0 : 0.0));
+        mx = ev > mx || ev != ev ? ev : mx;
+      }
+    }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const double t = __shfl_xor_sync(FULL, mx, o);
+    mx = t > mx || t != t ? t : mx;
+  }
+  if (lane == 0)
+    atomicMax(&ctl->emax[pass], (unsigned long long)(__double_as_longlong(mx)) & ~(1ull << 63));
+}
+
+// ---- Z <- Z (I - E_up), 16 rows per CTA (blockIdx.x; blockIdx.y = task)
+constexpr int AR = 16;
+__global__ void __launch_bounds__(GT)
+k_mid_apply(double* __restrict__ base, const TridTask* __restrict__ tasks,
+            double* __restrict__ xws, int pass) {
+  grid_entry();
+  const TridTask tk = tasks[blockIdx.y];
+  const int n = tk.n, kk = tk.keep, r0 = blockIdx.x * AR;
+  if (n < 3 || kk <= 0 || r0 >= n) return;
+  double* X = xws + tk.x_off;
+  MidCtl* ctl = mid_ctl(X, n, kk);
+  if (!round_active(ctl, pass)) return;
+  // the rounds square E: what is not small enough for the rounds that remain goes to k_mid_cholqr
+  const double lim = pass == 0 ? 1e-3 : (pass == 1 ? 1e-5 : 1e-9);
+  if (!(__longlong_as_double(ctl->emax[pass]) <= lim)) {
+    if (threadIdx.x == 0) ctl->slow = 1ull;
+    return;
+  }
+  double* Z = X + mid_z_off(n, kk);
+  const double* G = X + mid_g_off(n, kk);
+  const int ldz = kk | 1;
+  extern __shared__ __align__(16) double sm[];         // kk x AR: row r of the slab at [p * AR + r]
+  const int tid = threadIdx.x;
+  for (int x = tid; x < AR * kk; x += GT) {
+    const int r = x / kk, p = x - r * kk;
+    sm[p * AR + r] = r0 + r < n ? Z[int64_t(r0 + r) * ldz + p] : 0.0;
+  }
+  __syncthreads();
+  for (int q = tid; q < kk; q += GT) {
+    double acc[AR];
+#pragma unroll
+    for (int r = 0; r < AR; ++r) acc[r] = 0.0;
+#pragma unroll 4
+    for (int p = 0; p < q; ++p) {
+      const double g = G[int64_t(p) * kk + q];
+      const double2* zp = reinterpret_cast<const double2*>(sm + p * AR);
+#pragma unroll
+      for (int r = 0; r < AR / 2; ++r) {
+        const double2 z = zp[r];
+        acc[2 * r] += z.x * g;
+        acc[2 * r + 1] += z.y * g;
+      }
+    }
+    const double h = 0.5 * (G[int64_t(q) * kk + q] - 1.0);
+#pragma unroll
+    for (int r = 0; r < AR; ++r)
+      if (r0 + r < n) {
+        const double z = sm[q * AR + r];
+        Z[int64_t(r0 + r) * ldz + q] = z - fma(h, z, acc[r]);
+      }
+  }
 }
 
 // Packed upper triangle by rows of a k x k matrix: row p starts at gpk(p, k).
 __host__ __device__ __forceinline__ int gpk(int p, int k) { return p * k - (p * (p - 1)) / 2; }
 
-// Shared memory of k_trid_mid_vectors: d, e (n each), rinv, sq (k each) and, for k <= kg, the
+// Shared memory of k_mid_cholqr: rinv, sq (k each) and, for k <= kg, the
 // packed Gram matrix. kg = the largest k for which all of it fits.
-__host__ __device__ inline size_t mid_vec_smem_k(int n, int k, bool gram) {
-  return sizeof(double) * (2 * size_t(n) + 2 * size_t(k) +
+__host__ __device__ inline size_t mid_vec_smem_k(int k, bool gram) {
+  return sizeof(double) * (2 * size_t(k) +
                            (gram ? size_t(k) * (k + 1) / 2 : 0)) + 64;
 }
-int mid_vec_kg(int max_n) {
+int mid_vec_kg() {
   int kg = 0;
-  while (mid_vec_smem_k(max_n, kg + 1, true) <= MID_SMEM_LIMIT) ++kg;
+  while (mid_vec_smem_k(kg + 1, true) <= MID_SMEM_LIMIT) ++kg;
   return kg;
 }
 
 __global__ void __launch_bounds__(MT, 1)
-k_trid_mid_vectors(double* __restrict__ base, const TridTask* __restrict__ tasks,
-                   double* __restrict__ xws, int kg) {
+k_mid_cholqr(double* __restrict__ base, const TridTask* __restrict__ tasks,
+             double* __restrict__ xws, int kg) {
   grid_entry();
   const TridTask tk = tasks[blockIdx.x];
   const int n = tk.n, kk = tk.keep;
   if (n < 3 || kk <= 0) return;
+  double* X = xws + tk.x_off;
+  if (mid_ctl(X, n, kk)->slow == 0ull) return;
   const int ldz = kk | 1;
   extern __shared__ double sm[];
-  double* d = sm;                          // n
-  double* e = d + n;                       // n
-  double* rinv = e + n;                    // kk
+  double* rinv = sm;                       // kk
   double* sq = rinv + kk;                  // kk
   __shared__ double red[32];
-  __shared__ double s_tn;
   __shared__ int s_flag, s_need2;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  double* X = xws + tk.x_off;
-  double* Un = X;                                          // 4 n kk factors
-  int* piv = reinterpret_cast<int*>(X + 4 * int64_t(n) * kk);
-  double* Z = X + 4 * int64_t(n) * kk + (int64_t(n) * kk + 1) / 2;   // n x ldz
-  double* G = Z + int64_t(n) * ldz;                        // kk x kk row-major, upper triangle
-  const double* ws = base + tk.ws_off;
-  const double* W = base + tk.w_off;
-  for (int i = tid; i < n; i += MT) { d[i] = ws[i]; e[i] = ws[n + i]; }
-  if (warp == 0) {
-    double tn = 0.0;
-    for (int i = lane; i < n; i += 32) tn = fmax(tn, fabs(W[i]));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) tn = fmax(tn, __shfl_xor_sync(FULL, tn, o));
-    if (lane == 0) {
-      s_tn = fmax(tn, 1e-300);
-      s_flag = 0;
-      s_need2 = 0;
-    }
-  }
-  __syncthreads();
-  const double tn = s_tn;
-  // ---- inverse iteration: one thread per kept vector; factor element q of thread j at
-  // [q * kk + j], so that a warp's accesses to one factor element form one line
-  for (int b0 = 0; b0 < kk; b0 += MT) {
-    const int j = b0 + tid;
-    if (j < kk) {
-      LUSlot f{Un + j, Un + int64_t(n) * kk + j, Un + 2 * int64_t(n) * kk + j,
-               Un + 3 * int64_t(n) * kk + j, piv + j, kk};
-      for (int r = 0; r < n; ++r) Z[int64_t(r) * ldz + j] = prand(r, j);
-      if (W[j] > 1e-13 * tn) inverse_iteration(d, e, n, W[j], Z, ldz, j, tn, f);
-    }
-  }
+  double* Z = X + mid_z_off(n, kk);                        // n x ldz
+  double* G = X + mid_g_off(n, kk);                        // kk x kk row-major, upper triangle
+  if (tid == 0) { s_flag = 0; s_need2 = 0; }
   __syncthreads();
   // ---- Cholesky QR: G = Z^T Z = R^T R with R = D^(1/2) U (U unit upper), Z <- Z U^-1 D^(-1/2);
   // a second pass unless G was within 1e-3/k of the identity. When the packed upper triangle of
@@ -290,153 +491,132 @@ k_trid_mid_vectors(double* __restrict__ base, const TridTask* __restrict__ tasks
   }
 }
 
-// Back-transformation U = H_0 H_1 ... H_{n-3} Z for one slice of BT_W kept vectors per CTA
-// (blockIdx.y = slice): the slice of Z is staged in shared memory, the reflectors are read from
-// the matrix in global memory (L2-resident, shared by the slices), applied in blocks of
-// MID_BT_NB with their compact-WY T factors (built by each CTA: cheap next to the product).
-constexpr int BT_W = 32;
-__global__ void __launch_bounds__(MT, 1)
-k_trid_mid_backtransform(double* __restrict__ base, const TridTask* __restrict__ tasks,
-                         const double* __restrict__ xws) {
+// Sums of s[0..5) over the warp, in every lane: exchanges that halve the values a lane carries,
+// then one broadcast each.
+__device__ __forceinline__ void wsum5(double (&s)[5], int lane) {
+  const bool b0 = lane & 1, b1 = lane & 2, b2 = lane & 4;
+  const double u0 = (b0 ? s[1] : s[0]) + __shfl_xor_sync(FULL, b0 ? s[0] : s[1], 1);
+  const double u1 = (b0 ? s[3] : s[2]) + __shfl_xor_sync(FULL, b0 ? s[2] : s[3], 1);
+  const double u2 = (b0 ? 0.0 : s[4]) + __shfl_xor_sync(FULL, b0 ? s[4] : 0.0, 1);
+  const double w0 = (b1 ? u1 : u0) + __shfl_xor_sync(FULL, b1 ? u0 : u1, 2);
+  const double w1 = (b1 ? 0.0 : u2) + __shfl_xor_sync(FULL, b1 ? u2 : 0.0, 2);
+  double v = (b2 ? w1 : w0) + __shfl_xor_sync(FULL, b2 ? w0 : w1, 4);
+  v += __shfl_xor_sync(FULL, v, 8);
+  v += __shfl_xor_sync(FULL, v, 16);
+#pragma unroll
+  for (int q = 0; q < 5; ++q) s[q] = __shfl_sync(FULL, v, q);
+}
+
+// Back-transformation U = H_0 H_1 ... H_{n-3} Z: two kept vectors per warp in registers (lane l
+// has rows l, l + 32, ...), n <= 32 RM. Two reflectors per step, a = v_k and b = v_{k-1}: their
+// four products with the vectors and a.b are one warp sum, and the next pair is loaded before it.
+// Bound by that sum's latency (about 300 of 500 cycles a step): blocks of more reflectors would
+// add products that the two warps per scheduler have no free issue slots for.
+constexpr int BW = 4;                    // warps per CTA
+template <int RM>
+__global__ void __launch_bounds__(32 * BW)
+k_mid_back(double* __restrict__ base, const TridTask* __restrict__ tasks,
+           const double* __restrict__ xws) {
   grid_entry();
-  const TridTask tk = tasks[blockIdx.x];
+  const TridTask tk = tasks[blockIdx.y];
   const int n = tk.n, kk = tk.keep;
-  const int q0 = blockIdx.y * BT_W;
-  if (n < 3 || q0 >= kk) return;
-  const int w = min(BT_W, kk - q0);
+  const int lane = threadIdx.x & 31, q0 = 2 * (blockIdx.x * BW + (threadIdx.x >> 5));
+  if (n < 3 || n > 32 * RM || q0 >= kk) return;
+  const bool two = q0 + 1 < kk;
   const int ldz = kk | 1;
-  const int nblk = (n - 2 + MID_BT_NB - 1) / MID_BT_NB;
-  extern __shared__ double sm[];
-  double* Zs = sm;                               // n x BT_W, row-major (Zs[r * BT_W + q])
-  double* Wv = Zs + size_t(n) * BT_W;            // MID_BT_NB x BT_W
-  double* Yv = Wv + MID_BT_NB * BT_W;            // MID_BT_NB x BT_W
-  double* Tb = Yv + MID_BT_NB * BT_W;            // nblk x 64
-  double* Sw = Tb + size_t(nblk) * 64;           // NW x 64
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const double* X = xws + tk.x_off;
-  const double* Z = X + 4 * int64_t(n) * kk + (int64_t(n) * kk + 1) / 2;
+  const double* Z = xws + tk.x_off + mid_z_off(n, kk);
   const double* V = base + tk.a_off;             // reflector k: V[k n + r], r > k + 1
   const double* tau = base + tk.ws_off + 2 * n;
-  for (int x = tid; x < n * BT_W; x += MT) {
-    const int r = x / BT_W, q = x - r * BT_W;
-    Zs[x] = q < w ? Z[int64_t(r) * ldz + q0 + q] : 0.0;
+  double z0[RM], z1[RM], a[RM], b[RM];
+  double ta = 0.0, tb = 0.0;
+  auto load = [&](int k) {                       // the pair (k, k - 1)
+    ta = k >= 0 ? tau[k] : 0.0;
+    tb = k >= 1 ? tau[k - 1] : 0.0;
+#pragma unroll
+    for (int r = 0; r < RM; ++r) {
+      const int i = lane + 32 * r;
+      double va = 0.0, vb = 0.0;
+      if (32 * r + 31 >= k && i < n) {
+        if (k >= 0 && i >= k + 1) va = i == k + 1 ? 1.0 : V[int64_t(k) * n + i];
+        if (k >= 1 && i >= k) vb = i == k ? 1.0 : V[int64_t(k - 1) * n + i];
+      }
+      a[r] = va;
+      b[r] = vb;
+    }
+  };
+#pragma unroll
+  for (int r = 0; r < RM; ++r) {
+    const int i = lane + 32 * r;
+    z0[r] = i < n ? Z[int64_t(i) * ldz + q0] : 0.0;
+    z1[r] = i < n && two ? Z[int64_t(i) * ldz + q0 + 1] : 0.0;
   }
-  // T factor of every reflector block (one warp per block)
-  for (int bb = warp; bb < nblk; bb += NW) {
-    const int k0 = bb * MID_BT_NB, nb = min(MID_BT_NB, n - 2 - k0);
-    double* Sg = Sw + warp * 64;
-    if (lane < 28) {                      // Sg[c][i] = v_c . v_i, c < i
-      int c = 0, i = 0, x = lane;
-      for (int cc = 0; cc < MID_BT_NB; ++cc) {
-        const int cnt = MID_BT_NB - 1 - cc;
-        if (x < cnt) { c = cc; i = cc + 1 + x; break; }
-        x -= cnt;
-      }
-      if (i < nb) {
-        const int kc = k0 + c, ki = k0 + i;
-        const double* vc = V + int64_t(kc) * n;
-        const double* vi = V + int64_t(ki) * n;
-        double s0 = vc[ki + 1], s1 = 0.0;      // v_i[ki+1] = 1
-        int r = ki + 2;
-        for (; r + 2 <= n; r += 2) { s0 += vc[r] * vi[r]; s1 += vc[r + 1] * vi[r + 1]; }
-        if (r < n) s0 += vc[r] * vi[r];
-        Sg[c * 8 + i] = s0 + s1;
-      }
-    }
-    __syncwarp();
-    if (lane < nb) {                      // row a of T: T[a][i] = -tau_i sum_{c=a}^{i-1} T[a][c] S[c][i]
-      const int a = lane;
-      double Tr[MID_BT_NB];
+  load(n - 3);
+  for (int k = n - 3; k >= 0; k -= 2) {
+    double s[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    double ca[RM], cb[RM];
+    const double cta = ta, ctb = tb;
 #pragma unroll
-      for (int i = 0; i < MID_BT_NB; ++i) {
-        double v = 0.0;
-        if (i == a) {
-          v = tau[k0 + a];
-        } else if (i > a && i < nb) {
-          double sacc = 0.0;
-#pragma unroll
-          for (int c = 0; c < MID_BT_NB; ++c)
-            if (c >= a && c < i) sacc += Tr[c] * Sg[c * 8 + i];
-          v = -tau[k0 + i] * sacc;
-        }
-        Tr[i] = v;
+    for (int r = 0; r < RM; ++r) {
+      ca[r] = a[r];
+      cb[r] = b[r];
+      if (32 * r + 31 >= k) {
+        s[0] = fma(ca[r], z0[r], s[0]);
+        s[1] = fma(ca[r], z1[r], s[1]);
+        s[2] = fma(cb[r], z0[r], s[2]);
+        s[3] = fma(cb[r], z1[r], s[3]);
+        s[4] = fma(ca[r], cb[r], s[4]);
       }
+    }
+    load(k - 2);
+    wsum5(s, lane);
+    const double x0 = cta * s[0], x1 = cta * s[1];
+    const double y0 = ctb * fma(-x0, s[4], s[2]), y1 = ctb * fma(-x1, s[4], s[3]);
 #pragma unroll
-      for (int i = 0; i < MID_BT_NB; ++i) Tb[bb * 64 + a * 8 + i] = Tr[i];
-    }
-    __syncwarp();
-  }
-  __syncthreads();
-  for (int bb = nblk - 1; bb >= 0; --bb) {
-    const int k0 = bb * MID_BT_NB, nb = min(MID_BT_NB, n - 2 - k0);
-    const double* T = Tb + bb * 64;
-    {   // W = V^T Zs: pair (a, q) with the rows split between the two halves of the block
-      const int half = tid / (MT / 2), pq = tid - half * (MT / 2);
-      const int a = pq / BT_W, q = pq - a * BT_W;
-      double sacc = 0.0;
-      if (a < nb) {
-        const int k = k0 + a;
-        const double* vk = V + int64_t(k) * n;
-        if (half == 0) sacc = Zs[(k + 1) * BT_W + q];
-        for (int r = k + 2 + half; r < n; r += 2) sacc += vk[r] * Zs[r * BT_W + q];
+    for (int r = 0; r < RM; ++r) {
+      if (32 * r + 31 >= k) {
+        z0[r] = fma(-y0, cb[r], fma(-x0, ca[r], z0[r]));
+        z1[r] = fma(-y1, cb[r], fma(-x1, ca[r], z1[r]));
       }
-      if (half == 1 && a < MID_BT_NB) Wv[a * BT_W + q] = sacc;
-      __syncthreads();
-      if (half == 0 && a < MID_BT_NB) Wv[a * BT_W + q] += sacc;
     }
-    __syncthreads();
-    if (tid < MID_BT_NB * BT_W) {         // Y = T W
-      const int a = tid / BT_W, q = tid - a * BT_W;
-      double y = 0.0;
-      if (a < nb)
-        for (int c = a; c < nb; ++c) y += T[a * 8 + c] * Wv[c * BT_W + q];
-      Yv[a * BT_W + q] = y;
-    }
-    __syncthreads();
-    // Zs -= V Y on rows k0+1..n-1
-    for (int x = (k0 + 1) * BT_W + tid; x < n * BT_W; x += MT) {
-      const int r = x / BT_W, q = x - r * BT_W;
-      double sacc = 0.0;
-#pragma unroll
-      for (int a = 0; a < MID_BT_NB; ++a) {
-        const int k = k0 + a;
-        if (a < nb && r >= k + 1) {
-          const double va = (r == k + 1) ? 1.0 : V[int64_t(k) * n + r];
-          sacc += va * Yv[a * BT_W + q];
-        }
-      }
-      Zs[x] -= sacc;
-    }
-    __syncthreads();
   }
   double* U = base + tk.u_off;
-  for (int x = tid; x < n * w; x += MT) {
-    const int q = x / n, r = x - q * n;
-    U[int64_t(q0 + q) * n + r] = Zs[r * BT_W + q];
+#pragma unroll
+  for (int r = 0; r < RM; ++r) {
+    const int i = lane + 32 * r;
+    if (i < n) {
+      U[int64_t(q0) * n + i] = z0[r];
+      if (two) U[int64_t(q0 + 1) * n + i] = z1[r];
+    }
   }
 }
 
 }  // namespace
 
 int64_t syevt_mid_workspace(int n, int k) { return mid_vec_workspace(n, k); }
-int syevt_mid_gram_limit(int max_n) { return mid_vec_kg(max_n); }
 
 void launch_trid_mid_vectors(cudaStream_t s, double* base, const TridTask* tasks, int ntasks,
                              int max_n, int max_k, double* xws) {
   if (ntasks <= 0) return;
-  // the Gram matrix in shared memory only when every task's fits (callers split the tasks)
-  const int kg = max_k <= mid_vec_kg(max_n) ? max_k : 0;
-  const size_t sm = mid_vec_smem_k(max_n, max_k, kg > 0);
-  raise_smem_limit(reinterpret_cast<const void*>(k_trid_mid_vectors), sm);
-  launch_k(k_trid_mid_vectors, ntasks, MT, sm, s, base, tasks, xws, kg);
-  count_launch();
-  const int nblk = max_n >= 3 ? (max_n - 2 + MID_BT_NB - 1) / MID_BT_NB : 0;
-  const size_t sb = sizeof(double) * (size_t(max_n) * BT_W + 2 * MID_BT_NB * BT_W +
-                                      size_t(nblk) * 64 + NW * 64);
-  raise_smem_limit(reinterpret_cast<const void*>(k_trid_mid_backtransform), sb);
-  const dim3 grid(ntasks, (max_k + BT_W - 1) / BT_W);
-  launch_k(k_trid_mid_backtransform, grid, MT, sb, s, base, tasks, xws);
-  count_launch();
+  launch_k(k_mid_invit, dim3((max_k + 31) / 32, ntasks), 32, sizeof(double) * 2 * size_t(max_n), s,
+           base, tasks, xws);
+  launch_k(k_mid_runs, ntasks, RUN_THREADS, 0, s, base, tasks, xws);
+  const int nt = (max_k + 31) / 32;
+  const size_t sa = sizeof(double) * AR * size_t(max_k);
+  raise_smem_limit(reinterpret_cast<const void*>(k_mid_apply), sa);
+  for (int pass = 0; pass < 3; ++pass) {
+    launch_k(k_mid_gram, dim3(nt * (nt + 1) / 2, ntasks), GT, 0, s, base, tasks, xws, pass);
+    launch_k(k_mid_apply, dim3((max_n + AR - 1) / AR, ntasks), GT, sa, s, base, tasks, xws, pass);
+  }
+  const int kg = mid_vec_kg();
+  const size_t sm = std::max(mid_vec_smem_k(std::min(max_k, kg), true), mid_vec_smem_k(max_k, false));
+  raise_smem_limit(reinterpret_cast<const void*>(k_mid_cholqr), sm);
+  launch_k(k_mid_cholqr, ntasks, MT, sm, s, base, tasks, xws, kg);
+  const dim3 gb((max_k + 2 * BW - 1) / (2 * BW), ntasks);
+  if (max_n <= 160) launch_k(k_mid_back<5>, gb, 32 * BW, 0, s, base, tasks, xws);
+  else if (max_n <= 256) launch_k(k_mid_back<8>, gb, 32 * BW, 0, s, base, tasks, xws);
+  else if (max_n <= 352) launch_k(k_mid_back<11>, gb, 32 * BW, 0, s, base, tasks, xws);
+  else launch_k(k_mid_back<16>, gb, 32 * BW, 0, s, base, tasks, xws);
+  count_launch(10);
 }
 
 }  // namespace dmrg
