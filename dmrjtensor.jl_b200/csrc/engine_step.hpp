@@ -106,7 +106,8 @@ struct Group {
 };
 
 // The reduced density matrix of every group (rows: M M^T, else M^T M), its eigenvalues
-// (tridiagonal path up to SYEVT_MID_NMAX, block Jacobi above), and their download.
+// (tridiagonal path up to SYEVT_MID_NMAX or SYEVT_RESOLVE_NMAX, block Jacobi above), and their
+// download.
 // c->R layout: [rho | eigenvalues | d,e,tau | eigenvectors | block-Jacobi workspace].
 struct RhoSolve {
   bool rows = true;
@@ -119,7 +120,8 @@ struct RhoSolve {
 };
 // Host plan: group offsets (moff, roff, woff), eigen tasks, the rho GEMM list; ensures c->M and
 // c->R. eig_max_n: the largest block.
-void plan_rho(dmrg_ctx* c, std::vector<Group>& G, bool rows, RhoSolve& rs, int* eig_max_n);
+void plan_rho(dmrg_ctx* c, std::vector<Group>& G, bool rows, const dmrg_params& P, RhoSolve& rs,
+              int* eig_max_n);
 // Launches (after the group matrices are in c->M and grho is uploaded at db): rho, eigenvalues,
 // and the asynchronous eigenvalue download into c->h_lam.
 void launch_rho(dmrg_ctx* c, RhoSolve& rs, char* db);

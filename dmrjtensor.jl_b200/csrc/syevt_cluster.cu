@@ -14,6 +14,8 @@
 //     order (bit-identical in all CTAs). The reflector stays unscaled (x, with v = s x and
 //     v_first = 1) until its norm is known: an extra warp sums the squares and takes the root
 //     and the reciprocal while the others sweep their columns and exchange messages.
+// Blocks above HN = 512 rows start in k_trid_lead, a cluster of 16 CTAs that takes the same steps
+// on the matrix in global memory (L2-resident) until 512 or fewer rows are left.
 // What bounds it: the latency of a step's chain (sweep, warp sums, message, elementwise update:
 // ~1,500 cycles for small blocks, ~2,500 at n = 345) and the issue rate of the two warps per
 // scheduler, not bandwidth or arithmetic. Fewer warps with more columns each beat more warps: the
@@ -31,7 +33,7 @@ namespace {
 
 constexpr int HW = 7;                // column warps per CTA
 constexpr int HT = 32 * HW;          // threads of the column warps
-constexpr int HN = 512;              // largest block
+constexpr int HN = 512;              // largest block of k_trid_cluster
 constexpr int HTX = HT + 32;         // and of the reflector warp
 // Bit pattern (a NaN) that k_trid_cluster leaves in d[0] when a wait gave up.
 constexpr long long TRID_GAVE_UP = 0x7ff8000000d06e0fLL;
@@ -109,6 +111,181 @@ __device__ __forceinline__ double wsum_cols(const double (&s)[N], int lane) {
   }
 }
 
+constexpr int LC = 16;               // CTAs of k_trid_lead's cluster
+constexpr int LT = 512;              // threads of each
+constexpr int LWARPS = LT / 32;
+constexpr int LCOLS = 4;             // columns per warp and sweep
+
+// First column that k_trid_cluster takes (a multiple of 32, so that both kernels store reflectors
+// from the same 32-row boundaries).
+__host__ __device__ __forceinline__ int trid_lead_steps(int n) {
+  return n <= HN ? 0 : (n - HN + 31) / 32 * 32;
+}
+
+__device__ __forceinline__ void peer_store(unsigned addr, double a, double b) {
+  asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" :: "r"(addr), "d"(a), "d"(b) : "memory");
+}
+__device__ __forceinline__ void peer_store(unsigned addr, double a) {
+  asm volatile("st.shared::cluster.f64 [%0], %1;" :: "r"(addr), "d"(a) : "memory");
+}
+
+template <int N, int MASK>
+__device__ __forceinline__ double wsum_cols(const double (&s)[N], int lane);
+
+// The first trid_lead_steps(n) Householder steps of a block above HN rows: columns dealt cyclically
+// to the CTAs, four per warp and sweep; each sweep applies the previous step's rank-2 update,
+// stores, and multiplies by the new reflector (unscaled, as in k_trid_cluster). One cluster
+// barrier per step. Bound by the L2 bandwidth of 16 SMs: the trailing block is read and written
+// once a step.
+__global__ void __launch_bounds__(LT, 1)
+k_trid_lead(double* __restrict__ base, const TridTask* __restrict__ tasks) {
+  grid_entry();
+  const TridTask tk = tasks[blockIdx.x / LC];
+  const int n = tk.n, ks = trid_lead_steps(n);
+  if (ks == 0) return;                     // the same in every CTA of the cluster
+  const int rank = cluster_rank();
+  extern __shared__ __align__(16) double sm[];
+  double2* pc = reinterpret_cast<double2*>(sm);   // 2 x n: (x.B(:,j), pivot-row element j)
+  double* xb = sm + 4 * size_t(n);         // 2 x n: unscaled reflectors, by parity
+  double* w = xb + 2 * size_t(n);          // n
+  __shared__ double kw[2][LC * LWARPS];    // shares of x.B x, every warp of every CTA
+  __shared__ double red[LWARPS];
+  __shared__ double s_alpha;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  double* Ag = base + tk.a_off;
+  double* ws = base + tk.ws_off;           // d | e | tau
+  const bool head = rank == 0;
+
+  double part = 0.0;
+  for (int i = tid; i < n; i += LT) {
+    const double a = Ag[i];
+    xb[i] = i >= 2 ? a : 0.0;
+    xb[n + i] = 0.0;
+    w[i] = 0.0;
+    if (i >= 2) part += a * a;
+    if (i == 1) s_alpha = a;
+    if (i == 0 && head) ws[0] = a;
+  }
+  part = wsum(part);
+  if (lane == 0) red[warp] = part;
+  cluster_sync_all();                      // every CTA runs before any remote store
+
+  double sc_p = 0.0, tau = 0.0, sc = 0.0, first = 0.0;   // first: the reflector's first element
+  auto reflect = [&](int k) {              // reflector k's scalars, and the reflector into column k
+    double t[LWARPS];
+#pragma unroll
+    for (int q = 0; q < LWARPS; ++q) t[q] = red[q];
+#pragma unroll
+    for (int h = LWARPS / 2; h > 0; h >>= 1)
+#pragma unroll
+      for (int q = 0; q < h; ++q) t[q] += t[q + h];
+    const double alpha = s_alpha;
+    double beta = alpha;
+    tau = 0.0;
+    sc = 0.0;
+    first = 0.0;
+    if (t[0] != 0.0) {
+      beta = -copysign(sqrt(fma(alpha, alpha, t[0])), alpha);
+      tau = (beta - alpha) / beta;
+      first = alpha - beta;
+      sc = 1.0 / first;
+    }
+    if (head && tid == 0) { ws[n + k] = beta; ws[2 * n + k] = tau; }
+    if (rank == k % LC) {
+      const double* x = xb + (k & 1) * n;
+      for (int i = (k & ~31) + tid; i < n; i += LT)
+        Ag[int64_t(k) * n + i] = i > k + 1 ? x[i] * sc : (i == k + 1 ? 1.0 : 0.0);
+    }
+  };
+  // columns j >= f of this CTA: pending update, and (dot) the product with x
+  auto sweep = [&](int f, const double* x, const double* xp, bool dot, double2* pck) {
+    const int s0 = (f - rank + LC - 1) / LC, i0 = f & ~31;
+    double kpart = 0.0;
+    for (int s = s0 + warp; s * LC + rank < n; s += LCOLS * LWARPS) {
+      double* col[LCOLS];
+      double wj[LCOLS], xj[LCOLS], acc[LCOLS];
+      const int jl = s * LC + rank;
+      const int nq = min(LCOLS, (n - jl + LC * LWARPS - 1) / (LC * LWARPS));
+#pragma unroll
+      for (int q = 0; q < LCOLS; ++q) {
+        const int j = jl + (q < nq ? q : 0) * LC * LWARPS;   // a missing column repeats the first
+        col[q] = Ag + int64_t(j) * n;
+        wj[q] = -sc_p * w[j];
+        xj[q] = -sc_p * xp[j];
+        acc[q] = 0.0;
+      }
+#pragma unroll 4
+      for (int i = i0 + lane; i < n; i += 32) {
+        const bool live = i >= f;
+        const double xi = x[i], xpi = xp[i], wi = w[i];
+        double v[LCOLS];
+#pragma unroll
+        for (int q = 0; q < LCOLS; ++q) v[q] = col[q][i];
+#pragma unroll
+        for (int q = 0; q < LCOLS; ++q) {
+          v[q] = fma(wi, xj[q], fma(xpi, wj[q], v[q]));
+          if (live && q < nq) col[q][i] = v[q];
+          if (live) acc[q] = fma(v[q], xi, acc[q]);
+        }
+      }
+      if (dot) {
+        const double dt = wsum_cols<LCOLS, 1>(acc, lane);
+        __syncwarp();
+        const int q = lane & 3, j = jl + q * LC * LWARPS;
+        if (j < n) {
+          kpart += dt * x[j];
+          const double piv = Ag[int64_t(j) * n + f];
+          const unsigned dst = smem_addr(&pck[j]);
+          for (int r = lane >> 2; r < LC; r += 8) peer_store(peer_addr(dst, r), dt, piv);
+        }
+      }
+    }
+    return kpart;
+  };
+  reflect(0);
+  for (int k = 0; k < ks; ++k) {
+    const int par = k & 1, f = k + 1;
+    const double* x = xb + par * n;                // reflector k, x[k+1] = 0
+    double* xn = xb + (par ^ 1) * n;               // reflector k-1, then k+1
+    double2* pck = pc + size_t(par) * n;
+    double kpart = sweep(f, x, xn, true, pck);
+    kpart += __shfl_xor_sync(FULL, kpart, 1);
+    kpart += __shfl_xor_sync(FULL, kpart, 2);
+    if (lane < LC) peer_store(peer_addr(smem_addr(&kw[par][rank * LWARPS + warp]), lane), kpart);
+    cluster_sync_all();
+    double K = 0.0;
+#pragma unroll
+    for (int q = 0; q < LC * LWARPS / 32; ++q) K += kw[par][lane + 32 * q];
+    K = wsum(K);
+    const double2 pf = pck[f];
+    const double hk = 0.5 * tau * (tau * fma(sc, fma(sc, K, 2.0 * pf.x), pf.y));
+    const double w0 = tau * fma(sc, pf.x, pf.y) - hk;
+    part = 0.0;
+    for (int i = f + tid; i < n; i += LT) {
+      const double2 pi = pck[i];
+      const double vi = i == f ? 1.0 : sc * x[i];
+      const double wi = tau * fma(sc, pi.x, pi.y) - hk * vi;
+      const double ci = pi.y - fma(vi, w0, wi);
+      w[i] = wi;
+      xn[i] = i >= f + 2 ? ci : 0.0;
+      if (i >= f + 2) part = fma(ci, ci, part);
+      if (i == f && head) ws[f] = ci;              // d[k+1]
+      if (i == f + 1) s_alpha = ci;
+    }
+    part = wsum(part);
+    if (lane == 0) red[warp] = part;
+    __syncthreads();
+    sc_p = sc;
+    if (k + 1 < ks) reflect(f);
+  }
+  // the pending update of step ks - 1, its pivot row included, so that the trailing block is a
+  // problem of its own
+  if (tid == 0) xb[((ks - 1) & 1) * n + ks] = first;
+  __syncthreads();
+  sweep(ks, xb + (ks & 1) * n, xb + ((ks - 1) & 1) * n, false, pc);
+  cluster_sync_all();                      // no CTA leaves before the others have read its stores
+}
+
 template <int V>
 struct Lo {
   static constexpr int v = V;
@@ -122,11 +299,11 @@ k_trid_cluster(double* __restrict__ base, const TridTask* __restrict__ tasks) {
   constexpr int G = CC <= 1 ? 1 : (CC <= 2 ? 2 : (CC <= 4 ? 4 : 8));   // lanes per column group
   constexpr int EPT = (32 * RM + HTX - 1) / HTX;          // elements per thread
   const TridTask tk = tasks[blockIdx.x / C];
-  const int n = tk.n;
+  const int k0 = trid_lead_steps(tk.n), ld = tk.n, n = ld - k0;   // the block from column k0 on
   if (n < 3 || n > 32 * RM || n > HW * CC * C) return;   // the same in all of the cluster
   __shared__ __align__(16) double2 pc[2][HN];      // (x.B(:,j), pivot-row element j), by parity
-  __shared__ __align__(16) double kw[2][C];     // the CTAs' shares of x.B x
-  __shared__ __align__(16) double kp[HW + 1];          // the warps' shares
+  __shared__ __align__(16) double kw[2][C];        // the CTAs' shares of x.B x
+  __shared__ __align__(16) double kp[HW + 1];      // the warps' shares
   __shared__ double s_pv[HW][CC];                  // the warps' pivot-row elements
   __shared__ double xb[2][HN];                     // unscaled reflectors, by parity
   __shared__ double w[HN];
@@ -134,8 +311,8 @@ k_trid_cluster(double* __restrict__ base, const TridTask* __restrict__ tasks) {
   __shared__ __align__(8) unsigned long long mbar[2];
   const int rank = cluster_rank();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  double* Ag = base + tk.a_off;
-  double* ws = base + tk.ws_off;                   // d | e | tau
+  double* Ag = base + tk.a_off + int64_t(k0) * (ld + 1);
+  double* ws = base + tk.ws_off + k0;              // d | e | tau, ld apart
   const bool head = rank == 0;
   const unsigned bar0 = smem_addr(&mbar[0]);
 
@@ -147,7 +324,7 @@ k_trid_cluster(double* __restrict__ base, const TridTask* __restrict__ tasks) {
 #pragma unroll
     for (int r = 0; r < RM; ++r) {
       const int i = lane + 32 * r;
-      a[q][r] = (jc[q] < n && i < n) ? Ag[int64_t(jc[q]) * n + i] : 0.0;
+      a[q][r] = (jc[q] < n && i < n) ? Ag[int64_t(jc[q]) * ld + i] : 0.0;
     }
   }
   double xi[EPT];                                  // this thread's elements of the reflector
@@ -197,9 +374,12 @@ k_trid_cluster(double* __restrict__ base, const TridTask* __restrict__ tasks) {
         sv = 1.0 / (al - be);
       }
       if (lane == 0) { s_tau = t; s_sc = sv; }
-      if (head && lane == 0) { ws[n + k] = be; ws[2 * n + k] = t; }
-      if (rank == k % C)                           // reflector tail, below the subdiagonal
-        for (int i = f + 1 + lane; i < n; i += 32) Ag[int64_t(k) * n + i] = x[i] * sv;
+      if (head && lane == 0) { ws[ld + k] = be; ws[2 * ld + k] = t; }
+      // reflector k, its unit entry and the zeros above it in its first 32 rows included: the
+      // back-transformation reads whole 32-row chunks of column k
+      if (rank == k % C)
+        for (int i = (k & ~31) + lane; i < n; i += 32)
+          Ag[int64_t(k) * ld + i] = i > f ? x[i] * sv : (i == f ? 1.0 : 0.0);
     } else {
       if (tid == 0)
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
@@ -300,7 +480,7 @@ k_trid_cluster(double* __restrict__ base, const TridTask* __restrict__ tasks) {
         if (i == f && head) ws[f] = ci;          // d[k+1]
         if (i == f + 1) {
           s_alpha = ci;
-          if (head && k + 3 == n) ws[n + n - 2] = ci;
+          if (head && k + 3 == n) ws[ld + n - 2] = ci;
         }
       }
     }
@@ -321,15 +501,15 @@ k_trid_cluster(double* __restrict__ base, const TridTask* __restrict__ tasks) {
             ws[n - 1] = a[q][r] - 2.0 * (sc_p * xb[(n - 3) & 1][n - 1]) * w[n - 1];
       }
     if (head && tid == 0) {
-      ws[n + n - 1] = 0.0;
-      ws[2 * n + n - 2] = 0.0;
-      ws[2 * n + n - 1] = 0.0;
+      ws[ld + n - 1] = 0.0;
+      ws[2 * ld + n - 2] = 0.0;
+      ws[2 * ld + n - 1] = 0.0;
     }
   } else {
     for (int r = 0; r < 1000; ++r) __nanosleep(1000);   // messages still in flight land
   }
   cluster_sync_all();                              // no CTA leaves before the others are done
-  if (!ok && tid == 0) ws[0] = __longlong_as_double(TRID_GAVE_UP);
+  if (!ok && tid == 0) ws[-k0] = __longlong_as_double(TRID_GAVE_UP);
 }
 
 constexpr int CT = 64;               // threads of k_trid_sturm
@@ -424,6 +604,13 @@ bool trid_gave_up(double w) {
 void launch_trid_cluster(cudaStream_t s, double* base, const TridTask* tasks, int ntasks,
                          int max_n, int64_t sum_n) {
   if (ntasks <= 0) return;
+  if (max_n > HN) {                    // such blocks come first
+    const size_t sl = sizeof(double) * 7 * size_t(max_n);
+    raise_smem_limit(reinterpret_cast<const void*>(k_trid_lead), sl);
+    allow_wide_clusters(reinterpret_cast<const void*>(k_trid_lead));
+    launch_cluster_k(k_trid_lead, LC, ntasks * LC, LT, sl, s, base, tasks);
+    count_launch();
+  }
   auto go = [&](auto kernel, int c) {
     allow_wide_clusters(reinterpret_cast<const void*>(kernel));
     launch_cluster_k(kernel, c, ntasks * c, HTX, 0, s, base, tasks);

@@ -88,120 +88,131 @@ __device__ double bsum(double v, double* red) {
 }
 
 // LU factors of one solver thread in shared memory: element k at [k * stride] (threads
-// interleaved, so that neighbouring threads touch neighbouring words).
+// interleaved, so that neighbouring threads touch neighbouring words). U has two superdiagonals;
+// the second is e[k+1] where rows were swapped and zero elsewhere, so it is not stored.
 struct LUSlot {
-  double *u0, *u1, *u2, *l;
+  double *u0, *u1, *l;     // reciprocal pivots, first superdiagonal, multipliers
   int* piv;
   int stride;
 };
 
-// One thread: z <- (T - lam I)^{-1} z twice (with lam good to the last bits the first solve leaves
-// other eigenvectors at ~1e-16 ||T|| / gap and the second squares that; a third only turns the
-// vectors of equal eigenvalues towards each other: the worst residual of degenerate test blocks
-// fell from 5e-13 to 3e-14 without it), z = column col of the row-major Z (leading
-// dimension ldz). The solves run in groups of 8 steps whose loads are issued first, so that only
-// the arithmetic recurrence is on the dependent chain.
+// One thread: the vector of (T - lam I)^{-1} applied twice to the pseudo-random start vector of
+// column col, normalised, into z (element r at z[r * zs]). With lam good to the last bits the
+// first solve leaves other eigenvectors at ~1e-16 ||T|| / gap and the second squares that; a third
+// only turns the vectors of equal eigenvalues towards each other (the worst residual of degenerate
+// test blocks fell from 5e-13 to 3e-14 without it). The factorisation carries the first forward
+// solve along and takes one reciprocal a step, for either pivot; the solves run in groups of 8
+// steps whose loads are issued first; the normalisation is applied in the next pass. What bounds it is the chain of dependent steps: ~115 cycles for a factorisation
+// step (the reciprocal), ~25 for a solve step.
 __device__ void inverse_iteration(const double* __restrict__ d, const double* __restrict__ e, int n,
-                                  double lam, double* Z, int ldz, int col, double tn, LUSlot f) {
+                                  double lam, double* z, int zs, int col, double tn, LUSlot f) {
   const int S = f.stride;
-  // factor (T - lam I) = P L U with U having two superdiagonals; u0 keeps reciprocal pivots
   const double pert = 2.2e-16 * tn;
   double dk = d[0] - lam, ek = n > 1 ? e[0] : 0.0;
+  double zk = prand(0, col);
+#pragma unroll 4
   for (int k = 0; k + 1 < n; ++k) {
     const double sub = e[k];                  // T(k+1, k)
     const double dn = d[k + 1] - lam;
     const double en = (k + 2 < n) ? e[k + 1] : 0.0;
-    if (fabs(dk) >= fabs(sub)) {              // no swap
-      const double r = 1.0 / ((dk == 0.0) ? pert : dk);
-      const double lk = sub * r;
-      f.u0[k * S] = r; f.u1[k * S] = ek; f.u2[k * S] = 0.0; f.piv[k * S] = 0; f.l[k * S] = lk;
-      dk = dn - lk * ek;
-      ek = en;
-    } else {                                  // swap rows k and k+1
-      const double r = 1.0 / sub;
-      const double lk = dk * r;
-      f.u0[k * S] = r; f.u1[k * S] = dn; f.u2[k * S] = en; f.piv[k * S] = 1; f.l[k * S] = lk;
-      dk = ek - lk * dn;
-      ek = -lk * en;
-    }
+    const bool sw = fabs(dk) < fabs(sub);     // swap rows k and k+1
+    const double r = 1.0 / (sw ? sub : (dk == 0.0 ? pert : dk));
+    const double lk = (sw ? dk : sub) * r;
+    const double u1 = sw ? dn : ek;
+    f.u0[k * S] = r;
+    f.u1[k * S] = u1;
+    f.l[k * S] = lk;
+    f.piv[k * S] = sw;
+    dk = fma(-lk, u1, sw ? ek : dn);
+    ek = sw ? -lk * en : en;
+    const double zr = prand(k + 1, col);
+    const double zt = sw ? zr : zk;           // row k of P z
+    z[k * zs] = zt;
+    zk = fma(-lk, zt, sw ? zk : zr);
   }
   f.u0[(n - 1) * S] = 1.0 / ((dk == 0.0) ? pert : dk);
-  f.u1[(n - 1) * S] = 0.0; f.u2[(n - 1) * S] = 0.0; f.piv[(n - 1) * S] = 0;
-  double* z = Z + col;                        // z[r] at z[r * ldz]
+  f.u1[(n - 1) * S] = 0.0;
+  f.piv[(n - 1) * S] = 0;
+  z[(n - 1) * zs] = zk;
+  double inv = 1.0;
   for (int it = 0; it < 2; ++it) {
-    // solve P L y = z; z[k] is carried in a register. Loads of a group precede its stores, and
-    // every store goes below the indices still to be loaded.
-    double zk = z[0];
-    int k = 0;
-    for (; k + 8 < n; k += 8) {
-      double zz[8], ll[8];
-      int pp[8];
+    if (it > 0) {
+      // solve P L y = inv z; z[k] is carried in a register. Loads of a group precede its stores,
+      // and every store goes below the indices still to be loaded.
+      zk = inv * z[0];
+      int k = 0;
+      for (; k + 8 < n; k += 8) {
+        double zz[8], ll[8];
+        int pp[8];
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        zz[q] = z[(k + 1 + q) * ldz];
-        ll[q] = f.l[(k + q) * S];
-        pp[q] = f.piv[(k + q) * S];
-      }
+        for (int q = 0; q < 8; ++q) {
+          zz[q] = inv * z[(k + 1 + q) * zs];
+          ll[q] = f.l[(k + q) * S];
+          pp[q] = f.piv[(k + q) * S];
+        }
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        double zn = zz[q];
-        if (pp[q]) { const double tt = zk; zk = zn; zn = tt; }
-        zn -= ll[q] * zk;
-        z[(k + q) * ldz] = zk;
-        zk = zn;
+        for (int q = 0; q < 8; ++q) {
+          const double zt = pp[q] ? zz[q] : zk;
+          z[(k + q) * zs] = zt;
+          zk = fma(-ll[q], zt, pp[q] ? zk : zz[q]);
+        }
       }
+      for (; k + 1 < n; ++k) {
+        const double zn = inv * z[(k + 1) * zs];
+        const bool sw = f.piv[k * S];
+        const double zt = sw ? zn : zk;
+        z[k * zs] = zt;
+        zk = fma(-f.l[k * S], zt, sw ? zk : zn);
+      }
+      z[(n - 1) * zs] = zk;
     }
-    for (; k + 1 < n; ++k) {
-      double zn = z[(k + 1) * ldz];
-      if (f.piv[k * S]) { const double tt = zk; zk = zn; zn = tt; }
-      zn -= f.l[k * S] * zk;
-      z[k * ldz] = zk;
-      zk = zn;
-    }
-    z[(n - 1) * ldz] = zk;
     // solve U x = y (x[k+1], x[k+2] carried in registers)
     double x1 = 0.0, x2 = 0.0;
-    k = n - 1;
+    int k = n - 1;
     for (; k >= 7; k -= 8) {
       double zz[8], a0[8], a1[8], a2[8];
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
-        zz[q] = z[(k - q) * ldz];
+        zz[q] = z[(k - q) * zs];
         a0[q] = f.u0[(k - q) * S];
         a1[q] = f.u1[(k - q) * S];
-        a2[q] = f.u2[(k - q) * S];
+        a2[q] = f.piv[(k - q) * S] && k - q + 2 < n ? e[k - q + 1] : 0.0;
       }
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
-        const double xk = (zz[q] - a1[q] * x1 - a2[q] * x2) * a0[q];
-        z[(k - q) * ldz] = xk;
+        const double xk = fma(-a2[q], x2, fma(-a1[q], x1, zz[q])) * a0[q];
+        z[(k - q) * zs] = xk;
         x2 = x1;
         x1 = xk;
       }
     }
     for (; k >= 0; --k) {
-      const double xk = (z[k * ldz] - f.u1[k * S] * x1 - f.u2[k * S] * x2) * f.u0[k * S];
-      z[k * ldz] = xk;
+      const double a2 = f.piv[k * S] && k + 2 < n ? e[k + 1] : 0.0;
+      const double xk = fma(-a2, x2, fma(-f.u1[k * S], x1, z[k * zs])) * f.u0[k * S];
+      z[k * zs] = xk;
       x2 = x1;
       x1 = xk;
     }
     double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
     int i = 0;
+#pragma unroll 2
     for (; i + 4 <= n; i += 4) {
-      s0 += z[i * ldz] * z[i * ldz];
-      s1 += z[(i + 1) * ldz] * z[(i + 1) * ldz];
-      s2 += z[(i + 2) * ldz] * z[(i + 2) * ldz];
-      s3 += z[(i + 3) * ldz] * z[(i + 3) * ldz];
+      s0 = fma(z[i * zs], z[i * zs], s0);
+      s1 = fma(z[(i + 1) * zs], z[(i + 1) * zs], s1);
+      s2 = fma(z[(i + 2) * zs], z[(i + 2) * zs], s2);
+      s3 = fma(z[(i + 3) * zs], z[(i + 3) * zs], s3);
     }
-    for (; i < n; ++i) s0 += z[i * ldz] * z[i * ldz];
+    for (; i < n; ++i) s0 = fma(z[i * zs], z[i * zs], s0);
     const double nr = sqrt((s0 + s1) + (s2 + s3));
     if (nr == 0.0) {
-      for (int r = 0; r < n; ++r) z[r * ldz] = prand(r, col + 7 * it);
-      continue;
+      for (int r = 0; r < n; ++r) z[r * zs] = prand(r, col + 7 * (it + 1));
+      inv = 1.0;
+    } else {
+      inv = 1.0 / nr;
     }
-    const double inv = 1.0 / nr;
-    for (int r = 0; r < n; ++r) z[r * ldz] *= inv;
   }
+#pragma unroll 8
+  for (int r = 0; r < n; ++r) z[r * zs] *= inv;
 }
 
 }  // namespace

@@ -1,9 +1,9 @@
 // syevt_mid.cu -- eigenvectors of mid-size density-matrix blocks, SYEVT_NMAX < n <= SYEVT_MID_NMAX
 // (their tridiagonal matrices and eigenvalues come from syevt_cluster.cu). Every part runs on many
 // CTAs; one CTA per block for all of it took 1.6 + 0.54 ms at n = 345 with 200 kept vectors.
-//   * k_mid_invit: inverse iteration, one thread per kept vector, one warp per CTA; LU factors in
-//     a global workspace interleaved by thread, so that a warp's accesses to one factor element
-//     form one line. Bound by the latency of the recurrences.
+//   * k_mid_invit: inverse iteration, one thread per kept vector, a few vectors per CTA so that
+//     their LU factors and the vectors stay in shared memory (with 32 vectors per CTA and the
+//     factors in global memory 290 us at n = 345). Bound by the latency of the recurrences.
 //   * k_mid_runs: vectors of (nearly) equal eigenvalues, which come out as independent but not
 //     orthogonal vectors of their common eigenspace, are orthonormalised among themselves.
 //   * up to three rounds of k_mid_gram and k_mid_apply: G = Z^T Z = I + E with a small E (vectors
@@ -14,8 +14,8 @@
 //   * k_mid_cholqr: blocks that round zero cannot treat (long runs of equal or numerically zero
 //     eigenvalues, nearly dependent vectors) take the Cholesky QR or Gram-Schmidt of one CTA; it
 //     returns at once for all others.
-//   * k_mid_back: U = H_0 ... H_{n-3} Z, two vectors per warp in registers, the reflectors read
-//     from the matrix in global memory two at a time, one pair ahead.
+//   * k_mid_back: U = H_0 ... H_{n-3} Z, two vectors per warp in registers, the reflectors two at
+//     a time through a shared-memory ring.
 #include <algorithm>
 
 #include "kernels.cuh"
@@ -29,18 +29,13 @@ constexpr int MT = 512;             // threads per CTA
 constexpr int NW = MT / 32;         // warps
 constexpr size_t MID_SMEM_LIMIT = 227 * 1024 - 2048;
 
-// Workspace of one task, in doubles from x_off: LU factors (4 n k), pivots (n k ints), Z (n x
-// (k|1), row-major), Gram matrix (k x k, row-major, upper triangle), control words.
+// Workspace of one task, in doubles from x_off: Z (n x (k|1), row-major), Gram matrix (k x k,
+// row-major, upper triangle), control words.
 struct MidCtl {
   unsigned long long emax[3];   // largest |E| of each round (bits of a non-negative double)
   unsigned long long slow;      // set: the block goes to k_mid_cholqr
 };
-__host__ __device__ inline int64_t mid_z_off(int n, int k) {
-  return 4 * int64_t(n) * k + (int64_t(n) * k + 1) / 2;
-}
-__host__ __device__ inline int64_t mid_g_off(int n, int k) {
-  return mid_z_off(n, k) + int64_t(n) * (k | 1);
-}
+__host__ __device__ inline int64_t mid_g_off(int n, int k) { return int64_t(n) * (k | 1); }
 __host__ __device__ inline int64_t mid_vec_workspace(int n, int k) {
   return mid_g_off(n, k) + int64_t(k) * k + 8;
 }
@@ -48,31 +43,43 @@ __device__ __forceinline__ MidCtl* mid_ctl(double* X, int n, int k) {
   return reinterpret_cast<MidCtl*>(X + mid_g_off(n, k) + int64_t(k) * k);
 }
 
-// ---- inverse iteration: one warp per CTA, blockIdx.x = group of 32 vectors, blockIdx.y = task
+// ---- inverse iteration: `lanes` vectors per CTA (the first lanes of its one warp), blockIdx.x =
+// group of vectors, blockIdx.y = task
 __global__ void __launch_bounds__(32)
 k_mid_invit(double* __restrict__ base, const TridTask* __restrict__ tasks,
-            double* __restrict__ xws) {
+            double* __restrict__ xws, int lanes) {
   grid_entry();
   const TridTask tk = tasks[blockIdx.y];
-  const int n = tk.n, kk = tk.keep, j = blockIdx.x * 32 + threadIdx.x;
-  if (int(blockIdx.x) * 32 >= kk) return;
-  extern __shared__ double sm[];
-  double* d = sm;
-  double* e = sm + n;
+  const int n = tk.n, kk = tk.keep, lane = threadIdx.x, j0 = blockIdx.x * lanes, j = j0 + lane;
+  if (j0 >= kk) return;
+  extern __shared__ __align__(16) double sm[];
+  double* d = sm;                          // n
+  double* e = d + n;                       // n
+  double* F = e + n;                       // u0, u1, l, z: n x lanes each; pivots
   const double* ws = base + tk.ws_off;
   const double* W = base + tk.w_off;
-  for (int i = threadIdx.x; i < n; i += 32) { d[i] = ws[i]; e[i] = ws[n + i]; }
+  for (int i = lane; i < n; i += 32) { d[i] = ws[i]; e[i] = ws[n + i]; }
   __syncwarp();
-  if (j >= kk) return;
-  const double tn = fmax(fmax(fabs(W[0]), fabs(W[n - 1])), 1e-300);   // descending
-  double* X = xws + tk.x_off;
-  double* Z = X + mid_z_off(n, kk);
-  const int ldz = kk | 1;
-  LUSlot f{X + j, X + int64_t(n) * kk + j, X + 2 * int64_t(n) * kk + j,
-           X + 3 * int64_t(n) * kk + j, reinterpret_cast<int*>(X + 4 * int64_t(n) * kk) + j, kk};
-  for (int r = 0; r < n; ++r) Z[int64_t(r) * ldz + j] = prand(r, j);
-  // kept eigenvalues that are numerically zero keep the pseudo-random vector alone
-  if (W[j] > 1e-13 * tn) inverse_iteration(d, e, n, W[j], Z, ldz, j, tn, f);
+  const size_t nl = size_t(n) * lanes;
+  double* z = F + 3 * nl;
+  if (lane < lanes && j < kk) {
+    const double tn = fmax(fmax(fabs(W[0]), fabs(W[n - 1])), 1e-300);   // descending
+    LUSlot f{F + lane, F + nl + lane, F + 2 * nl + lane, reinterpret_cast<int*>(F + 4 * nl) + lane,
+             lanes};
+    // kept eigenvalues that are numerically zero keep the pseudo-random vector alone
+    if (W[j] > 1e-13 * tn) inverse_iteration(d, e, n, W[j], z + lane, lanes, j, tn, f);
+    else for (int r = 0; r < n; ++r) z[r * lanes + lane] = prand(r, j);
+  }
+  __syncwarp();
+  double* Z = xws + tk.x_off;
+  const int w = min(lanes, kk - j0), ldz = kk | 1;
+  for (int x = lane; x < n * lanes; x += 32) {
+    const int r = x / lanes, q = x - r * lanes;
+    if (q < w) Z[int64_t(r) * ldz + j0 + q] = z[x];
+  }
+}
+size_t invit_smem(int n, int lanes) {
+  return sizeof(double) * (2 * size_t(n) + 4 * size_t(n) * lanes) + sizeof(int) * size_t(n) * lanes;
 }
 
 // ---- runs of nearly equal eigenvalues (neighbours within 1e-12 ||T||): modified Gram-Schmidt
@@ -89,7 +96,7 @@ k_mid_runs(double* __restrict__ base, const TridTask* __restrict__ tasks,
   const double* W = base + tk.w_off;
   const double tol = 1e-12 * fmax(fmax(fabs(W[0]), fabs(W[n - 1])), 1e-300);
   double* X = xws + tk.x_off;
-  double* Z = X + mid_z_off(n, kk);
+  double* Z = X;
   MidCtl* ctl = mid_ctl(X, n, kk);
   const int ldz = kk | 1;
   if (threadIdx.x < 4) (threadIdx.x < 3 ? ctl->emax[threadIdx.x] : ctl->slow) = 0ull;
@@ -150,7 +157,7 @@ k_mid_gram(double* __restrict__ base, const TridTask* __restrict__ tasks, double
   double* X = xws + tk.x_off;
   MidCtl* ctl = mid_ctl(X, n, kk);
   if (!round_active(ctl, pass)) return;
-  const double* Z = X + mid_z_off(n, kk);
+  const double* Z = X;
   double* G = X + mid_g_off(n, kk);
   const int ldz = kk | 1;
   __shared__ double sa[32][33], sb[32][33];
@@ -206,8 +213,8 @@ k_mid_gram(double* __restrict__ base, const TridTask* __restrict__ tasks, double
     atomicMax(&ctl->emax[pass], (unsigned long long)(__double_as_longlong(mx)) & ~(1ull << 63));
 }
 
-// ---- Z <- Z (I - E_up), 16 rows per CTA (blockIdx.x; blockIdx.y = task)
-constexpr int AR = 16;
+// ---- Z <- Z (I - E_up), AR rows per CTA (blockIdx.x; blockIdx.y = task)
+template <int AR>
 __global__ void __launch_bounds__(GT)
 k_mid_apply(double* __restrict__ base, const TridTask* __restrict__ tasks,
             double* __restrict__ xws, int pass) {
@@ -224,7 +231,7 @@ k_mid_apply(double* __restrict__ base, const TridTask* __restrict__ tasks,
     if (threadIdx.x == 0) ctl->slow = 1ull;
     return;
   }
-  double* Z = X + mid_z_off(n, kk);
+  double* Z = X;
   const double* G = X + mid_g_off(n, kk);
   const int ldz = kk | 1;
   extern __shared__ __align__(16) double sm[];         // kk x AR: row r of the slab at [p * AR + r]
@@ -290,7 +297,7 @@ k_mid_cholqr(double* __restrict__ base, const TridTask* __restrict__ tasks,
   __shared__ double red[32];
   __shared__ int s_flag, s_need2;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  double* Z = X + mid_z_off(n, kk);                        // n x ldz
+  double* Z = X;                        // n x ldz
   double* G = X + mid_g_off(n, kk);                        // kk x kk row-major, upper triangle
   if (tid == 0) { s_flag = 0; s_need2 = 0; }
   __syncthreads();
@@ -509,73 +516,99 @@ __device__ __forceinline__ void wsum5(double (&s)[5], int lane) {
 
 // Back-transformation U = H_0 H_1 ... H_{n-3} Z: two kept vectors per warp in registers (lane l
 // has rows l, l + 32, ...), n <= 32 RM. Two reflectors per step, a = v_k and b = v_{k-1}: their
-// four products with the vectors and a.b are one warp sum, and the next pair is loaded before it.
-// Bound by that sum's latency (about 300 of 500 cycles a step): blocks of more reflectors would
-// add products that the two warps per scheduler have no free issue slots for.
-constexpr int BW = 4;                    // warps per CTA
-template <int RM>
+// four products with the vectors and a.b are one warp sum. The pairs come through a ring of
+// BSTAGES shared-memory stages, several steps ahead (cp.async): read straight from L2 one pair
+// ahead, a step waited for them (n = 345, 200 vectors: 191 us against 128 us).
+// Bound by the latency of the warp sum: blocks of more reflectors would add products that the two
+// warps per scheduler have no free issue slots for.
+constexpr int BW = 4, BSTAGES = 6;       // warps per CTA, stages of the ring
+template <int RM, int NV>                // NV vectors per warp
 __global__ void __launch_bounds__(32 * BW)
 k_mid_back(double* __restrict__ base, const TridTask* __restrict__ tasks,
            const double* __restrict__ xws) {
   grid_entry();
+  constexpr int LD = 32 * RM;
+  constexpr int KR = RM <= 16 ? RM : 1;          // reflectors kept in registers between their uses
   const TridTask tk = tasks[blockIdx.y];
-  const int n = tk.n, kk = tk.keep;
-  const int lane = threadIdx.x & 31, q0 = 2 * (blockIdx.x * BW + (threadIdx.x >> 5));
-  if (n < 3 || n > 32 * RM || q0 >= kk) return;
-  const bool two = q0 + 1 < kk;
+  const int n = tk.n, kk = tk.keep, tid = threadIdx.x, lane = tid & 31;
+  if (n < 3 || n > LD || int(blockIdx.x) * NV * BW >= kk) return;
+  extern __shared__ __align__(16) double sm[];
+  double* stau = sm + BSTAGES * 2 * LD;          // n
+  const int q0 = NV * (blockIdx.x * BW + (tid >> 5));
+  const bool one = q0 < kk, two = NV > 1 && q0 + 1 < kk;
   const int ldz = kk | 1;
-  const double* Z = xws + tk.x_off + mid_z_off(n, kk);
-  const double* V = base + tk.a_off;             // reflector k: V[k n + r], r > k + 1
+  const double* Z = xws + tk.x_off;
+  const double* V = base + tk.a_off;             // reflector k: V[k n + r], r >= 32 (k / 32)
   const double* tau = base + tk.ws_off + 2 * n;
-  double z0[RM], z1[RM], a[RM], b[RM];
-  double ta = 0.0, tb = 0.0;
-  auto load = [&](int k) {                       // the pair (k, k - 1)
-    ta = k >= 0 ? tau[k] : 0.0;
-    tb = k >= 1 ? tau[k - 1] : 0.0;
-#pragma unroll
-    for (int r = 0; r < RM; ++r) {
-      const int i = lane + 32 * r;
-      double va = 0.0, vb = 0.0;
-      if (32 * r + 31 >= k && i < n) {
-        if (k >= 0 && i >= k + 1) va = i == k + 1 ? 1.0 : V[int64_t(k) * n + i];
-        if (k >= 1 && i >= k) vb = i == k ? 1.0 : V[int64_t(k - 1) * n + i];
+  const int np = (n - 1) / 2;                    // pairs (k, k - 1), k = n - 3, n - 5, ...
+  auto fill = [&](int t) {
+    const int k = n - 3 - 2 * t;
+    if (t < np) {
+      double* st = sm + (t % BSTAGES) * 2 * LD;
+      for (int i = (k & ~31) + tid; i < n; i += 32 * BW) {
+        const unsigned da = unsigned(__cvta_generic_to_shared(st + i));
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" :: "r"(da), "l"(V + int64_t(k) * n + i));
+        if (k >= 1)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 8;"
+                       :: "r"(da + 8 * LD), "l"(V + int64_t(k - 1) * n + i));
       }
-      a[r] = va;
-      b[r] = vb;
     }
+    asm volatile("cp.async.commit_group;");
   };
+  // rows past the block stay zero in every stage
+  for (int x = tid; x < BSTAGES * 2 * LD; x += 32 * BW)
+    if (x % LD >= n) sm[x] = 0.0;
+  __syncthreads();
+  for (int t = 0; t < BSTAGES - 1; ++t) fill(t);
+  for (int i = tid; i < n; i += 32 * BW) stau[i] = i < n - 2 ? tau[i] : 0.0;
+  double z0[RM], z1[NV > 1 ? RM : 1];
 #pragma unroll
   for (int r = 0; r < RM; ++r) {
     const int i = lane + 32 * r;
-    z0[r] = i < n ? Z[int64_t(i) * ldz + q0] : 0.0;
-    z1[r] = i < n && two ? Z[int64_t(i) * ldz + q0 + 1] : 0.0;
+    z0[r] = i < n && one ? Z[int64_t(i) * ldz + q0] : 0.0;
+    if (NV > 1) z1[r] = i < n && two ? Z[int64_t(i) * ldz + q0 + 1] : 0.0;
   }
-  load(n - 3);
-  for (int k = n - 3; k >= 0; k -= 2) {
+  for (int t = 0; t < np; ++t) {
+    const int k = n - 3 - 2 * t;
+    asm volatile("cp.async.wait_group %0;" :: "n"(BSTAGES - 2) : "memory");
+    __syncthreads();                             // pair t is there, pair t - 1 is done with
+    fill(t + BSTAGES - 1);
+    if (!one) continue;
+    const double* st = sm + (t % BSTAGES) * 2 * LD + lane;
+    const double ta = stau[k], tb = k >= 1 ? stau[k - 1] : 0.0;   // tb = 0: no partner
     double s[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    double ca[RM], cb[RM];
-    const double cta = ta, ctb = tb;
+    double a[KR], b[KR];
+    if (KR == RM) {                              // all at once: rows above the pair's are not used
 #pragma unroll
-    for (int r = 0; r < RM; ++r) {
-      ca[r] = a[r];
-      cb[r] = b[r];
-      if (32 * r + 31 >= k) {
-        s[0] = fma(ca[r], z0[r], s[0]);
-        s[1] = fma(ca[r], z1[r], s[1]);
-        s[2] = fma(cb[r], z0[r], s[2]);
-        s[3] = fma(cb[r], z1[r], s[3]);
-        s[4] = fma(ca[r], cb[r], s[4]);
+      for (int r = 0; r < KR; ++r) {
+        a[r] = st[32 * r];
+        b[r] = st[LD + 32 * r];
       }
     }
-    load(k - 2);
-    wsum5(s, lane);
-    const double x0 = cta * s[0], x1 = cta * s[1];
-    const double y0 = ctb * fma(-x0, s[4], s[2]), y1 = ctb * fma(-x1, s[4], s[3]);
 #pragma unroll
     for (int r = 0; r < RM; ++r) {
-      if (32 * r + 31 >= k) {
-        z0[r] = fma(-y0, cb[r], fma(-x0, ca[r], z0[r]));
-        z1[r] = fma(-y1, cb[r], fma(-x1, ca[r], z1[r]));
+      if (32 * r + 31 >= k && 32 * r < n) {
+        const double av = KR == RM ? a[r % KR] : st[32 * r];
+        const double bv = KR == RM ? b[r % KR] : st[LD + 32 * r];
+        s[0] = fma(av, z0[r], s[0]);
+        s[2] = fma(bv, z0[r], s[2]);
+        if (NV > 1) {
+          s[1] = fma(av, z1[r], s[1]);
+          s[3] = fma(bv, z1[r], s[3]);
+        }
+        s[4] = fma(av, bv, s[4]);
+      }
+    }
+    wsum5(s, lane);
+    const double x0 = ta * s[0], x1 = ta * s[1];
+    const double y0 = tb * fma(-x0, s[4], s[2]), y1 = tb * fma(-x1, s[4], s[3]);
+#pragma unroll
+    for (int r = 0; r < RM; ++r) {
+      if (32 * r + 31 >= k && 32 * r < n) {
+        const double av = KR == RM ? a[r % KR] : st[32 * r];
+        const double bv = KR == RM ? b[r % KR] : st[LD + 32 * r];
+        z0[r] = fma(-y0, bv, fma(-x0, av, z0[r]));
+        if (NV > 1) z1[r] = fma(-y1, bv, fma(-x1, av, z1[r]));
       }
     }
   }
@@ -584,10 +617,18 @@ k_mid_back(double* __restrict__ base, const TridTask* __restrict__ tasks,
   for (int r = 0; r < RM; ++r) {
     const int i = lane + 32 * r;
     if (i < n) {
-      U[int64_t(q0) * n + i] = z0[r];
-      if (two) U[int64_t(q0 + 1) * n + i] = z1[r];
+      if (one) U[int64_t(q0) * n + i] = z0[r];
+      if (NV > 1 && two) U[int64_t(q0 + 1) * n + i] = z1[r];
     }
   }
+}
+template <int RM, int NV>
+void launch_back(cudaStream_t s, double* base, const TridTask* tasks, int ntasks, int max_n,
+                 int max_k, const double* xws) {
+  const size_t sm = sizeof(double) * (BSTAGES * 2 * 32 * RM + size_t(max_n));
+  raise_smem_limit(reinterpret_cast<const void*>(k_mid_back<RM, NV>), sm);
+  launch_k(k_mid_back<RM, NV>, dim3((max_k + NV * BW - 1) / (NV * BW), ntasks), 32 * BW, sm, s, base,
+           tasks, xws);
 }
 
 }  // namespace
@@ -597,25 +638,33 @@ int64_t syevt_mid_workspace(int n, int k) { return mid_vec_workspace(n, k); }
 void launch_trid_mid_vectors(cudaStream_t s, double* base, const TridTask* tasks, int ntasks,
                              int max_n, int max_k, double* xws) {
   if (ntasks <= 0) return;
-  launch_k(k_mid_invit, dim3((max_k + 31) / 32, ntasks), 32, sizeof(double) * 2 * size_t(max_n), s,
-           base, tasks, xws);
+  int lanes = 8;                           // 152 KB at n = 512
+  while (lanes > 1 && invit_smem(max_n, lanes) > MID_SMEM_LIMIT) lanes /= 2;
+  const size_t si = invit_smem(max_n, lanes);
+  raise_smem_limit(reinterpret_cast<const void*>(k_mid_invit), si);
+  launch_k(k_mid_invit, dim3((max_k + lanes - 1) / lanes, ntasks), 32, si, s, base, tasks, xws,
+           lanes);
   launch_k(k_mid_runs, ntasks, RUN_THREADS, 0, s, base, tasks, xws);
   const int nt = (max_k + 31) / 32;
-  const size_t sa = sizeof(double) * AR * size_t(max_k);
-  raise_smem_limit(reinterpret_cast<const void*>(k_mid_apply), sa);
+  const int ar = sizeof(double) * 16 * size_t(max_k) <= MID_SMEM_LIMIT ? 16 : 8;
+  const auto apply = ar == 16 ? k_mid_apply<16> : k_mid_apply<8>;
+  const size_t sa = sizeof(double) * ar * size_t(max_k);
+  raise_smem_limit(reinterpret_cast<const void*>(apply), sa);
   for (int pass = 0; pass < 3; ++pass) {
     launch_k(k_mid_gram, dim3(nt * (nt + 1) / 2, ntasks), GT, 0, s, base, tasks, xws, pass);
-    launch_k(k_mid_apply, dim3((max_n + AR - 1) / AR, ntasks), GT, sa, s, base, tasks, xws, pass);
+    launch_k(apply, dim3((max_n + ar - 1) / ar, ntasks), GT, sa, s, base, tasks, xws, pass);
   }
   const int kg = mid_vec_kg();
   const size_t sm = std::max(mid_vec_smem_k(std::min(max_k, kg), true), mid_vec_smem_k(max_k, false));
   raise_smem_limit(reinterpret_cast<const void*>(k_mid_cholqr), sm);
   launch_k(k_mid_cholqr, ntasks, MT, sm, s, base, tasks, xws, kg);
-  const dim3 gb((max_k + 2 * BW - 1) / (2 * BW), ntasks);
-  if (max_n <= 160) launch_k(k_mid_back<5>, gb, 32 * BW, 0, s, base, tasks, xws);
-  else if (max_n <= 256) launch_k(k_mid_back<8>, gb, 32 * BW, 0, s, base, tasks, xws);
-  else if (max_n <= 352) launch_k(k_mid_back<11>, gb, 32 * BW, 0, s, base, tasks, xws);
-  else launch_k(k_mid_back<16>, gb, 32 * BW, 0, s, base, tasks, xws);
+  auto back = [&](auto launch) { launch(s, base, tasks, ntasks, max_n, max_k, xws); };
+  if (max_n <= 160) back(launch_back<5, 2>);
+  else if (max_n <= 256) back(launch_back<8, 2>);
+  else if (max_n <= 352) back(launch_back<11, 2>);
+  else if (max_n <= 512) back(launch_back<16, 2>);
+  else if (max_n <= 1024) back(launch_back<32, 2>);
+  else back(launch_back<64, 1>);
   count_launch(10);
 }
 

@@ -332,7 +332,7 @@ DMRG_API int dmrg_test_gemm(dmrg_ctx* ctx, int transA, int transB, int M, int N,
  * (columns) overwrite A. */
 DMRG_API int dmrg_test_eigh(dmrg_ctx* ctx, int nmat, const int* n, double* A, double* w);
 
-/* Tridiagonal-path eigensolver (n[i] <= 512; blocks above 112 take the mid-size kernels): all
+/* Tridiagonal-path eigensolver (n[i] <= 2048; blocks above 112 take the mid-size kernels): all
  * eigenvalues (descending, packed in w) and the
  * eigenvectors of the k[i] largest (packed n[i] x k[i] column-major in U). A is overwritten. */
 DMRG_API int dmrg_test_syevt(dmrg_ctx* ctx, int nmat, const int* n, const int* k, double* A,
