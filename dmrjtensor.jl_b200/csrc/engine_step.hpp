@@ -105,6 +105,9 @@ struct Group {
   int64_t moff = 0, roff = 0, woff = 0;
 };
 
+// x /= |x| (n elements on the device), with <x,x> left in the scalar slot.
+void normalise_vec(dmrg_ctx* c, double* x, int64_t n, int slot);
+
 // The reduced density matrix of every group (rows: M M^T, else M^T M), its eigenvalues
 // (tridiagonal path up to SYEVT_MID_NMAX or SYEVT_RESOLVE_NMAX, block Jacobi above), and their
 // download.

@@ -74,6 +74,12 @@ void Timing::flush() {
   used = 0;
 }
 
+void normalise_vec(dmrg_ctx* c, double* x, int64_t n, int slot) {
+  if (launch_krylov(c->stream, KRY_NORMALISE, x, nullptr, n, c->d_scal, slot, 0.0)) return;
+  launch_mdot(c->stream, x, 0, 1, x, n, c->d_partial, c->d_scal + slot);
+  launch_scale_rsqrt(c->stream, x, n, c->d_scal + slot);
+}
+
 // Krylov solve: see engine_step.hpp. P.graph: everything of the solve after its first Heff
 // application (which makes every scratch allocation the step needs) is captured into a CUDA graph
 // and launched as one graph; the context keeps the executable graph and updates it in place from
@@ -115,29 +121,36 @@ KrylovRun krylov_solve(dmrg_state* st, const dmrg_params& P, const HeffPlan& hp,
     // simplelanczos (algs/DMRG.jl:57-90): H is applied to AA before its normalisation
     heff(K, H);
     tv = tm.begin();
-    launch_dot2(s, K, H, n, c->d_partial, scal + lz::KK);
-    launch_lanczos2_orth(s, K, H, n, scal, c->d_partial);   // K /= |K|, H -= a1 K, |H|^2
     double* K1 = K + n;
-    launch_next_vector(s, H, K1, n, scal, 0, P.betatest);
+    if (!launch_krylov(s, KRY_FIRST, K, H, n, scal, 0, P.betatest)) {
+      launch_dot2(s, K, H, n, c->d_partial, scal + lz::KK);
+      launch_lanczos2_orth(s, K, H, n, scal, c->d_partial);   // K /= |K|, H -= a1 K, |H|^2
+      launch_next_vector(s, H, K1, n, scal, 0, P.betatest);
+    }
     cuda_check(cudaGetLastError(), "Krylov vector");
     tm.end(tv, 3);
     heff(K1, H);
     tv = tm.begin();
-    launch_mdot(s, K1, 0, 1, H, n, c->d_partial, scal + lz::ALPHA + 1);
+    if (!launch_krylov(s, KRY_ALPHA, K, H, n, scal, 1, P.betatest))
+      launch_mdot(s, K1, 0, 1, H, n, c->d_partial, scal + lz::ALPHA + 1);
     launch_ritz(s, scal, 2, 0.0, false);
     launch_lincomb(s, K, n, 2, scal + lz::COEF, H, n);
     tm.end(tv, 3);
   } else {
     tv = tm.begin();
-    launch_mdot(s, K, 0, 1, K, n, c->d_partial, scal + lz::KK);
-    launch_scale_rsqrt(s, K, n, scal + lz::KK);
+    normalise_vec(c, K, n, lz::KK);
     tm.end(tv, 3);
     for (int jj = 0; jj < kdim; ++jj) {
       double* Kj = K + int64_t(jj) * n;
       heff(Kj, H);
       tv = tm.begin();
+      const bool last = jj == kdim - 1;
+      if (launch_krylov(s, last ? KRY_ALPHA : KRY_STEP, K, H, n, scal, jj, P.betatest)) {
+        tm.end(tv, 3);
+        continue;
+      }
       launch_mdot(s, Kj, 0, 1, H, n, c->d_partial, scal + lz::ALPHA + jj);
-      if (jj == kdim - 1) { tm.end(tv, 3); break; }
+      if (last) { tm.end(tv, 3); break; }
       launch_axpby(s, n, 0.0, scal + lz::ALPHA + jj, -1.0, Kj, 1.0, nullptr, 0, H, 0);
       if (jj > 0)
         launch_axpby(s, n, 0.0, scal + lz::BETA + jj - 1, -1.0, Kj - n, 1.0, nullptr, 0, H, 0);
@@ -348,9 +361,7 @@ void twostep(dmrg_state* st, const dmrg_params& P, int j, int iL, int iR, bool f
   // the device
   int tv = tm.begin();
   const int ic = j > 0 ? iL : iR;
-  launch_mdot(s, st->A[ic].p, 0, 1, st->A[ic].p, st->lay[ic].size, c->d_partial,
-              c->d_scal + lz::NRM);
-  launch_scale_rsqrt(s, st->A[ic].p, st->lay[ic].size, c->d_scal + lz::NRM);
+  normalise_vec(c, st->A[ic].p, st->lay[ic].size, lz::NRM);
   cuda_check(cudaGetLastError(), "centre normalisation");
 
   HeffPlan hp;

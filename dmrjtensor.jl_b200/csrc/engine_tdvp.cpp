@@ -48,9 +48,7 @@ void evolve_site(dmrg_state* st, const dmrg_params& P, int i, double tau, Timing
 
 void normalise(dmrg_state* st, int i) {
   dmrg_ctx* c = st->ctx;
-  launch_mdot(c->stream, st->A[i].p, 0, 1, st->A[i].p, st->lay[i].size, c->d_partial,
-              c->d_scal + lz::NRM);
-  launch_scale_rsqrt(c->stream, st->A[i].p, st->lay[i].size, c->d_scal + lz::NRM);
+  normalise_vec(c, st->A[i].p, st->lay[i].size, lz::NRM);
   cuda_check(cudaGetLastError(), "centre normalisation");
 }
 

@@ -217,6 +217,17 @@ void raise_smem_limit(const void* func, size_t bytes) {
     c = bytes;
 }
 
+void allow_wide_clusters(const void* func) {
+  static std::mutex mu;
+  static std::map<std::pair<int, const void*>, bool> done;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lk(mu);
+  bool& d = done[{dev, func}];
+  if (!d) d = cudaFuncSetAttribute(func, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
+              cudaSuccess;
+}
+
 static std::atomic<long long> g_launches{0};
 void count_launch(int n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 long long launch_count() { return g_launches.load(std::memory_order_relaxed); }

@@ -218,6 +218,16 @@ void launch_pair_dot(cudaStream_t s, const double* X, const double* Y, const Pai
 void launch_pair_dot_rows(cudaStream_t s, const double* X, int64_t x_stride, const double* Y,
                           const PairTask* tasks, int ntasks, int nrows, double* out,
                           int64_t out_stride);
+// The vector work between two Heff applications as one launch (krylov.cu), with the numbers of the
+// launches above bit for bit: false (nothing launched) for vectors above KRY_MAX elements.
+//   KRY_NORMALISE  s[j] = <K,K>, K /= |K|                       (mdot, scale_rsqrt)
+//   KRY_FIRST      the first half of the 2-vector step           (dot2, lanczos2_orth, next_vector)
+//   KRY_STEP       Lanczos iteration j: alpha_j, two-term recursion, CGS2, next vector K_{j+1}
+//   KRY_ALPHA      alpha_j alone                                 (mdot)
+constexpr int KRY_MAX = 65536;
+constexpr int KRY_NORMALISE = 0, KRY_FIRST = 1, KRY_STEP = 2, KRY_ALPHA = 3;
+bool launch_krylov(cudaStream_t s, int mode, double* K, double* H, int64_t n, double* scal, int j,
+                   double betatest);
 // y = sum_j c[j] X_j, j < k
 void launch_lincomb(cudaStream_t s, const double* X, int64_t ldx, int k, const double* c,
                     double* y, int64_t n);
@@ -250,6 +260,8 @@ int device_sm_count();
 // Raises (never lowers) a kernel's dynamic shared-memory limit on the current device; safe when
 // several host threads launch the same kernel with different sizes.
 void raise_smem_limit(const void* func, size_t bytes);
+// Allows a kernel clusters of up to 16 CTAs on the current device.
+void allow_wide_clusters(const void* func);
 // Process-wide count of kernel launches issued by this library.
 void count_launch(int n = 1);
 long long launch_count();

@@ -45,10 +45,7 @@ inline void launch_k(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, c
 }
 
 // The same with thread-block clusters of c CTAs (grid: a multiple of c). Above 8 CTAs the size is
-// not portable and has to be allowed first, once per kernel and device.
-inline void allow_wide_clusters(const void* func) {
-  (void)cudaFuncSetAttribute(func, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-}
+// not portable and has to be allowed first (allow_wide_clusters).
 template <typename... P, typename... A>
 inline void launch_cluster_k(void (*kernel)(P...), int c, dim3 grid, dim3 block, size_t smem,
                              cudaStream_t s, A&&... args) {

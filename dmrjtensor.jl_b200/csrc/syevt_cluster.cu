@@ -24,6 +24,7 @@
 // one CTA with the matrix in global and shared memory: 4.6 ms with the eigenvalues).
 #include <cstring>
 
+#include "cluster.cuh"
 #include "kernels.cuh"
 #include "launch.cuh"
 #include "syevt_common.cuh"
@@ -38,24 +39,6 @@ constexpr int HTX = HT + 32;         // and of the reflector warp
 // Bit pattern (a NaN) that k_trid_cluster leaves in d[0] when a wait gave up.
 constexpr long long TRID_GAVE_UP = 0x7ff8000000d06e0fLL;
 
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ int cluster_rank() {
-  unsigned r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return int(r);
-}
-__device__ __forceinline__ unsigned smem_addr(const void* p) {
-  return unsigned(__cvta_generic_to_shared(p));
-}
-// the address in CTA `rank` of the cluster of the shared-memory address a of this CTA
-__device__ __forceinline__ unsigned peer_addr(unsigned a, int rank) {
-  unsigned r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
-  return r;
-}
 // stores into another CTA that count their bytes into its mbarrier
 __device__ __forceinline__ void async_store(unsigned addr, unsigned bar, double a, double b) {
   asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];"
@@ -120,13 +103,6 @@ constexpr int LCOLS = 4;             // columns per warp and sweep
 // from the same 32-row boundaries).
 __host__ __device__ __forceinline__ int trid_lead_steps(int n) {
   return n <= HN ? 0 : (n - HN + 31) / 32 * 32;
-}
-
-__device__ __forceinline__ void peer_store(unsigned addr, double a, double b) {
-  asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" :: "r"(addr), "d"(a), "d"(b) : "memory");
-}
-__device__ __forceinline__ void peer_store(unsigned addr, double a) {
-  asm volatile("st.shared::cluster.f64 [%0], %1;" :: "r"(addr), "d"(a) : "memory");
 }
 
 template <int N, int MASK>

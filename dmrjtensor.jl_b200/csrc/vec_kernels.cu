@@ -348,10 +348,13 @@ __global__ void k_next_vector(const double* __restrict__ H, double* __restrict__
 }
 
 // Ritz step of the Krylov solve, one warp: T = tridiag(alpha, beta) of the m active vectors
-// (m = 1 + number of leading non-zero beta_j, at most kdim), cyclic Jacobi (serial rotation
-// order; lanes own the rows/columns of one rotation) until the off-diagonal is at the rounding
-// level of the diagonal, lowest
-// eigenvalue -> s[EN], its eigenvector -> s[COEF + j] (0 for j >= m).
+// (m = 1 + number of leading non-zero beta_j, at most kdim), Jacobi rotations until the
+// off-diagonal is at the rounding level of the diagonal, lowest eigenvalue -> s[EN], its
+// eigenvector -> s[COEF + j] (0 for j >= m). The rotations of a round are disjoint pairs (the
+// round-robin order of a tournament), one lane per angle and one lane per element of the row,
+// column and vector updates: m - 1 rounds a sweep instead of m (m - 1) / 2 rotations one after the
+// other, each of which is a chain of square roots and divisions (m = 8: 81 -> 35 us). A
+// 2-vector step is one rotation, written out.
 // expo = 0: the lowest Ritz pair (s[EN], s[COEF + j]). expo = 1: s[COEF + j] = (exp(tau T) e_1)_j
 // (krylovTimeEvol, algs/time.jl:182-203: the Krylov vectors are orthonormal, so these are the
 // coefficients of exp(tau H) applied to the normalised start vector), from the eigenpairs of T;
@@ -359,6 +362,8 @@ __global__ void k_next_vector(const double* __restrict__ H, double* __restrict__
 __global__ void k_ritz(double* s, int kdim, double tau, int expo) {
   grid_entry();
   __shared__ double A[MAXK * MAXK], V[MAXK * MAXK];
+  __shared__ double rc[MAXK / 2], rs[MAXK / 2];
+  __shared__ int rp[MAXK / 2], rq[MAXK / 2];
   const int lane = threadIdx.x;
   int m = 1;
   while (m < kdim && s[lz::BETA + m - 1] > 0.0) ++m;
@@ -372,37 +377,90 @@ __global__ void k_ritz(double* s, int kdim, double tau, int expo) {
     V[e] = (r == c) ? 1.0 : 0.0;
   }
   __syncwarp();
+  // this lane's elements e = lane, lane + 32, ... of a row or column update: pair e / m, index e % m
+  const int x0 = lane / m, i0 = lane - x0 * m, xs = 32 / m, is = 32 - xs * m;
+  const int mm = (m + 1) & ~1;                    // an odd m sits one index out per round
   for (int sweep = 0; sweep < 100; ++sweep) {
     double off = 0.0, dg = 0.0;
-    for (int p = 0; p < m; ++p) {
-      dg += A[p + p * m] * A[p + p * m];
-      for (int q = p + 1; q < m; ++q) off += A[p + q * m] * A[p + q * m];
+    for (int e = lane; e < m * m; e += 32) {
+      const int r = e % m, c = e / m;
+      if (r == c) dg += A[e] * A[e];
+      else if (r < c) off += A[e] * A[e];
     }
+    off = warp_sum(off);
+    dg = warp_sum(dg);
     if (off < 1e-300 || off <= 1e-32 * dg) break;   // off-diagonal at the rounding level
-    for (int p = 0; p < m; ++p)
-      for (int q = p + 1; q < m; ++q) {
-        const double apq = A[p + q * m];
-        if (fabs(apq) < 1e-300) continue;
-        const double theta = (A[q + q * m] - A[p + p * m]) / (2.0 * apq);
-        const double t = (theta >= 0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
-        const double c = 1.0 / sqrt(t * t + 1.0), sn = t * c;
-        __syncwarp();
-        if (lane < m) {   // rows p, q
-          const double ap = A[p + lane * m], aq = A[q + lane * m];
-          A[p + lane * m] = c * ap - sn * aq;
-          A[q + lane * m] = sn * ap + c * aq;
-        }
-        __syncwarp();
-        if (lane < m) {   // columns p, q
-          const double ap = A[lane + p * m], aq = A[lane + q * m];
-          A[lane + p * m] = c * ap - sn * aq;
-          A[lane + q * m] = sn * ap + c * aq;
-          const double vp = V[lane + p * m], vq = V[lane + q * m];
-          V[lane + p * m] = c * vp - sn * vq;
-          V[lane + q * m] = sn * vp + c * vq;
-        }
-        __syncwarp();
+    if (m == 2) {
+      const int p = 0, q = 1;
+      const double apq = A[p + q * m];
+      const double theta = (A[q + q * m] - A[p + p * m]) / (2.0 * apq);
+      const double t = (theta >= 0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
+      const double c = 1.0 / sqrt(t * t + 1.0), sn = t * c;
+      __syncwarp();
+      if (lane < m) {   // rows p, q
+        const double ap = A[p + lane * m], aq = A[q + lane * m];
+        A[p + lane * m] = c * ap - sn * aq;
+        A[q + lane * m] = sn * ap + c * aq;
       }
+      __syncwarp();
+      if (lane < m) {   // columns p, q
+        const double ap = A[lane + p * m], aq = A[lane + q * m];
+        A[lane + p * m] = c * ap - sn * aq;
+        A[lane + q * m] = sn * ap + c * aq;
+        const double vp = V[lane + p * m], vq = V[lane + q * m];
+        V[lane + p * m] = c * vp - sn * vq;
+        V[lane + q * m] = sn * vp + c * vq;
+      }
+      __syncwarp();
+      continue;
+    }
+    for (int round = 0; round < mm - 1; ++round) {
+      if (lane < mm / 2) {
+        // pair of this lane: index mm - 1 stays, the others move one place a round
+        int p = lane == 0 ? mm - 1 : (round + lane) % (mm - 1);
+        int q = lane == 0 ? round : (round - lane + mm - 1) % (mm - 1);
+        if (p > q) { const int x = p; p = q; q = x; }
+        double c = 1.0, sn = 0.0;
+        if (q < m) {
+          const double apq = A[p + q * m];
+          if (fabs(apq) >= 1e-300) {
+            // t = tan of the smaller rotation angle
+            const double df = A[q + q * m] - A[p + p * m], o2 = 2.0 * apq;
+            const double t = (df >= 0 ? o2 : -o2) / (fabs(df) + sqrt(fma(df, df, o2 * o2)));
+            c = rsqrt(fma(t, t, 1.0));
+            sn = t * c;
+          }
+        }
+        rp[lane] = p;
+        rq[lane] = q;
+        rc[lane] = c;
+        rs[lane] = sn;
+      }
+      __syncwarp();
+      for (int x = x0, i = i0; x < mm / 2; x += xs, i += is) {   // rows p, q
+        if (i >= m) { i -= m; ++x; if (x >= mm / 2) break; }
+        const int p = rp[x], q = rq[x];
+        if (q < m) {
+          const double ap = A[p + i * m], aq = A[q + i * m], c = rc[x], sn = rs[x];
+          A[p + i * m] = c * ap - sn * aq;
+          A[q + i * m] = sn * ap + c * aq;
+        }
+      }
+      __syncwarp();
+      for (int x = x0, i = i0; x < mm / 2; x += xs, i += is) {   // columns p, q
+        if (i >= m) { i -= m; ++x; if (x >= mm / 2) break; }
+        const int p = rp[x], q = rq[x];
+        if (q < m) {
+          const double ap = A[i + p * m], aq = A[i + q * m], c = rc[x], sn = rs[x];
+          A[i + p * m] = c * ap - sn * aq;
+          A[i + q * m] = sn * ap + c * aq;
+          const double vp = V[i + p * m], vq = V[i + q * m];
+          V[i + p * m] = c * vp - sn * vq;
+          V[i + q * m] = sn * vp + c * vq;
+        }
+      }
+      __syncwarp();
+    }
   }
   int o = 0;
   for (int k = 1; k < m; ++k)
