@@ -431,6 +431,7 @@ struct StepPlan {
   GemmList g1t, g3t;        // retiled copies for the split-precision kernel (split != 0)
   int split = 0;            // split form of the two GEMMs, 0 = FP64
   MixList mx;
+  bool direct = false;      // the site's operator is the identity: g3 reads T1, mx is empty
   EnvLayout out;
   int64_t t1 = 0, t2 = 0;   // scratch sizes in doubles
   double flops() const { return g1.flops + g3.flops + mx.flops; }
@@ -452,6 +453,8 @@ void env_step_dense(dmrg_ctx* c, bool left, int ml, int d, int mr, int wl, int w
                     const double* env_in, const double* dual, const double* psi, const double* W,
                     double* env_out);
 
+// Creates the context's second stream and its fork and join events.
+void ensure_env_stream(dmrg_ctx* c);
 void env_boundaries(dmrg_state* st);
 void lupdate(dmrg_state* st, int i, double* flops, int precision = DMRG_PREC_FP64);
 void rupdate(dmrg_state* st, int i, double* flops, int precision = DMRG_PREC_FP64);

@@ -308,6 +308,16 @@ void env_boundaries(dmrg_state* st) {
   st->Rvalid[L - 1] = 1;
 }
 
+namespace {
+// One MPO state on either side and the identity between them: mixing would copy T1.
+bool identity_site(const MPOSite& ms) {
+  if (ms.wl != 1 || ms.wr != 1 || int(ms.nz.size()) != ms.d) return false;
+  for (const auto& e : ms.nz)
+    if (e.s != e.t || e.v != 1.0) return false;
+  return true;
+}
+}  // namespace
+
 void plan_left_step(const Bond& Bl, const Bond& Br, const MPOSite& ms, const SiteLayout& lay,
                     const EnvLayout& LL, StepPlan& sp) {
   sp.out = make_left_env_layout(Br, ms.rr);
@@ -332,6 +342,25 @@ void plan_left_step(const Bond& Bl, const Bond& Br, const MPOSite& ms, const Sit
     if (LL.rows[kb] == 0 || lay.gcols[kb] == 0) continue;
     g1.add(t1off[kb], LL.rows[kb], LL.rows[kb], lay.gcols[kb], 1.0, 0.0);
     g1.seg(LL.goff[kb], LL.rows[kb], lay.goff[kb], Bl.dim[kb], Bl.dim[kb]);
+  }
+  sp.direct = identity_site(ms);
+  if (sp.direct) {
+    sp.t2 = 0;
+    for (int kbp = 0; kbp < Br.nsec(); ++kbp) {
+      const int kap = LN.other[kbp];
+      if (kap < 0) continue;
+      g3.add(LN.goff[kbp] + LN.rowoff[kbp], LN.rows[kbp], Br.dim[kap], Br.dim[kbp], 1.0, 0.0);
+      for (int t = 0; t < d; ++t) {
+        const int ka = Bl.find(Br.q[kap] - ms.p[t]);
+        if (ka < 0 || lay.kb[ka * d + t] != kap) continue;
+        const int kb = Bl.find(Bl.q[ka] + ms.rl[0]);
+        if (kb < 0 || LL.other[kb] != ka || lay.kb[kb * d + t] != kbp) continue;
+        const int64_t col = (lay.off[kb * d + t] - lay.goff[kb]) / Bl.dim[kb];
+        g3.seg(lay.off[ka * d + t], Bl.dim[ka],
+               t1off[kb] + LL.rowoff[kb] + col * LL.rows[kb], LL.rows[kb], Bl.dim[ka]);
+      }
+    }
+    return;
   }
   // non-zeros grouped by (t, w')
   std::vector<std::vector<const MPOSite::El*>> byTW(size_t(d) * wr);
@@ -412,6 +441,22 @@ void plan_right_step(const Bond& Bl, const Bond& Br, const MPOSite& ms, const Si
       g1.add(t1off[ka * d + t], RL.rows[kap], RL.rows[kap], Bl.dim[ka], 1.0, 0.0);
       g1.seg(RL.goff[kap], RL.rows[kap], lay.off[ka * d + t], Bl.dim[ka], Br.dim[kap]);
     }
+  sp.direct = identity_site(ms);
+  if (sp.direct) {
+    sp.t2 = 0;
+    for (int ka = 0; ka < Bl.nsec(); ++ka) {
+      const int kb = RN.other[ka];
+      if (kb < 0) continue;
+      g3.add(RN.goff[ka] + RN.rowoff[ka], RN.rows[ka], Bl.dim[kb], Bl.dim[ka], 1.0, 0.0);
+      for (int s = 0; s < d; ++s) {
+        const int kbp = lay.kb[kb * d + s], kap = lay.kb[ka * d + s];
+        if (kbp < 0 || kap < 0 || RL.rows[kap] == 0 || RL.other[kap] != kbp) continue;
+        g3.seg(lay.off[kb * d + s], Bl.dim[kb], t1off[ka * d + s] + RL.rowoff[kap], RL.rows[kap],
+               Br.dim[kbp]);
+      }
+    }
+    return;
+  }
   std::vector<std::vector<const MPOSite::El*>> byWS(size_t(wl) * d);
   for (const auto& e : ms.nz) byWS[size_t(e.w) * d + e.s].push_back(&e);
 
@@ -480,10 +525,11 @@ void run_step(dmrg_ctx* c, const StepPlan& sp, char* db, const double* env_in, i
   else
     run_gemm(c, sp.g1, db, env_in, n_in, first.p, first.n, c->T1.p, c->T1.n);
   run_mix(c, sp.mx, db, c->T1.p, c->T1.n, c->T2.p, c->T2.n);
+  const DBuf& mixed = sp.direct ? c->T1 : c->T2;
   if (sp.split)
-    run_gemm_split(c, sp.g3t, db, last.p, last.n, c->T2.p, c->T2.n, env_out, n_out, sp.split);
+    run_gemm_split(c, sp.g3t, db, last.p, last.n, mixed.p, mixed.n, env_out, n_out, sp.split);
   else
-    run_gemm(c, sp.g3, db, last.p, last.n, c->T2.p, c->T2.n, env_out, n_out);
+    run_gemm(c, sp.g3, db, last.p, last.n, mixed.p, mixed.n, env_out, n_out);
 }
 
 void env_step_dense(dmrg_ctx* c, bool left, int ml, int d, int mr, int wl, int wr,

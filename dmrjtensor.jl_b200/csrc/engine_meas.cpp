@@ -130,53 +130,97 @@ void run_pair(dmrg_ctx* c, const PairPlan& pp, char* db, const DBuf& X, const DB
                   int(pp.t.size()), pp.total, c->d_partial, out);
 }
 
-// `sp` repeated for `nrows` environments stored back to back: copy r reads env_in + r*in_stride,
-// writes env_out + r*out_stride and uses the scratch T1 + r*sp.t1, T2 + r*sp.t2; the site tensor
-// is shared by every copy.
-StepPlan replicate_step(const StepPlan& sp, int nrows, int64_t in_stride, int64_t out_stride) {
-  StepPlan b;
-  b.g1.tA = sp.g1.tA;
-  b.g1.tB = sp.g1.tB;
-  b.g3.tA = sp.g3.tA;
-  b.g3.tB = sp.g3.tB;
-  for (int r = 0; r < nrows; ++r) {
-    for (const GemmTask& t : sp.g1.tasks) {       // env_in x site -> T1
-      b.g1.add(t.c_off + r * sp.t1, t.ldc, t.M, t.N, t.alpha, t.beta);
-      for (int k = t.seg0; k < t.seg0 + t.nseg; ++k) {
-        const GemmSeg& g = sp.g1.segs[k];
-        b.g1.seg(g.a_off + r * in_stride, g.lda, g.b_off, g.ldb, g.K);
-      }
-    }
-    for (const MixTask& t : sp.mx.tasks) {        // T1 -> T2
-      b.mx.add(t.out_off + r * sp.t2, t.ld, t.rows, t.cols);
-      for (int k = t.term0; k < t.term0 + t.nterm; ++k) {
-        const MixTerm& m = sp.mx.terms[k];
-        b.mx.term(m.in_off + r * sp.t1, m.ld, m.coef);
-      }
-    }
-    for (const GemmTask& t : sp.g3.tasks) {       // site x T2 -> env_out
-      b.g3.add(t.c_off + r * out_stride, t.ldc, t.M, t.N, t.alpha, t.beta);
-      for (int k = t.seg0; k < t.seg0 + t.nseg; ++k) {
-        const GemmSeg& g = sp.g3.segs[k];
-        b.g3.seg(g.a_off, g.lda, g.b_off + r * sp.t2, g.ldb, g.K);
-      }
-    }
-  }
-  b.out = sp.out;
-  b.t1 = sp.t1 * nrows;
-  b.t2 = sp.t2 * nrows;
-  return b;
+// The tile shape of a measurement list: 32 x 32 where the blocks are small (a 64 x 64 tile of a
+// 30 x 60 block is mostly padding), 64 x 64 otherwise.
+void pick_tiles(GemmList& g) {
+  double area = 0.0, n = 0.0;
+  for (const GemmTask& t : g.tasks) { area += double(t.M) * t.N; n += 1.0; }
+  if (n > 0 && area < 96.0 * 96.0 * n) g = retile(g, GEMM_SMALL_TILE, GEMM_SMALL_TILE);
 }
 
-// out[r * out_stride] = pair contraction of row r of X (rows of x_stride doubles) with Y.
-void run_pair_rows(dmrg_ctx* c, const PairPlan& pp, char* db, const DBuf& X, int nrows,
-                   int64_t x_stride, const DBuf& Y, double* out, int64_t out_stride) {
-  check_pair(pp, x_stride, Y.n);
-  if (int64_t(nrows) * x_stride > X.n)
-    fail(DMRG_ERR_ARG, "internal plan check failed: pair rows out of bounds");
-  launch_pair_dot_rows(c->stream, X.p, x_stride, Y.p,
-                       reinterpret_cast<const PairTask*>(db + pp.off), int(pp.t.size()), nrows,
-                       out, out_stride);
+void launch_list(dmrg_ctx* c, const GemmList& g, char* db, const double* A, const double* B,
+                 double* C, const GemmBatch& b = GemmBatch{}) {
+  launch_gemm_f64(c->stream, g.bm, g.tA, g.tB, A, B, C,
+                  reinterpret_cast<const GemmTask*>(db + g.t_off), int(g.tasks.size()),
+                  reinterpret_cast<const GemmSeg*>(db + g.s_off), g.tiles, c->nsm * 4, b);
+}
+
+// One environment step of `nrows` rows through the same site: row r reads env_in + r * in_stride
+// (the last row `last` instead, when given), writes out + r * out_stride and uses row r of the
+// scratch.
+void run_step_rows(dmrg_ctx* c, const StepPlan& sp, char* db, int nrows, const double* env_in,
+                   int64_t in_stride, int64_t n_in, const DBuf* last, const DBuf& A, double* out,
+                   int64_t out_stride, int64_t n_out) {
+  const int own = last ? nrows - 1 : nrows;      // rows in env_in
+  if (c->T1.n < sp.t1 * nrows || c->T2.n < sp.t2 * nrows || n_out < out_stride * nrows ||
+      out_stride < sp.out.size || n_in < in_stride * own || (last && last->n < in_stride))
+    fail(DMRG_ERR_ARG, "internal plan check failed: environment rows out of bounds");
+  check_gemm_list(sp.g1, in_stride, A.n, sp.t1);
+  check_mix_list(sp.mx, sp.t1, sp.t2);
+  check_gemm_list(sp.g3, A.n, sp.direct ? sp.t1 : sp.t2, out_stride);
+  GemmBatch b;
+  b.n = nrows;
+  b.a = in_stride;
+  b.c = sp.t1;
+  b.a_last = last ? last->p : nullptr;
+  launch_list(c, sp.g1, db, env_in, A.p, c->T1.p, b);
+  launch_mix(c->stream, c->T1.p, c->T2.p, reinterpret_cast<const MixTask*>(db + sp.mx.t_off),
+             int(sp.mx.tasks.size()), reinterpret_cast<const MixTerm*>(db + sp.mx.m_off),
+             sp.mx.tiles, nrows, sp.t1, sp.t2);
+  b = GemmBatch{};
+  b.n = nrows;
+  b.b = sp.direct ? sp.t1 : sp.t2;
+  b.c = out_stride;
+  launch_list(c, sp.g3, db, A.p, sp.direct ? c->T1.p : c->T2.p, out, b);
+}
+
+// Many independent steps (different sites) as one: lists with absolute element offsets (address /
+// 8, zero bases), scratch one after the other.
+struct ManySteps {
+  StepPlan sp;
+  int64_t t1 = 0, t2 = 0;
+};
+int64_t element_of(const double* p) { return int64_t(reinterpret_cast<uintptr_t>(p) / 8); }
+void add_step(ManySteps& m, const StepPlan& sp, const DBuf& env_in, const DBuf& A,
+              const DBuf& out, double* T1, double* T2) {
+  check_gemm_list(sp.g1, env_in.n, A.n, sp.t1);
+  check_mix_list(sp.mx, sp.t1, sp.t2);
+  check_gemm_list(sp.g3, A.n, sp.direct ? sp.t1 : sp.t2, out.n);
+  m.sp.g1.tA = sp.g1.tA;
+  m.sp.g1.tB = sp.g1.tB;
+  m.sp.g3.tA = sp.g3.tA;
+  m.sp.g3.tB = sp.g3.tB;
+  const int64_t x1 = element_of(T1) + m.t1, x2 = element_of(T2) + m.t2;
+  auto copy = [](GemmList& to, const GemmList& g, int64_t a, int64_t b, int64_t c) {
+    for (const GemmTask& t : g.tasks) {
+      to.add(t.c_off + c, t.ldc, t.M, t.N, t.alpha, t.beta);
+      for (int k = t.seg0; k < t.seg0 + t.nseg; ++k) {
+        const GemmSeg& q = g.segs[k];
+        to.seg(q.a_off + a, q.lda, q.b_off + b, q.ldb, q.K);
+      }
+    }
+  };
+  copy(m.sp.g1, sp.g1, element_of(env_in.p), element_of(A.p), x1);
+  for (const MixTask& t : sp.mx.tasks) {
+    m.sp.mx.add(t.out_off + x2, t.ld, t.rows, t.cols);
+    for (int k = t.term0; k < t.term0 + t.nterm; ++k)
+      m.sp.mx.term(sp.mx.terms[k].in_off + x1, sp.mx.terms[k].ld, sp.mx.terms[k].coef);
+  }
+  copy(m.sp.g3, sp.g3, element_of(A.p), sp.direct ? x1 : x2, element_of(out.p));
+  m.t1 += sp.t1;
+  m.t2 += sp.t2;
+}
+void put_many(Upload& u, ManySteps& m) {
+  pick_tiles(m.sp.g1);
+  pick_tiles(m.sp.g3);
+  put_step(u, m.sp);
+}
+void run_many(dmrg_ctx* c, const ManySteps& m, char* db) {
+  launch_list(c, m.sp.g1, db, nullptr, nullptr, nullptr);
+  launch_mix(c->stream, nullptr, nullptr, reinterpret_cast<const MixTask*>(db + m.sp.mx.t_off),
+             int(m.sp.mx.tasks.size()), reinterpret_cast<const MixTerm*>(db + m.sp.mx.m_off),
+             m.sp.mx.tiles);
+  launch_list(c, m.sp.g3, db, nullptr, nullptr, nullptr);
 }
 
 void set_one(dmrg_ctx* c, DBuf& b) {
@@ -190,6 +234,17 @@ int64_t plan_scratch(const StepPlan& sp, int64_t& t1, int64_t& t2) {
   t2 = std::max(t2, sp.t2);
   return sp.out.size;
 }
+
+// Waits (on the context's stream) for the chain on env_stream, at the latest when the scope ends.
+struct JoinGuard {
+  dmrg_ctx* c;
+  bool done = false;
+  void now() {
+    if (!done) cudaStreamWaitEvent(c->stream, c->env_join, 0);
+    done = true;
+  }
+  ~JoinGuard() { now(); }
+};
 
 void check_edges(const dmrg_state* st) {
   const Bond& b0 = st->bond[0];
@@ -277,140 +332,226 @@ void measure_correlation(dmrg_state* st, int d, const double* Cc_, const double*
   const std::vector<double> onsite = matmul(Cc, Ca, d);  // contract(Cc, 2, Ca, 1)
   const QN zero;
 
-  // ---- plans
+  // ---- plans of every step
   std::vector<EnvLayout> ELl(L + 1), ERl(L + 1);
-  std::vector<StepPlan> spL(L), spR(L), spC(L);
+  std::vector<StepPlan> spL(L), spR(L), spC(L), spD(L), spS(L), spF(L);
   ELl[0] = make_left_env_layout(st->bond[0], {zero});
   ERl[L] = make_right_env_layout(st->bond[L], {zero});
   if (ELl[0].other[0] != 0 || ERl[L].other[0] != 0)
     fail(DMRG_ERR_QN, "edge sectors of the MPS do not connect");
-  int64_t t1 = 1, t2 = 1;
+  int64_t t1 = 1, t2 = 1, r1 = 1, r2 = 1;
   Upload u;
+  double fl = 0.0;
   for (int i = 0; i < L; ++i) {
     const MPOSite id = op_site(Id, d, st->mpo->site[i].p, zero, true);
     plan_left_step(st->bond[i], st->bond[i + 1], id, st->lay[i], ELl[i], spL[i]);
     ELl[i + 1] = spL[i].out;
     plan_scratch(spL[i], t1, t2);
+    pick_tiles(spL[i].g1);
+    pick_tiles(spL[i].g3);
     put_step(u, spL[i]);
   }
   for (int i = L - 1; i >= 0; --i) {
     const MPOSite id = op_site(Id, d, st->mpo->site[i].p, zero, true);
     plan_right_step(st->bond[i], st->bond[i + 1], id, st->lay[i], ERl[i + 1], spR[i]);
     ERl[i] = spR[i].out;
-    plan_scratch(spR[i], t1, t2);
+    plan_scratch(spR[i], r1, r2);
+    pick_tiles(spR[i].g1);
+    pick_tiles(spR[i].g3);
     put_step(u, spR[i]);
   }
   for (int j = 1; j < L; ++j) {
     const MPOSite ca = op_site(Ca, d, st->mpo->site[j].p, zero, false);
     plan_right_step(st->bond[j], st->bond[j + 1], ca, st->lay[j], ERl[j + 1], spC[j]);
-    plan_scratch(spC[j], t1, t2);
-    put_step(u, spC[j]);
   }
   // diagonal: (Cc Ca) at site i between EL[i] and ER[i+1]
-  std::vector<StepPlan> spD(L);
-  std::vector<PairPlan> ppD(L);
-  int64_t dmax = 1;
   for (int i = 0; i < L; ++i) {
     const MPOSite on = op_site(onsite, d, st->mpo->site[i].p, zero, true);
     plan_left_step(st->bond[i], st->bond[i + 1], on, st->lay[i], ELl[i], spD[i]);
-    dmax = std::max(dmax, plan_scratch(spD[i], t1, t2));
-    put_step(u, spD[i]);
-    ppD[i] = plan_pair(st->bond[i + 1], spD[i].out, ERl[i + 1]);
-    ppD[i].off = u.put(ppD[i].t);
   }
   // off-diagonal, one bond (column) j at a time: the rows i < j hold X_i at bond j back to back
-  // (one layout per bond, since every row carries the same charge label); X_{j-1} starts from
-  // EL[j-1] through (Cc F) at site j-1, the older rows move through F at site j-1 in one
-  // replicated step, and one launch contracts every row with RC[j].
-  std::vector<StepPlan> spS(L), spF(L);     // [j]: start of row j-1 / batched F step into bond j
+  // (one layout per bond, since every row carries the same charge label). Row j-1 starts from
+  // EL[j-1] through (Cc F) at site j-1 (S[j]: all rows' starts are independent and run as one
+  // step); the older rows move through F at site j-1 in one step of j-1 rows, and one launch
+  // contracts every row with RC[j].
   std::vector<PairPlan> ppC(L);
   std::vector<int64_t> xs(L, 0);            // X layout size at bond j
-  int64_t xmax = 1;
+  int64_t xmax = 1, f1 = 1, f2 = 1;
   QN label;
   for (int j = 1; j < L; ++j) {
     const MPOSite fc = op_site(FCc, d, st->mpo->site[j - 1].p, zero, true);
     label = fc.rr[0];
     plan_left_step(st->bond[j - 1], st->bond[j], fc, st->lay[j - 1], ELl[j - 1], spS[j]);
-    plan_scratch(spS[j], t1, t2);
-    put_step(u, spS[j]);
     xs[j] = spS[j].out.size;
     if (j >= 2) {
       const MPOSite f = op_site(F, d, st->mpo->site[j - 1].p, label, true);
-      StepPlan one;
-      plan_left_step(st->bond[j - 1], st->bond[j], f, st->lay[j - 1], spS[j - 1].out, one);
-      if (one.out.size != xs[j]) fail(DMRG_ERR_ARG, "internal plan check failed: row layouts differ");
-      spF[j] = replicate_step(one, j - 1, xs[j - 1], xs[j]);
-      plan_scratch(spF[j], t1, t2);
-      put_step(u, spF[j]);
+      plan_left_step(st->bond[j - 1], st->bond[j], f, st->lay[j - 1], spS[j - 1].out, spF[j]);
+      if (spF[j].out.size != xs[j])
+        fail(DMRG_ERR_ARG, "internal plan check failed: row layouts differ");
+      pick_tiles(spF[j].g1);
+      pick_tiles(spF[j].g3);
+      f1 = std::max(f1, spF[j].t1 * (j - 1));
+      f2 = std::max(f2, spF[j].t2 * (j - 1));
+      fl += spF[j].flops() * (j - 1);
     }
     xmax = std::max(xmax, int64_t(j) * std::max<int64_t>(xs[j], 1));
     ppC[j] = plan_pair(st->bond[j], spS[j].out, spC[j].out);
-    ppC[j].off = u.put(ppC[j].t);
+    fl += 2.0 * ppC[j].total * j;
   }
   PairPlan norm = plan_pair(st->bond[L], ELl[L], ERl[L]);
   norm.off = u.put(norm.t);
 
   // ---- device buffers and launches
-  std::vector<DBuf> EL(L + 1), ER(L + 1), RC(L);
-  DBuf D, X[2], out;
+  std::vector<DBuf> EL(L + 1), ER(L + 1), RC(L), S(L);
+  std::vector<DBuf> D;
+  DBuf X[2], out, TR1, TR2;
   auto release = [&] {
-    for (auto& b : EL) dfree(c, b);
-    for (auto& b : ER) dfree(c, b);
-    for (auto& b : RC) dfree(c, b);
-    dfree(c, D);
-    dfree(c, X[0]);
-    dfree(c, X[1]);
-    dfree(c, out);
+    for (auto* v : {&EL, &ER, &RC, &S, &D})
+      for (auto& b : *v) dfree(c, b);
+    for (DBuf* b : {&X[0], &X[1], &out, &TR1, &TR2}) dfree(c, *b);
+  };
+  // Independent steps in groups whose scratch stays within 64 MB (or one step's)
+  constexpr int64_t GROUP = 8 << 20;
+  auto group_end = [&](const std::vector<StepPlan>& sp, int from) {
+    int64_t a = 0, b = 0;
+    int k = from;
+    for (; k < L; ++k) {
+      if (k > from && std::max(a + sp[k].t1, b + sp[k].t2) > GROUP) break;
+      a += sp[k].t1;
+      b += sp[k].t2;
+    }
+    ensure(c, c->T1, std::max<int64_t>(a, 1));
+    ensure(c, c->T2, std::max<int64_t>(b, 1));
+    return k;
   };
   try {
-    char* db = u.send(c, MEAS_SLOT);
-    ensure(c, c->T1, t1);
-    ensure(c, c->T2, t2);
     for (int b = 0; b <= L; ++b) {
       dalloc(c, EL[b], std::max<int64_t>(ELl[b].size, 1));
       dalloc(c, ER[b], std::max<int64_t>(ERl[b].size, 1));
     }
     for (int j = 1; j < L; ++j) dalloc(c, RC[j], std::max<int64_t>(spC[j].out.size, 1));
-    dalloc(c, D, dmax);
-    dalloc(c, X[0], xmax);
-    dalloc(c, X[1], xmax);
     dalloc(c, out, int64_t(L) * L + 1);
+    ensure(c, c->T1, t1);
+    ensure(c, c->T2, t2);
+    dalloc(c, TR1, r1);
+    dalloc(c, TR2, r2);
+    char* db = u.send(c, MEAS_SLOT);
     cuda_check(cudaMemsetAsync(out.p, 0, sizeof(double) * (size_t(L) * L + 1), c->stream),
                "correlation clear");
     set_one(c, EL[0]);
     set_one(c, ER[L]);
-    double fl = 0.0;
+    // the identity environments from the two ends, side by side on two streams
+    ensure_env_stream(c);
+    cuda_check(cudaEventRecord(c->env_fork, c->stream), "correlation fork");
+    cuda_check(cudaStreamWaitEvent(c->env_stream, c->env_fork, 0), "correlation fork");
+    JoinGuard join{c};
+    {
+      struct Swap {                          // the second chain: its own stream and scratch
+        dmrg_ctx* c;
+        DBuf &a, &b;
+        cudaStream_t main;
+        Swap(dmrg_ctx* c_, DBuf& a_, DBuf& b_) : c(c_), a(a_), b(b_), main(c_->stream) {
+          turn(c->env_stream);
+        }
+        ~Swap() {
+          cudaEventRecord(c->env_join, c->env_stream);
+          turn(main);
+        }
+        void turn(cudaStream_t s) {
+          c->stream = s;
+          std::swap(c->T1, a);
+          std::swap(c->T2, b);
+        }
+      } swap(c, TR1, TR2);
+      for (int i = L - 1; i >= 0; --i) {
+        run_step(c, spR[i], db, ER[i + 1].p, ER[i + 1].n, st->A[i], ER[i].p, ER[i].n);
+        fl += spR[i].flops();
+      }
+    }
     for (int i = 0; i < L; ++i) {
       run_step(c, spL[i], db, EL[i].p, EL[i].n, st->A[i], EL[i + 1].p, EL[i + 1].n);
       fl += spL[i].flops();
     }
-    for (int i = L - 1; i >= 0; --i) {
-      run_step(c, spR[i], db, ER[i + 1].p, ER[i + 1].n, st->A[i], ER[i].p, ER[i].n);
-      fl += spR[i].flops();
+    join.now();
+    run_pair(c, norm, db, EL[L], ER[L], out.p + int64_t(L) * L);
+    for (int j = 1; j < L;) {                // RC[j] = right step of ER[j+1] through Ca at site j
+      const int e = group_end(spC, j);
+      ManySteps m;
+      Upload v;
+      for (; j < e; ++j) {
+        add_step(m, spC[j], ER[j + 1], st->A[j], RC[j], c->T1.p, c->T2.p);
+        fl += spC[j].flops();
+      }
+      put_many(v, m);
+      run_many(c, m, v.send(c, MEAS_SLOT));
     }
+    D.resize(L);
+    for (int i = 0; i < L;) {                // diagonal
+      const int i0 = i, e = group_end(spD, i);
+      ManySteps m;
+      Upload v;
+      std::vector<PairTask> pt;
+      std::vector<int2> ranges;
+      for (; i < e; ++i) {
+        dalloc(c, D[i], std::max<int64_t>(spD[i].out.size, 1));
+        add_step(m, spD[i], EL[i], st->A[i], D[i], c->T1.p, c->T2.p);
+        const PairPlan pp = plan_pair(st->bond[i + 1], spD[i].out, ERl[i + 1]);
+        check_pair(pp, D[i].n, ER[i + 1].n);
+        const int p0 = int(pt.size());
+        for (PairTask t : pp.t) {
+          t.x_off += element_of(D[i].p);
+          t.y_off += element_of(ER[i + 1].p);
+          pt.push_back(t);
+        }
+        ranges.push_back(make_int2(p0, int(pt.size())));
+        fl += spD[i].flops() + 2.0 * pp.total;
+      }
+      put_many(v, m);
+      const size_t po = v.put(pt), ro = v.put(ranges);
+      char* dv = v.send(c, MEAS_SLOT);
+      run_many(c, m, dv);
+      launch_pair_dot_rows(c->stream, nullptr, 0, nullptr, nullptr,
+                           reinterpret_cast<const PairTask*>(dv + po), int(pt.size()),
+                           reinterpret_cast<const int2*>(dv + ro), e - i0,
+                           out.p + i0 + int64_t(i0) * L, int64_t(L) + 1);
+      for (int k = i0; k < e; ++k) dfree(c, D[k]);
+    }
+    for (auto& b : ER) dfree(c, b);
+    for (int j = 1; j < L; ++j) dalloc(c, S[j], std::max<int64_t>(xs[j], 1));
+    for (int j = 1; j < L;) {                // the rows' starts
+      const int e = group_end(spS, j);
+      ManySteps m;
+      Upload v;
+      for (; j < e; ++j) {
+        add_step(m, spS[j], EL[j - 1], st->A[j - 1], S[j], c->T1.p, c->T2.p);
+        fl += spS[j].flops();
+      }
+      put_many(v, m);
+      run_many(c, m, v.send(c, MEAS_SLOT));
+    }
+    for (auto& b : EL) dfree(c, b);
+    ensure(c, c->T1, f1);
+    ensure(c, c->T2, f2);
+    dalloc(c, X[0], xmax);
+    dalloc(c, X[1], xmax);
+    Upload w;
     for (int j = 1; j < L; ++j) {
-      run_step(c, spC[j], db, ER[j + 1].p, ER[j + 1].n, st->A[j], RC[j].p, RC[j].n);
-      fl += spC[j].flops();
+      if (j >= 2) put_step(w, spF[j]);
+      ppC[j].off = w.put(ppC[j].t);
     }
-    for (int i = 0; i < L; ++i) {
-      run_step(c, spD[i], db, EL[i].p, EL[i].n, st->A[i], D.p, D.n);
-      run_pair(c, ppD[i], db, D, ER[i + 1], out.p + i + int64_t(i) * L);
-      fl += spD[i].flops() + 2.0 * ppD[i].total;
-    }
+    db = w.send(c, MEAS_SLOT);
     for (int j = 1; j < L; ++j) {
       DBuf& xo = X[j & 1];
       const DBuf& xi = X[(j - 1) & 1];
-      if (j >= 2) {
-        run_step(c, spF[j], db, xi.p, xi.n, st->A[j - 1], xo.p, xo.n);
-        fl += spF[j].flops();
-      }
-      const int64_t at = int64_t(j - 1) * xs[j];
-      run_step(c, spS[j], db, EL[j - 1].p, EL[j - 1].n, st->A[j - 1], xo.p + at, xo.n - at);
-      fl += spS[j].flops();
-      run_pair_rows(c, ppC[j], db, xo, j, xs[j], RC[j], out.p + int64_t(j) * L, 1);
-      fl += 2.0 * ppC[j].total * j;
+      // rows 0 .. j-3 at bond j-1 lie in xi, row j-2 is S[j-1]
+      if (j >= 2)
+        run_step_rows(c, spF[j], db, j - 1, xi.p, xs[j - 1], xi.n, &S[j - 1], st->A[j - 1], xo.p,
+                      xs[j], xo.n);
+      check_pair(ppC[j], xs[j], RC[j].n);
+      launch_pair_dot_rows(c->stream, xo.p, xs[j], S[j].p, RC[j].p,
+                           reinterpret_cast<const PairTask*>(db + ppC[j].off),
+                           int(ppC[j].t.size()), nullptr, j, out.p + int64_t(j) * L, 1);
     }
-    run_pair(c, norm, db, EL[L], ER[L], out.p + int64_t(L) * L);
     cuda_check(cudaGetLastError(), "correlation launches");
     std::vector<double> h(size_t(L) * L + 1);
     cuda_check(cudaMemcpyAsync(h.data(), out.p, sizeof(double) * h.size(), cudaMemcpyDeviceToHost,

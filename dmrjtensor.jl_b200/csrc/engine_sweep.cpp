@@ -214,6 +214,13 @@ KrylovRun krylov_solve(dmrg_state* st, const dmrg_params& P, const HeffPlan& hp,
   return kr;
 }
 
+void ensure_env_stream(dmrg_ctx* c) {
+  if (c->env_stream) return;
+  cuda_check(cudaStreamCreateWithFlags(&c->env_stream, cudaStreamNonBlocking), "env stream");
+  cuda_check(cudaEventCreateWithFlags(&c->env_fork, cudaEventDisableTiming), "env event");
+  cuda_check(cudaEventCreateWithFlags(&c->env_join, cudaEventDisableTiming), "env event");
+}
+
 void join_env(dmrg_ctx* c) {
   if (!c->env_pending) return;
   c->env_pending = false;
@@ -566,11 +573,7 @@ void do_sweep(dmrg_state* st, const dmrg_params& P, dmrg_sweep_stats& out) {
   // (their phase timings are taken on one stream) and in served solves (their Heff launches go
   // to the shared batcher).
   const bool overlap = !P.profile && !c->batch;
-  if (overlap && !c->env_stream) {
-    cuda_check(cudaStreamCreateWithFlags(&c->env_stream, cudaStreamNonBlocking), "env stream");
-    cuda_check(cudaEventCreateWithFlags(&c->env_fork, cudaEventDisableTiming), "env event");
-    cuda_check(cudaEventCreateWithFlags(&c->env_join, cudaEventDisableTiming), "env event");
-  }
+  if (overlap) ensure_env_stream(c);
   // on every exit, errors included: the context's own stream back in place, nothing pending
   struct EnvGuard {
     dmrg_ctx* c;

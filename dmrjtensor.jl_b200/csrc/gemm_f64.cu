@@ -48,9 +48,9 @@ __device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b)
 
 template <int BM, int BN, bool TA, bool TB>
 __global__ void __launch_bounds__(THREADS)
-k_gemm_f64(const double* __restrict__ A, const double* __restrict__ B, double* __restrict__ C,
+k_gemm_f64(const double* __restrict__ A0, const double* __restrict__ B0, double* __restrict__ C0,
            const GemmTask* __restrict__ tasks, int ntasks, const GemmSeg* __restrict__ segs,
-           int total_tiles) {
+           int total_tiles, GemmBatch batch) {
   grid_entry();
   using TL = F64Tile<BM, BN>;
   constexpr int LDS_A = TL::LDS_A, LDS_B = TL::LDS_B, MI = TL::MI, NI = TL::NI;
@@ -62,13 +62,13 @@ k_gemm_f64(const double* __restrict__ A, const double* __restrict__ B, double* _
   const int wm = warp & 1, wn = warp >> 1;
   const int g = lane >> 2, t = lane & 3;
 
-  for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
-    int lo = 0, hi = ntasks - 1;
-    while (lo < hi) {
-      int mid = (lo + hi + 1) >> 1;
-      if (tasks[mid].tile0 <= tile) lo = mid; else hi = mid - 1;
-    }
-    const GemmTask tk = tasks[lo];
+  for (int all = blockIdx.x; all < total_tiles * batch.n; all += gridDim.x) {
+    const int set = batch.n > 1 ? all / total_tiles : 0, tile = all - set * total_tiles;
+    const double* A = set == batch.n - 1 && batch.a_last ? batch.a_last
+                                                                    : A0 + set * batch.a;
+    const double* B = B0 + set * batch.b;
+    double* C = C0 + set * batch.c;
+    const GemmTask tk = tasks[find_task(tasks, ntasks, tile)];
     const int local = tile - tk.tile0;
     const int m0 = (local % tk.tiles_m) * BM;
     const int n0 = (local / tk.tiles_m) * BN;
@@ -166,39 +166,40 @@ k_gemm_f64(const double* __restrict__ A, const double* __restrict__ B, double* _
 template <int BM, int BN, bool TA, bool TB>
 void launch_variant(cudaStream_t s, const double* A, const double* B, double* C,
                     const GemmTask* tasks, int ntasks, const GemmSeg* segs, int total_tiles,
-                    int grid_cap) {
+                    int grid_cap, const GemmBatch& batch) {
   constexpr size_t SM = F64Tile<BM, BN>::SMEM;
   raise_smem_limit(reinterpret_cast<const void*>(k_gemm_f64<BM, BN, TA, TB>), SM);
-  int grid = total_tiles < grid_cap ? total_tiles : grid_cap;
+  const int64_t all = int64_t(total_tiles) * batch.n;
+  const int grid = int(all < grid_cap ? all : grid_cap);
   launch_k(k_gemm_f64<BM, BN, TA, TB>, grid, THREADS, SM, s, A, B, C, tasks, ntasks, segs,
-           total_tiles);
+           total_tiles, batch);
   count_launch();
 }
 
 template <int BM, int BN>
 void dispatch_f64(cudaStream_t s, bool transA, bool transB, const double* A, const double* B,
                   double* C, const GemmTask* tasks, int ntasks, const GemmSeg* segs,
-                  int total_tiles, int grid_cap) {
+                  int total_tiles, int grid_cap, const GemmBatch& batch) {
   if (!transA && !transB)
-    launch_variant<BM, BN, false, false>(s, A, B, C, tasks, ntasks, segs, total_tiles, grid_cap);
+    launch_variant<BM, BN, false, false>(s, A, B, C, tasks, ntasks, segs, total_tiles, grid_cap, batch);
   else if (!transA && transB)
-    launch_variant<BM, BN, false, true>(s, A, B, C, tasks, ntasks, segs, total_tiles, grid_cap);
+    launch_variant<BM, BN, false, true>(s, A, B, C, tasks, ntasks, segs, total_tiles, grid_cap, batch);
   else if (transA && !transB)
-    launch_variant<BM, BN, true, false>(s, A, B, C, tasks, ntasks, segs, total_tiles, grid_cap);
+    launch_variant<BM, BN, true, false>(s, A, B, C, tasks, ntasks, segs, total_tiles, grid_cap, batch);
   else
-    launch_variant<BM, BN, true, true>(s, A, B, C, tasks, ntasks, segs, total_tiles, grid_cap);
+    launch_variant<BM, BN, true, true>(s, A, B, C, tasks, ntasks, segs, total_tiles, grid_cap, batch);
 }
 
 }  // namespace
 
 void launch_gemm_f64(cudaStream_t s, int tile, bool transA, bool transB, const double* A,
                      const double* B, double* C, const GemmTask* tasks, int ntasks,
-                     const GemmSeg* segs, int total_tiles, int grid_cap) {
-  if (total_tiles <= 0 || ntasks <= 0) return;
+                     const GemmSeg* segs, int total_tiles, int grid_cap, const GemmBatch& batch) {
+  if (total_tiles <= 0 || ntasks <= 0 || batch.n <= 0) return;
   if (tile == 32)
-    dispatch_f64<32, 32>(s, transA, transB, A, B, C, tasks, ntasks, segs, total_tiles, grid_cap);
+    dispatch_f64<32, 32>(s, transA, transB, A, B, C, tasks, ntasks, segs, total_tiles, grid_cap, batch);
   else
-    dispatch_f64<64, 64>(s, transA, transB, A, B, C, tasks, ntasks, segs, total_tiles, grid_cap);
+    dispatch_f64<64, 64>(s, transA, transB, A, B, C, tasks, ntasks, segs, total_tiles, grid_cap, batch);
 }
 
 // Raises (never lowers) the dynamic shared-memory limit of a kernel on the current device. The

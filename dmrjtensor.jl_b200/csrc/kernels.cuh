@@ -104,9 +104,17 @@ constexpr int GEMM_SMALL_TILE = 32;   // the second tile shape of the FP64 GEMM 
 // Persistent grouped FP64 GEMM (DMMA m8n8k4 tensor-core path), square tiles of `tile` = 64 or
 // 32 (the task list's tile counts must match). Every output element accumulates its K products
 // in the same order for both tile shapes, so the results are bit-identical.
+// The list repeated for n sets of operands at fixed strides (elements); the last set's A operand
+// may lie elsewhere (a_last).
+struct GemmBatch {
+  int n = 1;
+  int64_t a = 0, b = 0, c = 0;
+  const double* a_last = nullptr;
+};
 void launch_gemm_f64(cudaStream_t s, int tile, bool transA, bool transB, const double* A,
                      const double* B, double* C, const GemmTask* tasks, int ntasks,
-                     const GemmSeg* segs, int total_tiles, int grid_cap);
+                     const GemmSeg* segs, int total_tiles, int grid_cap,
+                     const GemmBatch& batch = GemmBatch{});
 
 // Split-precision grouped GEMM on tcgen05 (FP32 accumulation in TMEM, FP64 in/out), direct form
 // with tiles of TF32_TILE_M x TF32_TILE_N_DIRECT: form SPLIT_TF32X3 = three TF32 products,
@@ -156,8 +164,10 @@ void launch_gemm_split_images(int form, int bn, cudaStream_t s, const unsigned c
 // slot of the context's status words that the split-precision GEMM sets on a timeout
 constexpr int STATUS_MMA = 8;
 
+// (nb: the list repeated for nb blocks of input and output at the given strides)
 void launch_mix(cudaStream_t s, const double* in, double* out, const MixTask* tasks, int ntasks,
-                const MixTerm* terms, int total_tiles);
+                const MixTerm* terms, int total_tiles, int nb = 1, int64_t in_stride = 0,
+                int64_t out_stride = 0);
 
 void launch_copy(cudaStream_t s, const double* src, double* dst, const CopyTask* tasks,
                  int ntasks, int total_tiles);
@@ -213,11 +223,12 @@ void launch_ritz(cudaStream_t s, double* scal, int kdim, double tau, bool expo);
 // out[0] = sum over the pair tasks (total elements `total`; deterministic order)
 void launch_pair_dot(cudaStream_t s, const double* X, const double* Y, const PairTask* tasks,
                      int ntasks, int64_t total, double* partial, double* out);
-// out[r * out_stride] = sum over the pair tasks with X shifted by r * x_stride, r < nrows (one
-// block per row; fixed order)
-void launch_pair_dot_rows(cudaStream_t s, const double* X, int64_t x_stride, const double* Y,
-                          const PairTask* tasks, int ntasks, int nrows, double* out,
-                          int64_t out_stride);
+// out[r * out_stride], r < nrows, one block per row (fixed order): the sum over the pair tasks with
+// X shifted by r * x_stride; the last row's X may lie elsewhere (x_last). With `ranges` row r sums
+// tasks [ranges[r].x, ranges[r].y) instead, X and Y unshifted.
+void launch_pair_dot_rows(cudaStream_t s, const double* X, int64_t x_stride, const double* x_last,
+                          const double* Y, const PairTask* tasks, int ntasks, const int2* ranges,
+                          int nrows, double* out, int64_t out_stride);
 // The vector work between two Heff applications as one launch (krylov.cu), with the numbers of the
 // launches above bit for bit: false (nothing launched) for vectors above KRY_MAX elements.
 //   KRY_NORMALISE  s[j] = <K,K>, K /= |K|                       (mdot, scale_rsqrt)

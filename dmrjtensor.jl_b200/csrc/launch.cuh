@@ -26,6 +26,24 @@ __device__ __forceinline__ void grid_entry() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// The task that owns `tile` in a list sorted by first tile (tile0): the whole block looks at
+// blockDim.x evenly spread tasks at once and narrows the range to the gap between two of them, so
+// a list of up to blockDim.x tasks costs one round of loads where a binary search by every thread
+// costs log2(ntasks) dependent ones (~600 cycles each from L2: the mixing and copy launches of a
+// U(1) sweep took 9.4 and 6.1 us on average against 7.8 and 5.3 us). All threads call it.
+template <class Task>
+__device__ __forceinline__ int find_task(const Task* __restrict__ tasks, int ntasks, int tile) {
+  int lo = 0, n = ntasks;                  // the owner is in [lo, lo + n)
+  while (n > 1) {
+    const int step = (n + int(blockDim.x) - 1) / int(blockDim.x);
+    const int i = int(threadIdx.x) * step;
+    const int c = __syncthreads_count(i < n && tasks[lo + i].tile0 <= tile);
+    lo += (c - 1) * step;
+    n = min(step, n - (c - 1) * step);
+  }
+  return lo;
+}
+
 // kernel<<<grid, block, smem, s>>>(args...) with programmatic stream serialisation allowed.
 // Errors are left for the caller's cudaGetLastError().
 template <typename... P, typename... A>

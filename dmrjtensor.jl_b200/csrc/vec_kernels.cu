@@ -55,17 +55,16 @@ __device__ void finish_rows(const double* partial, int nb, int k, double* out, u
   if (threadIdx.x == 0) *counter = 0u;
 }
 
-__global__ void k_mix(const double* __restrict__ in, double* __restrict__ out,
+__global__ void k_mix(const double* __restrict__ in0, double* __restrict__ out0,
                       const MixTask* __restrict__ tasks, int ntasks,
-                      const MixTerm* __restrict__ terms, int total_tiles) {
+                      const MixTerm* __restrict__ terms, int total_tiles, int nb,
+                      int64_t in_stride, int64_t out_stride) {
   grid_entry();
-  for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
-    int lo = 0, hi = ntasks - 1;
-    while (lo < hi) {
-      int mid = (lo + hi + 1) >> 1;
-      if (tasks[mid].tile0 <= tile) lo = mid; else hi = mid - 1;
-    }
-    const MixTask tk = tasks[lo];
+  for (int all = blockIdx.x; all < total_tiles * nb; all += gridDim.x) {
+    const int set = nb > 1 ? all / total_tiles : 0, tile = all - set * total_tiles;
+    const double* in = in0 + set * in_stride;
+    double* out = out0 + set * out_stride;
+    const MixTask tk = tasks[find_task(tasks, ntasks, tile)];
     const int c0 = (tile - tk.tile0) * MIX_COLS;
     const int ncol = min(MIX_COLS, tk.cols - c0);
     if (tk.rows >= MIX_TALL) {
@@ -117,12 +116,7 @@ __global__ void k_copy(const double* __restrict__ src, double* __restrict__ dst,
                        const CopyTask* __restrict__ tasks, int ntasks, int total_tiles) {
   grid_entry();
   for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
-    int lo = 0, hi = ntasks - 1;
-    while (lo < hi) {
-      int mid = (lo + hi + 1) >> 1;
-      if (tasks[mid].tile0 <= tile) lo = mid; else hi = mid - 1;
-    }
-    const CopyTask tk = tasks[lo];
+    const CopyTask tk = tasks[find_task(tasks, ntasks, tile)];
     const int c0 = (tile - tk.tile0) * MIX_COLS;
     const int ncol = min(MIX_COLS, tk.cols - c0);
     const int nel = ncol * tk.rows;
@@ -199,22 +193,43 @@ __global__ void k_pair_dot(const double* __restrict__ X, const double* __restric
   if (arrive_last(counter)) finish_rows(partial, gridDim.x, 1, out, counter);
 }
 
-__global__ void k_pair_dot_rows(const double* __restrict__ X, int64_t x_stride,
-                                const double* __restrict__ Y, const PairTask* __restrict__ tasks,
-                                int ntasks, double* out, int64_t out_stride) {
+// One row per block. X runs along its rows and Y along its columns, so Y goes through shared memory
+// in 32 x 32 tiles (read straight, a warp's lanes are `cols` apart in Y).
+__global__ void __launch_bounds__(RED_THREADS)
+k_pair_dot_rows(const double* __restrict__ X, int64_t x_stride, const double* __restrict__ x_last,
+                const double* __restrict__ Y, const PairTask* __restrict__ tasks, int ntasks,
+                const int2* __restrict__ ranges, double* out, int64_t out_stride) {
   grid_entry();
+  __shared__ double ty[32][33];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const double* Xr = X + int64_t(blockIdx.x) * x_stride;
+  if (x_last && blockIdx.x == gridDim.x - 1) Xr = x_last;
+  int k0 = 0, k1 = ntasks;
+  if (ranges) { k0 = ranges[blockIdx.x].x; k1 = ranges[blockIdx.x].y; }
   double acc = 0.0;
-  for (int k = 0; k < ntasks; ++k) {
+  for (int k = k0; k < k1; ++k) {
     const PairTask tk = tasks[k];
-    const int64_t n = int64_t(tk.rows) * tk.cols;
-    for (int64_t q = threadIdx.x; q < n; q += blockDim.x) {
-      const int64_t r = q % tk.rows, c = q / tk.rows;
-      acc += Xr[tk.x_off + q] * Y[tk.y_off + c + r * tk.cols];
-    }
+    const double* xs = Xr + tk.x_off;
+    const double* ys = Y + tk.y_off;
+    for (int r0 = 0; r0 < tk.rows; r0 += 32)
+      for (int c0 = 0; c0 < tk.cols; c0 += 32) {
+        const int c = c0 + lane, r = r0 + lane;
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int rr = wid + 8 * u;
+          ty[rr][lane] = r0 + rr < tk.rows && c < tk.cols ? ys[c + int64_t(r0 + rr) * tk.cols] : 0.0;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int cc = wid + 8 * u;
+          if (r < tk.rows && c0 + cc < tk.cols)
+            acc += xs[r + int64_t(c0 + cc) * tk.rows] * ty[lane][cc];
+        }
+      }
   }
   __shared__ double red[RED_THREADS / 32];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   acc = warp_sum(acc);
   if (lane == 0) red[wid] = acc;
   __syncthreads();
@@ -518,10 +533,13 @@ int grid_for(int64_t n) {
 }  // namespace
 
 void launch_mix(cudaStream_t s, const double* in, double* out, const MixTask* tasks, int ntasks,
-                const MixTerm* terms, int total_tiles) {
-  if (total_tiles <= 0) return;
-  int grid = total_tiles < 4096 ? total_tiles : 4096;
-  launch_k(k_mix, grid, 256, 0, s, in, out, tasks, ntasks, terms, total_tiles);
+                const MixTerm* terms, int total_tiles, int nb, int64_t in_stride,
+                int64_t out_stride) {
+  if (total_tiles <= 0 || nb <= 0) return;
+  const int64_t all = int64_t(total_tiles) * nb;
+  const int grid = int(all < 4096 ? all : 4096);
+  launch_k(k_mix, grid, 256, 0, s, in, out, tasks, ntasks, terms, total_tiles, nb, in_stride,
+           out_stride);
   count_launch();
 }
 
@@ -593,12 +611,12 @@ void launch_pair_dot(cudaStream_t s, const double* X, const double* Y, const Pai
   count_launch();
 }
 
-void launch_pair_dot_rows(cudaStream_t s, const double* X, int64_t x_stride, const double* Y,
-                          const PairTask* tasks, int ntasks, int nrows, double* out,
-                          int64_t out_stride) {
+void launch_pair_dot_rows(cudaStream_t s, const double* X, int64_t x_stride, const double* x_last,
+                          const double* Y, const PairTask* tasks, int ntasks, const int2* ranges,
+                          int nrows, double* out, int64_t out_stride) {
   if (nrows <= 0) return;
-  launch_k(k_pair_dot_rows, nrows, RED_THREADS, 0, s, X, x_stride, Y, tasks, ntasks, out,
-           out_stride);
+  launch_k(k_pair_dot_rows, nrows, RED_THREADS, 0, s, X, x_stride, x_last, Y, tasks, ntasks, ranges,
+           out, out_stride);
   count_launch();
 }
 
