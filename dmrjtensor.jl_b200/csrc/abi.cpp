@@ -1078,13 +1078,20 @@ int dmrg_test_syevt(dmrg_ctx* c, int nmat, const int* n, const int* k, double* A
     std::vector<TridTask> tasks;
     int64_t oa = 0, ow = ta, ows = ta + tw, ou = ta + 4 * tw;
     for (int i = 0; i < nmat; ++i) {
-      TridTask t{oa, ow, ows, ou, n[i], k[i], 0};
+      TridTask t{};
+      t.a_off = oa;
+      t.w_off = ow;
+      t.ws_off = ows;
+      t.u_off = ou;
+      t.n = n[i];
+      t.keep = k[i];
       tasks.push_back(t);
       oa += int64_t(n[i]) * n[i];
       ow += n[i];
       ows += 3 * n[i];
       ou += int64_t(n[i]) * k[i];
     }
+    set_trid_paths(tasks);
     DBuf buf;
     dalloc(c, buf, ta + 4 * tw + tu);
     cuda_check(cudaMemcpyAsync(buf.p, A, ta * 8, cudaMemcpyHostToDevice, c->stream), "A");

@@ -479,6 +479,7 @@ void measure_correlation(dmrg_state* st, int d, const double* Cc, const double* 
 // Tridiagonal-path eigenvalues of every task (n <= SYEVT_MID_NMAX; small and mid-size blocks in
 // one launch each), then the kept eigenvectors (tasks with keep > 0; mid-size blocks use c->W
 // as workspace). Offsets are checked against nbase before any launch.
+void set_trid_paths(std::vector<TridTask>& t);
 void run_trid_eigvals(dmrg_ctx* c, double* base, int64_t nbase, const std::vector<TridTask>& t,
                       int slot);
 void run_trid_vectors(dmrg_ctx* c, double* base, int64_t nbase, std::vector<TridTask> t,

@@ -10,7 +10,7 @@ namespace {
 void check_trid(const std::vector<TridTask>& ts, int64_t nbase, bool vectors) {
   for (const TridTask& t : ts) {
     const int64_t nn = int64_t(t.n) * t.n;
-    if (t.n <= 0 || t.n > SYEVT_MID_NMAX || t.a_off < 0 || t.a_off + nn > nbase ||
+    if (t.n <= 0 || t.n > (t.mid ? SYEVT_MID_NMAX : SYEVT_NMAX) || t.a_off < 0 || t.a_off + nn > nbase ||
         t.w_off < 0 || t.w_off + t.n > nbase || t.ws_off < 0 || t.ws_off + 3 * t.n > nbase)
       fail(DMRG_ERR_ARG, "internal plan check failed: tridiagonal eigensolver task");
     if (vectors && (t.keep < 0 || t.keep > t.n || t.u_off < 0 ||
@@ -20,6 +20,12 @@ void check_trid(const std::vector<TridTask>& ts, int64_t nbase, bool vectors) {
 }
 }  // namespace
 
+void set_trid_paths(std::vector<TridTask>& t) {
+  int nmax = 0;
+  for (const TridTask& x : t) nmax = std::max(nmax, x.n);
+  for (TridTask& x : t) x.mid = nmax > SYEVT_ROUTE ? 1 : 0;
+}
+
 void run_trid_eigvals(dmrg_ctx* c, double* base, int64_t nbase, const std::vector<TridTask>& t,
                       int slot) {
   check_trid(t, nbase, false);
@@ -27,7 +33,7 @@ void run_trid_eigvals(dmrg_ctx* c, double* base, int64_t nbase, const std::vecto
   int ns = 0;
   int64_t sum = 0;
   for (const TridTask& x : t) {
-    if (x.n <= SYEVT_NMAX) { small.push_back(x); ns = std::max(ns, x.n); }
+    if (!x.mid) { small.push_back(x); ns = std::max(ns, x.n); }
     else { mid.push_back(x); sum += x.n; }
   }
   // the largest first: not all clusters of a long list are resident at once
@@ -54,7 +60,7 @@ void run_trid_vectors(dmrg_ctx* c, double* base, int64_t nbase, std::vector<Trid
   int64_t xw = 0;
   for (TridTask x : t) {
     if (x.keep <= 0) continue;
-    if (x.n <= SYEVT_NMAX) {
+    if (!x.mid) {
       small.push_back(x);
       ns = std::max(ns, x.n);
       ks = std::max(ks, x.keep);

@@ -291,6 +291,7 @@ void plan_rho(dmrg_ctx* c, std::vector<Group>& G, bool rows, const dmrg_params& 
       rs.uoff[gi] = g.roff;      // block Jacobi returns the eigenvectors in place
     }
   }
+  set_trid_paths(rs.ttasks);
   const int64_t ews = eig_workspace(rs.etasks);
   ensure(c, c->M, std::max<int64_t>(rs.mtot, 1));
   ensure(c, c->R, std::max<int64_t>(rs.J0 + ews, 1));

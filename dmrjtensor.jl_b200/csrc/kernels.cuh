@@ -66,8 +66,8 @@ struct EigTask {
   int n, pad;
 };
 
-// Tridiagonal eigensolver for density-matrix blocks with n <= SYEVT_NMAX (syevt.cu, shared
-// memory) and SYEVT_NMAX < n <= SYEVT_MID_NMAX (syevt_cluster.cu and syevt_mid.cu; the line is
+// Tridiagonal eigensolver for density-matrix blocks: one CTA per block for n <= SYEVT_NMAX
+// (syevt.cu), clusters for n <= SYEVT_MID_NMAX (syevt_cluster.cu and syevt_mid.cu; that line is
 // where the smaller kernels' shared memory ends: at n = 1024 with 512 vectors 7.5 ms against about
 // 90 ms of block Jacobi sweeps).
 constexpr int SYEVT_NMAX = 112;
@@ -79,8 +79,16 @@ struct TridTask {
   int64_t ws_off;  // 3n workspace: d, e, tau
   int64_t u_off;   // n x keep eigenvectors (launch 2)
   int n, keep;
-  int64_t x_off;   // mid-size launches 2-3: workspace offset (syevt_mid_workspace(n, keep) doubles)
+  int64_t x_off;   // mid-size launches: workspace offset (syevt_mid_workspace(n, keep) doubles)
+  int mid = 0;     // the block takes the mid-size kernels (set_trid_paths)
+  int pad = 0;
 };
+// The blocks of one step run side by side, so they take one path where they can: the mid-size
+// kernels for all of them once the largest has more than SYEVT_ROUTE states. One CTA per block is
+// as fast up to there (values and vectors, largest block 48 states: 85 against 80 us), above it the
+// clusters win (85 states: 185 against 135 us), and both paths one after the other would cost
+// their sum.
+constexpr int SYEVT_ROUTE = 40;
 size_t syevt_smem_vals(int n);
 size_t syevt_smem_vecs(int n, int k);
 void launch_trid_eigvals(cudaStream_t s, double* base, const TridTask* tasks, int ntasks, int max_n);

@@ -1,4 +1,4 @@
-// syevt_cluster.cu -- tridiagonalisation of mid-size density-matrix blocks by a thread-block
+// syevt_cluster.cu -- tridiagonalisation of larger density-matrix blocks by a thread-block
 // cluster, and the eigenvalues of the tridiagonal matrices by the whole chip.
 //
 // k_trid_cluster: one cluster of c CTAs per block (c = 8, or 16 for large blocks). The matrix is
@@ -267,7 +267,7 @@ struct Lo {
   static constexpr int v = V;
 };
 
-// Blocks of 3 <= n <= HN with up to 32 RM rows and HW CC C columns.
+// Blocks of n <= HN with up to 32 RM rows and HW CC C columns.
 template <int RM, int CC, int C>
 __global__ void __launch_bounds__(HTX, 1)
 k_trid_cluster(double* __restrict__ base, const TridTask* __restrict__ tasks) {
@@ -276,7 +276,19 @@ k_trid_cluster(double* __restrict__ base, const TridTask* __restrict__ tasks) {
   constexpr int EPT = (32 * RM + HTX - 1) / HTX;          // elements per thread
   const TridTask tk = tasks[blockIdx.x / C];
   const int k0 = trid_lead_steps(tk.n), ld = tk.n, n = ld - k0;   // the block from column k0 on
-  if (n < 3 || n > 32 * RM || n > HW * CC * C) return;   // the same in all of the cluster
+  if (n > 32 * RM || n > HW * CC * C) return;      // the same in all of the cluster
+  if (n < 3) {                                     // tridiagonal as it is
+    if (cluster_rank() == 0 && threadIdx.x == 0 && n > 0) {
+      const double* A = base + tk.a_off;
+      double* ws = base + tk.ws_off;
+      for (int i = 0; i < n; ++i) {
+        ws[i] = A[i * (n + 1)];
+        ws[n + i] = i + 1 < n ? A[i * n + i + 1] : 0.0;
+        ws[2 * n + i] = 0.0;
+      }
+    }
+    return;
+  }
   __shared__ __align__(16) double2 pc[2][HN];      // (x.B(:,j), pivot-row element j), by parity
   __shared__ __align__(16) double kw[2][C];        // the CTAs' shares of x.B x
   __shared__ __align__(16) double kp[HW + 1];      // the warps' shares
@@ -595,7 +607,8 @@ void launch_trid_cluster(cudaStream_t s, double* base, const TridTask* tasks, in
   // 0.49 against 0.57 ms; below 256 rows the two are equal), but only eight such clusters fit on
   // the chip at once
   const bool wide = max_n > 352 || ntasks <= 8;
-  if (max_n <= 160) go(k_trid_cluster<5, 3, 8>, 8);
+  if (max_n <= 112) go(k_trid_cluster<4, 2, 8>, 8);
+  else if (max_n <= 160) go(k_trid_cluster<5, 3, 8>, 8);
   else if (max_n <= 224) go(k_trid_cluster<7, 4, 8>, 8);
   else if (max_n <= 256) go(k_trid_cluster<8, 5, 8>, 8);
   else if (!wide) go(k_trid_cluster<11, 7, 8>, 8);

@@ -1,5 +1,5 @@
-// syevt_mid.cu -- eigenvectors of mid-size density-matrix blocks, SYEVT_NMAX < n <= SYEVT_MID_NMAX
-// (their tridiagonal matrices and eigenvalues come from syevt_cluster.cu). Every part runs on many
+// syevt_mid.cu -- eigenvectors of the density-matrix blocks of a step whose largest has more than
+// SYEVT_ROUTE (up to SYEVT_MID_NMAX) states (their tridiagonal matrices and eigenvalues come from syevt_cluster.cu). Every part runs on many
 // CTAs; one CTA per block for all of it took 1.6 + 0.54 ms at n = 345 with 200 kept vectors.
 //   * k_mid_invit: inverse iteration, one thread per kept vector, a few vectors per CTA so that
 //     their LU factors and the vectors stay in shared memory (with 32 vectors per CTA and the
@@ -91,7 +91,7 @@ k_mid_runs(double* __restrict__ base, const TridTask* __restrict__ tasks,
   grid_entry();
   const TridTask tk = tasks[blockIdx.x];
   const int n = tk.n, kk = tk.keep;
-  if (n < 3 || kk <= 0) return;
+  if (n < 1 || kk <= 0) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const double* W = base + tk.w_off;
   const double tol = 1e-12 * fmax(fmax(fabs(W[0]), fabs(W[n - 1])), 1e-300);
@@ -148,7 +148,7 @@ k_mid_gram(double* __restrict__ base, const TridTask* __restrict__ tasks, double
   grid_entry();
   const TridTask tk = tasks[blockIdx.y];
   const int n = tk.n, kk = tk.keep;
-  if (n < 3 || kk <= 0) return;
+  if (n < 1 || kk <= 0) return;
   const int nt = (kk + 31) >> 5;
   if (int(blockIdx.x) >= nt * (nt + 1) / 2) return;
   int I = 0, x = blockIdx.x;
@@ -221,7 +221,7 @@ k_mid_apply(double* __restrict__ base, const TridTask* __restrict__ tasks,
   grid_entry();
   const TridTask tk = tasks[blockIdx.y];
   const int n = tk.n, kk = tk.keep, r0 = blockIdx.x * AR;
-  if (n < 3 || kk <= 0 || r0 >= n) return;
+  if (n < 1 || kk <= 0 || r0 >= n) return;
   double* X = xws + tk.x_off;
   MidCtl* ctl = mid_ctl(X, n, kk);
   if (!round_active(ctl, pass)) return;
@@ -287,7 +287,7 @@ k_mid_cholqr(double* __restrict__ base, const TridTask* __restrict__ tasks,
   grid_entry();
   const TridTask tk = tasks[blockIdx.x];
   const int n = tk.n, kk = tk.keep;
-  if (n < 3 || kk <= 0) return;
+  if (n < 1 || kk <= 0) return;
   double* X = xws + tk.x_off;
   if (mid_ctl(X, n, kk)->slow == 0ull) return;
   const int ldz = kk | 1;
@@ -531,7 +531,7 @@ k_mid_back(double* __restrict__ base, const TridTask* __restrict__ tasks,
   constexpr int KR = RM <= 16 ? RM : 1;          // reflectors kept in registers between their uses
   const TridTask tk = tasks[blockIdx.y];
   const int n = tk.n, kk = tk.keep, tid = threadIdx.x, lane = tid & 31;
-  if (n < 3 || n > LD || int(blockIdx.x) * NV * BW >= kk) return;
+  if (n < 1 || n > LD || int(blockIdx.x) * NV * BW >= kk) return;
   extern __shared__ __align__(16) double sm[];
   double* stau = sm + BSTAGES * 2 * LD;          // n
   const int q0 = NV * (blockIdx.x * BW + (tid >> 5));
@@ -659,7 +659,8 @@ void launch_trid_mid_vectors(cudaStream_t s, double* base, const TridTask* tasks
   raise_smem_limit(reinterpret_cast<const void*>(k_mid_cholqr), sm);
   launch_k(k_mid_cholqr, ntasks, MT, sm, s, base, tasks, xws, kg);
   auto back = [&](auto launch) { launch(s, base, tasks, ntasks, max_n, max_k, xws); };
-  if (max_n <= 160) back(launch_back<5, 2>);
+  if (max_n <= 128) back(launch_back<4, 2>);
+  else if (max_n <= 160) back(launch_back<5, 2>);
   else if (max_n <= 256) back(launch_back<8, 2>);
   else if (max_n <= 352) back(launch_back<11, 2>);
   else if (max_n <= 512) back(launch_back<16, 2>);
