@@ -168,10 +168,10 @@ def graph_report(pkg, ctx, dev, mfin, args, flush):
 
 def autotune_report(pkg, ctx, dev, mfin, args, flush):
     """Tile autotuner on the resident state: profiled sweeps with the tuned tile shapes and with
-    fixed 64 x 64 tiles (the numbers are identical; the GEMM device time and the sweep time are
+    fixed 32 x 32 tiles (the numbers are identical; the GEMM device time and the sweep time are
     compared), plus the tuner's table size."""
     rec = {}
-    for name, tune in (("fixed_64x64", False), ("tuned", True)):
+    for name, tune in (("fixed_32x32", False), ("tuned", True)):
         ms, gs, en = [], [], []
         for _ in range(3):
             flush()
@@ -181,8 +181,8 @@ def autotune_report(pkg, ctx, dev, mfin, args, flush):
             en.append(st["energy"])
         rec[name] = {"sweep_ms": min(ms), "heff_gemm_ms": min(gs)}
     sig, decided, small = ctx.tuner()
-    rec.update({"signatures": sig, "decided": decided, "won_by_32x32": small,
-                "gemm_speedup": rec["fixed_64x64"]["heff_gemm_ms"] / rec["tuned"]["heff_gemm_ms"]})
+    rec.update({"signatures": sig, "decided": decided, "won_by_32x16": small,
+                "gemm_speedup": rec["fixed_32x32"]["heff_gemm_ms"] / rec["tuned"]["heff_gemm_ms"]})
     return rec
 
 

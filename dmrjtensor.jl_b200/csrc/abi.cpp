@@ -1129,6 +1129,8 @@ int dmrg_test_gemm(dmrg_ctx* c, int transA, int transB, int M, int N, int K, con
     g.tB = transB != 0;
     g.add(0, ldc, M, N, 1.0, 0.0);
     g.seg(0, lda, 0, ldb, K);
+    tuner_collect(c);
+    tune_gemm(c, g);       // repeated calls take both tile shapes
     Upload u;
     u.put(g);
     char* db = u.send(c, 0);

@@ -16,7 +16,7 @@
 // larger step does not hold the others up for long), or when a solve leaves its sweeps. While a
 // round runs on the GPU the arriving requests collect for the next one: the GPU is never idle
 // for a request that waits. Each task's tiles are computed exactly as in a launch of its own
-// (tiles are independent; FP64 lists use 64 x 64 tiles, split lists the direct form), so a
+// (tiles are independent; FP64 lists use 32 x 32 tiles, split lists the direct form), so a
 // solve's numbers do not depend on the solves it is batched with.
 #include <algorithm>
 #include <chrono>
@@ -178,8 +178,8 @@ void fire(HeffBatcher* b) {
       const auto* t3 = reinterpret_cast<const GemmTask*>(dbase + m.o[4]);
       const auto* s3 = reinterpret_cast<const GemmSeg*>(dbase + m.o[5]);
       if (f == 0) {
-        launch_gemm_f64(b->stream, GEMM_BM, m.g1.tA, m.g1.tB, nullptr, nullptr, nullptr, t1,
-                        int(m.g1.tasks.size()), s1, m.g1.tiles, b->nsm * 4);
+        launch_gemm_f64(b->stream, GEMM_BN, m.g1.tA, m.g1.tB, nullptr, nullptr, nullptr, t1,
+                        int(m.g1.tasks.size()), s1, m.g1.tiles, b->nsm);
       } else {
         launch_gemm_split(f, b->stream, m.g1.tA, m.g1.tB, nullptr, nullptr, nullptr, t1,
                           int(m.g1.tasks.size()), s1, m.g1.tiles, b->nsm * 3, b->d_err);
@@ -187,8 +187,8 @@ void fire(HeffBatcher* b) {
       if (m.mix.tiles > 0)
         launch_mix(b->stream, nullptr, nullptr, mt, int(m.mix.tasks.size()), mm, m.mix.tiles);
       if (f == 0) {
-        launch_gemm_f64(b->stream, GEMM_BM, m.g3.tA, m.g3.tB, nullptr, nullptr, nullptr, t3,
-                        int(m.g3.tasks.size()), s3, m.g3.tiles, b->nsm * 4);
+        launch_gemm_f64(b->stream, GEMM_BN, m.g3.tA, m.g3.tB, nullptr, nullptr, nullptr, t3,
+                        int(m.g3.tasks.size()), s3, m.g3.tiles, b->nsm);
       } else {
         launch_gemm_split(f, b->stream, m.g3.tA, m.g3.tB, nullptr, nullptr, nullptr, t3,
                           int(m.g3.tasks.size()), s3, m.g3.tiles, b->nsm * 3, b->d_err);

@@ -160,13 +160,13 @@ namespace dmrg {
 struct HeffBatcher;   // shared Heff launches of a server's solves (batch.cpp)
 // Tile-shape autotuner of the FP64 grouped GEMM. A list's signature quantises its block-size
 // histogram (FLOP-weighted mean M, N and K, task count, total FLOPs, transposes, in half-octave
-// buckets). The first launches of a new signature are timed once in each tile shape (64 x 64 and
-// 32 x 32) with CUDA events; from then on the faster shape is used for that signature (64 x 64
-// unless 32 x 32 is more than 3% faster). Both shapes give bit-identical results, so the choice
+// buckets). The first launches of a new signature are timed once in each tile shape (32 x 32 and
+// 32 x 16) with CUDA events; from then on the faster shape is used for that signature (32 x 32
+// unless 32 x 16 is more than 3% faster). Both shapes give bit-identical results, so the choice
 // never changes a number, only the time. The table lives in the context (one device).
 struct GemmTuner {
   struct Entry {
-    int trials[2] = {0, 0};       // [0] 64 x 64, [1] 32 x 32
+    int trials[2] = {0, 0};       // [0] 32 x 32, [1] 32 x 16
     double best[2] = {1e30, 1e30};
     int choice = -1;
   };
@@ -313,7 +313,7 @@ void run_gemm(dmrg_ctx* c, const GemmList& g, char* dbase, const double* A, int6
 // The launch wrappers' bounds checks alone (DMRG_ERR_ARG on a violation).
 void check_gemm_list(const GemmList& g, int64_t nA, int64_t nB, int64_t nC);
 void check_mix_list(const MixList& m, int64_t nin, int64_t nout);
-// Picks the FP64 tile shape of a list (before its upload): retiles it to 32 x 32 when the tuner
+// Picks the FP64 tile shape of a list (before its upload): retiles it to 32 x 16 when the tuner
 // says so or while that shape is on trial, and marks trial launches for timing.
 void tune_gemm(dmrg_ctx* c, GemmList& g);
 // Folds the timings of completed trial launches into the tuner (no synchronisation).

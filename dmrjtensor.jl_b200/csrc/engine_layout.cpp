@@ -485,8 +485,7 @@ void run_gemm(dmrg_ctx* c, const GemmList& g, char* dbase, const double* A, int6
               const double* B, int64_t nB, double* C, int64_t nC) {
   if (g.tiles == 0) return;
   check_gemm_list(g, nA, nB, nC);
-  if ((g.bm != GEMM_BM || g.bn != GEMM_BN) &&
-      (g.bm != GEMM_SMALL_TILE || g.bn != GEMM_SMALL_TILE))
+  if (g.bm != GEMM_BM || (g.bn != GEMM_BN && g.bn != GEMM_BN_SMALL))
     bad_plan("gemm tiling");
   GemmTuner::Pending tp{};
   const bool timed = g.tune_trial && g.tune_key != 0 && !c->capturing;
@@ -500,12 +499,12 @@ void run_gemm(dmrg_ctx* c, const GemmList& g, char* dbase, const double* A, int6
       }
     }
     tp.key = g.tune_key;
-    tp.variant = g.bm == GEMM_SMALL_TILE ? 1 : 0;
+    tp.variant = g.bn == GEMM_BN_SMALL ? 1 : 0;
     cudaEventRecord(tp.a, c->stream);
   }
-  launch_gemm_f64(c->stream, g.bm, g.tA, g.tB, A, B, C,
+  launch_gemm_f64(c->stream, g.bn, g.tA, g.tB, A, B, C,
                   reinterpret_cast<const GemmTask*>(dbase + g.t_off), int(g.tasks.size()),
-                  reinterpret_cast<const GemmSeg*>(dbase + g.s_off), g.tiles, c->nsm * 4);
+                  reinterpret_cast<const GemmSeg*>(dbase + g.s_off), g.tiles, c->nsm);
   if (timed) {
     cudaEventRecord(tp.b, c->stream);
     c->tuner.pending.push_back(tp);
@@ -550,7 +549,7 @@ void tune_gemm(dmrg_ctx* c, GemmList& g) {
     g.tune_trial = 1;
   }
   if (v == 1) g = [&] {
-    GemmList r = retile(g, GEMM_SMALL_TILE, GEMM_SMALL_TILE);
+    GemmList r = retile(g, GEMM_BM, GEMM_BN_SMALL);
     r.tune_key = g.tune_key;
     r.tune_trial = g.tune_trial;
     return r;

@@ -130,19 +130,21 @@ void run_pair(dmrg_ctx* c, const PairPlan& pp, char* db, const DBuf& X, const DB
                   int(pp.t.size()), pp.total, c->d_partial, out);
 }
 
-// The tile shape of a measurement list: 32 x 32 where the blocks are small (a 64 x 64 tile of a
-// 30 x 60 block is mostly padding), 64 x 64 otherwise.
+
+// The tile shape of a measurement list (not timed by the tuner): 32 x 16 where the blocks are
+// small (a 32 x 32 tile of a 30 x 45 block is half padding) or the list is too short to give every
+// SM two 32 x 32 tiles.
 void pick_tiles(GemmList& g) {
   double area = 0.0, n = 0.0;
   for (const GemmTask& t : g.tasks) { area += double(t.M) * t.N; n += 1.0; }
-  if (n > 0 && area < 96.0 * 96.0 * n) g = retile(g, GEMM_SMALL_TILE, GEMM_SMALL_TILE);
+  if (area < 48.0 * 48.0 * n || g.tiles < 256) g = retile(g, GEMM_BM, GEMM_BN_SMALL);
 }
 
 void launch_list(dmrg_ctx* c, const GemmList& g, char* db, const double* A, const double* B,
                  double* C, const GemmBatch& b = GemmBatch{}) {
-  launch_gemm_f64(c->stream, g.bm, g.tA, g.tB, A, B, C,
+  launch_gemm_f64(c->stream, g.bn, g.tA, g.tB, A, B, C,
                   reinterpret_cast<const GemmTask*>(db + g.t_off), int(g.tasks.size()),
-                  reinterpret_cast<const GemmSeg*>(db + g.s_off), g.tiles, c->nsm * 4, b);
+                  reinterpret_cast<const GemmSeg*>(db + g.s_off), g.tiles, c->nsm, b);
 }
 
 // One environment step of `nrows` rows through the same site: row r reads env_in + r * in_stride

@@ -106,12 +106,13 @@ void launch_trid_cluster(cudaStream_t s, double* base, const TridTask* tasks, in
 void launch_trid_mid_vectors(cudaStream_t s, double* base, const TridTask* tasks, int ntasks,
                              int max_n, int max_k, double* xws);
 
-constexpr int GEMM_BM = 64, GEMM_BN = 64, GEMM_BK = 16;
-constexpr int GEMM_SMALL_TILE = 32;   // the second tile shape of the FP64 GEMM (32 x 32)
+// Tiles of the FP64 GEMM: 32 x 32, or 32 x 16 for lists too short to give every SM three of them.
+constexpr int GEMM_BM = 32, GEMM_BN = 32, GEMM_BN_SMALL = 16;
 
-// Persistent grouped FP64 GEMM (DMMA m8n8k4 tensor-core path), square tiles of `tile` = 64 or
-// 32 (the task list's tile counts must match). Every output element accumulates its K products
-// in the same order for both tile shapes, so the results are bit-identical.
+// Persistent grouped FP64 GEMM (DMMA m8n8k4 tensor-core path), tiles of GEMM_BM x bn, bn =
+// GEMM_BN or GEMM_BN_SMALL (the task list's tile counts must match), on nsm SMs. Every output
+// element accumulates its K products in the same order for both tile shapes, so the results are
+// bit-identical.
 // The list repeated for n sets of operands at fixed strides (elements); the last set's A operand
 // may lie elsewhere (a_last).
 struct GemmBatch {
@@ -119,9 +120,9 @@ struct GemmBatch {
   int64_t a = 0, b = 0, c = 0;
   const double* a_last = nullptr;
 };
-void launch_gemm_f64(cudaStream_t s, int tile, bool transA, bool transB, const double* A,
+void launch_gemm_f64(cudaStream_t s, int bn, bool transA, bool transB, const double* A,
                      const double* B, double* C, const GemmTask* tasks, int ntasks,
-                     const GemmSeg* segs, int total_tiles, int grid_cap,
+                     const GemmSeg* segs, int total_tiles, int nsm,
                      const GemmBatch& batch = GemmBatch{});
 
 // Split-precision grouped GEMM on tcgen05 (FP32 accumulation in TMEM, FP64 in/out), direct form

@@ -32,7 +32,7 @@ class Context:
         self.device = device
 
     def tuner(self):
-        """FP64 GEMM tile autotuner: (signatures seen, decided, won by 32 x 32 tiles)."""
+        """FP64 GEMM tile autotuner: (signatures seen, decided, won by 32 x 16 tiles)."""
         a, b, c = C.c_int(), C.c_int(), C.c_int()
         check(lib().dmrg_ctx_tuner(self.h, C.byref(a), C.byref(b), C.byref(c)), self.h)
         return a.value, b.value, c.value
