@@ -118,6 +118,8 @@ SIGNATURES = {
     "dmrg_expect": (C.c_int, [_P, _P, _DP]),
     "dmrg_env_step": (C.c_int, [_P, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, _DP,
                                 _DP, _DP, _DP, _DP]),
+    "dmrg_env_step_order": (C.c_int, [_P, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int,
+                                      _DP, _DP, _DP, _DP, _DP, C.c_int]),
     "dmrg_correlationmatrix": (C.c_int, [_P, C.c_int, _DP, _DP, _DP, _DP]),
     "dmrg_correlation": (C.c_int, [_P, C.c_int, C.c_int, _IP, _DP, _IP, _IP, _DP, _DP]),
     "dmrg_mps_download_all_blocks": (C.c_int, [_P, _DP, C.POINTER(C.c_int64)]),

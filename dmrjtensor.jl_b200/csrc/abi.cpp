@@ -186,6 +186,9 @@ int dmrg_ctx_destroy(dmrg_ctx* c) {
   cudaFree(c->d_status);
   cudaFreeHost(c->h_scal);
   if (c->h_lam) cudaFreeHost(c->h_lam);
+  if (c->h_stage) cudaFreeHost(c->h_stage);
+  for (cudaEvent_t e : c->stage_ev)
+    if (e) cudaEventDestroy(e);
   cudaFree(c->d_flags);
   cudaFreeHost(c->h_flags);
   cudaFree(c->d_floors);
@@ -782,7 +785,20 @@ int dmrg_env_step(dmrg_ctx* c, int left, int ml, int d, int mr, int wl, int wr,
   return guarded(c, [&] {
     if (!env_in || !psi || !W || !env_out) fail(DMRG_ERR_ARG, "env step: null array");
     set_device(c);
-    env_step_dense(c, left != 0, ml, d, mr, wl, wr, env_in, dual ? dual : psi, psi, W, env_out);
+    env_step_dense(c, left != 0, ml, d, mr, wl, wr, env_in, dual ? dual : psi, psi, W, env_out, 0);
+  });
+}
+
+int dmrg_env_step_order(dmrg_ctx* c, int left, int ml, int d, int mr, int wl, int wr,
+                        const double* env_in, const double* dual, const double* psi,
+                        const double* W, double* env_out, int row_major) {
+  if (!c) return DMRG_ERR_ARG;
+  return guarded(c, [&] {
+    if (!env_in || !psi || !W || !env_out) fail(DMRG_ERR_ARG, "env step: null array");
+    if (row_major & ~7) fail(DMRG_ERR_ARG, "env step: unknown order bits");
+    set_device(c);
+    env_step_dense(c, left != 0, ml, d, mr, wl, wr, env_in, dual ? dual : psi, psi, W, env_out,
+                   row_major);
   });
 }
 
@@ -830,24 +846,23 @@ int dmrg_env_get(dmrg_state* st, int site, int left, double* out, int* dims) {
     if (dims) { dims[0] = m; dims[1] = w; dims[2] = m; }
     if (!out) return;
     set_device(c);
-    std::vector<double> h(std::max<int64_t>(E.size, 1));
-    const DBuf& buf = isL ? st->Lenv[site] : st->Renv[site];
-    cuda_check(cudaMemcpyAsync(h.data(), buf.p, sizeof(double) * E.size, cudaMemcpyDeviceToHost,
-                               c->stream), "env download");
-    cuda_check(cudaStreamSynchronize(c->stream), "env download sync");
-    std::fill(out, out + size_t(m) * w * m, 0.0);
+    HostStage h(c, E.size);
+    if (E.size > 0) h.fetch(isL ? st->Lenv[site].p : st->Renv[site].p);
+    if (E.size < int64_t(m) * w * m) std::fill(out, out + size_t(m) * w * m, 0.0);
     const auto o = B.offsets();
     for (int k = 0; k < E.nsec; ++k)       // k = ket sector (L) / bra sector (R)
-      for (int wi = 0; wi < w; ++wi) {
-        const int ko = E.other[k * w + wi];
-        if (ko < 0) continue;
-        for (int col = 0; col < B.dim[k]; ++col)
-          for (int r = 0; r < B.dim[ko]; ++r) {
-            const double v = h[E.goff[k] + E.rowoff[k * w + wi] + r + int64_t(col) * E.rows[k]];
-            // L[bra, w, ket]: rows are bra (ko), cols ket (k); R[ket, w, bra]: rows ket (ko), cols bra (k)
-            out[(o[ko] + r) + size_t(m) * (wi + size_t(w) * (o[k] + col))] = v;
-          }
+      for (int col = 0; col < B.dim[k]; ++col) {
+        const int64_t src = E.goff[k] + int64_t(col) * E.rows[k];
+        h.need(src + E.rows[k]);
+        for (int wi = 0; wi < w; ++wi) {
+          const int ko = E.other[k * w + wi];
+          if (ko < 0) continue;
+          // L[bra, w, ket]: rows are bra (ko), cols ket (k); R[ket, w, bra]: rows ket (ko), cols bra (k)
+          std::memcpy(out + o[ko] + size_t(m) * (wi + size_t(w) * (o[k] + col)),
+                      h.data() + src + E.rowoff[k * w + wi], size_t(B.dim[ko]) * sizeof(double));
+        }
       }
+    h.finish();
   });
 }
 
@@ -880,38 +895,40 @@ static int heff_apply_reps(dmrg_state* st, const dmrg_mpo* mpo, int iL, const do
     const Bond& Br = st->bond[iL + 2];
     const int ml = int(Bl.total()), mr = int(Br.total()), d1 = tl.d1, d2 = tl.d2;
     const auto ol = Bl.offsets(), orr = Br.offsets();
-    std::vector<double> h(std::max<int64_t>(tl.size, 1), 0.0);
-    auto at = [&](int a, int s1, int s2, int b) {
-      return size_t(a) + size_t(ml) * (s1 + size_t(d1) * (s2 + size_t(d2) * b));
+    const int64_t n = std::max<int64_t>(tl.size, 1);
+    ensure(c, c->K, n);
+    ensure(c, c->H, n);
+    HostStage h(c, n);
+    // the blocks' columns, in the order of the block layout: f(dense offset, layout offset, rows)
+    auto columns = [&](auto&& f) {
+      for (int ka = 0; ka < tl.nl; ++ka)
+        for (int s1 = 0; s1 < d1; ++s1)
+          for (int s2 = 0; s2 < d2; ++s2) {
+            const int id = tl.idx(ka, s1, s2), kd = tl.kd[id];
+            if (kd < 0) continue;
+            for (int cb = 0; cb < Br.dim[kd]; ++cb)
+              f(size_t(ol[ka]) + size_t(ml) * (s1 + size_t(d1) * (s2 + size_t(d2) * (orr[kd] + cb))),
+                tl.off[id] + int64_t(cb) * Bl.dim[ka], Bl.dim[ka]);
+          }
     };
-    for (int ka = 0; ka < tl.nl; ++ka)
-      for (int s1 = 0; s1 < d1; ++s1)
-        for (int s2 = 0; s2 < d2; ++s2) {
-          const int id = tl.idx(ka, s1, s2), kd = tl.kd[id];
-          if (kd < 0) continue;
-          for (int cb = 0; cb < Br.dim[kd]; ++cb)
-            for (int ca = 0; ca < Bl.dim[ka]; ++ca)
-              h[tl.off[id] + ca + int64_t(cb) * Bl.dim[ka]] = psi_in[at(ol[ka] + ca, s1, s2, orr[kd] + cb)];
-        }
-    ensure(c, c->K, int64_t(h.size()));
-    ensure(c, c->H, int64_t(h.size()));
-    cuda_check(cudaMemcpyAsync(c->K.p, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice,
-                               c->stream), "psi upload");
+    columns([&](size_t dense, int64_t at, int rows) {
+      std::memcpy(h.data() + at, psi_in + dense, size_t(rows) * sizeof(double));
+      h.sent(c->K.p, at + rows);
+    });
+    h.sent(c->K.p, n);
     for (int r = 0; r < reps; ++r) apply_heff(st, iL, hp, c->K.p, c->H.p, precision);
-    cuda_check(cudaMemcpyAsync(h.data(), c->H.p, h.size() * sizeof(double), cudaMemcpyDeviceToHost,
-                               c->stream), "psi download");
-    cuda_check(cudaStreamSynchronize(c->stream), "heff sync");
-    check_mma_status(c);
-    std::fill(psi_out, psi_out + size_t(ml) * d1 * d2 * mr, 0.0);
-    for (int ka = 0; ka < tl.nl; ++ka)
-      for (int s1 = 0; s1 < d1; ++s1)
-        for (int s2 = 0; s2 < d2; ++s2) {
-          const int id = tl.idx(ka, s1, s2), kd = tl.kd[id];
-          if (kd < 0) continue;
-          for (int cb = 0; cb < Br.dim[kd]; ++cb)
-            for (int ca = 0; ca < Bl.dim[ka]; ++ca)
-              psi_out[at(ol[ka] + ca, s1, s2, orr[kd] + cb)] = h[tl.off[id] + ca + int64_t(cb) * Bl.dim[ka]];
-        }
+    if (split_form(precision))
+      to_host(c, c->h_scal + 20, c->dv_scal ? c->dv_scal + 20 : nullptr, c->d_status + STATUS_MMA,
+              sizeof(int), "MMA status");
+    h.fetch(c->H.p);
+    if (tl.size < int64_t(ml) * d1 * d2 * mr)
+      std::fill(psi_out, psi_out + size_t(ml) * d1 * d2 * mr, 0.0);
+    columns([&](size_t dense, int64_t at, int rows) {
+      h.need(at + rows);
+      std::memcpy(psi_out + dense, h.data() + at, size_t(rows) * sizeof(double));
+    });
+    h.finish();
+    if (split_form(precision)) check_mma_flag(c);
   });
 }
 

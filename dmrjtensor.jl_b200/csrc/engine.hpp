@@ -202,6 +202,9 @@ struct dmrg_ctx {
   double* h_scal = nullptr;      // pinned mirror of d_scal
   double* h_lam = nullptr;       // pinned eigenvalue download buffer (grow-only)
   size_t h_lam_cap = 0;
+  double* h_stage = nullptr;     // pinned staging of dense operands and results (HostStage)
+  int64_t h_stage_cap = 0;       // doubles
+  cudaEvent_t stage_ev[8] = {};
   double* dv_scal = nullptr;     // device addresses of h_scal / h_lam (null: not mapped, the
   double* dv_lam = nullptr;      // downloads then use a copy engine)
   cudaEvent_t ev[8] = {};
@@ -304,6 +307,36 @@ struct Upload {
   void put(CopyList& c) { c.t_off = put(c.tasks); }
   char* send(dmrg_ctx* c, int slot);   // returns the device base of the copied bytes
 };
+
+// A dense operand or result on its way through pinned memory: a copy engine moves 55 GB/s to or
+// from pinned pages and 7 to 22 GB/s to or from others, and it runs while the host packs or unpacks
+// the rest. One at a time per context; every use ends with the stream synchronised. Above
+// HOST_STAGE_MAX doubles ordinary memory takes its place.
+constexpr int64_t HOST_STAGE_MAX = 8 << 20;   // 64 MB
+class HostStage {
+ public:
+  HostStage(dmrg_ctx* c, int64_t n);
+  ~HostStage() { if (open) cudaStreamSynchronize(c->stream); }   // a call that failed half-way
+  HostStage(const HostStage&) = delete;
+  HostStage& operator=(const HostStage&) = delete;
+  double* data() const { return h; }
+  // Host to device: doubles [0, upto) are written; the last call has upto = n.
+  void sent(double* dev, int64_t upto);
+  // Device to host: starts all of it; then need(upto) waits until [0, upto) has arrived.
+  void fetch(const double* dev);
+  void need(int64_t upto);
+  // Waits for the stream: the end of a use.
+  void finish();
+
+ private:
+  dmrg_ctx* c;
+  int64_t n, chunk, at = 0;
+  int ready = 0;
+  bool open = false;
+  std::vector<double> own;
+  double* h = nullptr;
+};
+
 
 // Launch wrappers. Every launch first checks on the host that each task's extent lies inside
 // the sizes (in doubles) of the buffers it addresses; a violation is a DMRG_ERR_ARG, never a
@@ -408,6 +441,8 @@ void prepare_split(HeffPlan& hp);
 // Fails (DMRG_ERR_TIMEOUT) if a split-precision GEMM reported an MMA wait that gave up since the
 // last check, and clears the flag. Synchronous read; call after a stream synchronisation.
 void check_mma_status(dmrg_ctx* c);
+// The same for a flag that a copy in the stream brought to h_scal[20] (the stream synchronised).
+void check_mma_flag(dmrg_ctx* c);
 void apply_heff(dmrg_state* st, int iL, const HeffPlan& hp, const double* x, double* y,
                 int precision, GemmProfile* prof = nullptr);
 
@@ -451,7 +486,7 @@ void run_step(dmrg_ctx* c, const StepPlan& sp, char* db, const double* env_in, i
 // Lupdate(Lenv, dualpsi, psi, mpo) / Rupdate(...) as a pure function of dense host tensors.
 void env_step_dense(dmrg_ctx* c, bool left, int ml, int d, int mr, int wl, int wr,
                     const double* env_in, const double* dual, const double* psi, const double* W,
-                    double* env_out);
+                    double* env_out, int row_major);
 
 // Creates the context's second stream and its fork and join events.
 void ensure_env_stream(dmrg_ctx* c);

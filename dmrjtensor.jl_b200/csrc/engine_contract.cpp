@@ -7,6 +7,7 @@
 // Lupdate / Rupdate (lib/MPO_MPS/Lupdate.jl:17-26, Rupdate.jl:17-26) in the same three shapes.
 #include <algorithm>
 #include <atomic>
+#include <cstring>
 #include <map>
 
 #include "engine.hpp"
@@ -141,6 +142,15 @@ void check_mma_status(dmrg_ctx* c) {
              "MMA status");
   if (flag != 0) {
     cudaMemset(c->d_status + STATUS_MMA, 0, sizeof(int));
+    fail(DMRG_ERR_TIMEOUT, "split-precision GEMM: a tensor-core MMA completion wait gave up");
+  }
+}
+
+void check_mma_flag(dmrg_ctx* c) {
+  int flag = 0;
+  std::memcpy(&flag, c->h_scal + 20, sizeof(int));
+  if (flag != 0) {
+    cudaMemsetAsync(c->d_status + STATUS_MMA, 0, sizeof(int), c->stream);
     fail(DMRG_ERR_TIMEOUT, "split-precision GEMM: a tensor-core MMA completion wait gave up");
   }
 }
@@ -534,7 +544,7 @@ void run_step(dmrg_ctx* c, const StepPlan& sp, char* db, const double* env_in, i
 
 void env_step_dense(dmrg_ctx* c, bool left, int ml, int d, int mr, int wl, int wr,
                     const double* env_in, const double* dual, const double* psi, const double* W,
-                    double* env_out) {
+                    double* env_out, int row_major) {
   if (ml <= 0 || d <= 0 || mr <= 0 || wl <= 0 || wr <= 0)
     fail(DMRG_ERR_SHAPE, "env step: every dimension must be positive");
   // dense tensors: every bond and physical state carries charge 0 (one sector per bond)
@@ -555,16 +565,6 @@ void env_step_dense(dmrg_ctx* c, bool left, int ml, int d, int mr, int wl, int w
           if (v != 0.0) ms.nz.push_back({w, s, t, w2, v});
         }
   const SiteLayout lay = make_site_layout(Bl, ms.p, Br);
-  // site [ml, d, mr] column-major -> blocks (s) of [ml x mr], s-major
-  std::vector<double> hA(size_t(ml) * d * mr), hB(hA.size());
-  for (int s = 0; s < d; ++s)
-    for (int b = 0; b < mr; ++b)
-      for (int a = 0; a < ml; ++a) {
-        const size_t src = a + size_t(ml) * (s + size_t(d) * b);
-        const size_t dst = size_t(lay.off[s]) + a + size_t(ml) * b;
-        hA[dst] = psi[src];
-        hB[dst] = dual[src];
-      }
   StepPlan sp;
   EnvLayout in_lay;
   if (left) {
@@ -574,28 +574,57 @@ void env_step_dense(dmrg_ctx* c, bool left, int ml, int d, int mr, int wl, int w
     in_lay = make_right_env_layout(Br, ms.rr);
     plan_right_step(Bl, Br, ms, lay, in_lay, sp);
   }
-  // a dense environment [m, w, m] column-major is exactly the one-sector block layout
+  // The operands go up as they are, by way of the step's scratch, and are reordered on the device:
+  // a site [ml, d, mr] to blocks (s) of [ml x mr], s-major; a dense column-major environment
+  // [m, w, m] is exactly the one-sector block layout. Reordering them on the host (there, or in the
+  // caller's program to column-major order) took longer than the step itself.
+  const int me = left ? ml : mr, we = left ? wl : wr;
+  const int64_t nA = int64_t(ml) * d * mr;
+  const bool one = dual == psi && ((row_major >> 1) & 1) == ((row_major >> 2) & 1);
+  CopyList copy[3];   // psi, dual, environment
+  for (int q = 0; q < 2; ++q)
+    for (int s = 0; s < d; ++s)
+      if (row_major & (2 << q))
+        copy[q].add(int64_t(s) * mr, d * mr, lay.off[s], ml, ml, mr, 1, 1.0);
+      else
+        copy[q].add(int64_t(s) * ml, d * ml, lay.off[s], ml, ml, mr, 0, 1.0);
+  const bool env_rows = (row_major & 1) != 0;
+  if (env_rows)
+    for (int w = 0; w < we; ++w)
+      copy[2].add(int64_t(w) * me, we * me, int64_t(w) * me, we * me, me, me, 1, 1.0);
   Upload u;
   put_step(u, sp);
+  for (CopyList& l : copy) u.put(l);
   char* db = u.send(c, 2);
   DBuf dA, dB, din, dout;
   try {
-    dalloc(c, dA, int64_t(hA.size()));
-    dalloc(c, dB, int64_t(hB.size()));
+    dalloc(c, dA, nA);
+    if (!one) dalloc(c, dB, nA);
     dalloc(c, din, std::max<int64_t>(in_lay.size, 1));
     dalloc(c, dout, std::max<int64_t>(sp.out.size, 1));
-    ensure(c, c->T1, std::max<int64_t>(sp.t1, 1));
+    ensure(c, c->T1, std::max<int64_t>({sp.t1, nA, env_rows ? in_lay.size : 0}));
     ensure(c, c->T2, std::max<int64_t>(sp.t2, 1));
-    cuda_check(cudaMemcpyAsync(dA.p, hA.data(), hA.size() * 8, cudaMemcpyHostToDevice, c->stream),
-               "env step psi");
-    cuda_check(cudaMemcpyAsync(dB.p, hB.data(), hB.size() * 8, cudaMemcpyHostToDevice, c->stream),
-               "env step dual");
-    cuda_check(cudaMemcpyAsync(din.p, env_in, size_t(in_lay.size) * 8, cudaMemcpyHostToDevice,
-                               c->stream), "env step input");
-    run_step(c, sp, db, din.p, din.n, dA, dout.p, dout.n, &dB);
-    cuda_check(cudaMemcpyAsync(env_out, dout.p, size_t(sp.out.size) * 8, cudaMemcpyDeviceToHost,
-                               c->stream), "env step output");
-    cuda_check(cudaStreamSynchronize(c->stream), "env step sync");
+    auto put = [&](const double* host, double* dev, int64_t n, const char* what) {
+      cuda_check(cudaMemcpyAsync(dev, host, size_t(n) * 8, cudaMemcpyHostToDevice, c->stream), what);
+    };
+    put(psi, c->T1.p, nA, "env step psi");
+    run_copy(c, copy[0], db, c->T1.p, nA, dA.p, nA);
+    if (!one) {
+      put(dual, c->T1.p, nA, "env step dual");
+      run_copy(c, copy[1], db, c->T1.p, nA, dB.p, nA);
+    }
+    put(env_in, env_rows ? c->T1.p : din.p, in_lay.size, "env step input");
+    if (env_rows) run_copy(c, copy[2], db, c->T1.p, in_lay.size, din.p, din.n);
+    run_step(c, sp, db, din.p, din.n, dA, dout.p, dout.n, one ? &dA : &dB);
+    HostStage out(c, sp.out.size);
+    out.fetch(dout.p);
+    const int64_t piece = int64_t(1) << 17;
+    for (int64_t o = 0; o < sp.out.size; o += piece) {
+      const int64_t n = std::min(piece, sp.out.size - o);
+      out.need(o + n);
+      std::memcpy(env_out + o, out.data() + o, size_t(n) * sizeof(double));
+    }
+    out.finish();
   } catch (...) {
     dfree(c, dA); dfree(c, dB); dfree(c, din); dfree(c, dout);
     throw;

@@ -447,6 +447,63 @@ char* Upload::send(dmrg_ctx* c, int slot) {
   return s.d;
 }
 
+HostStage::HostStage(dmrg_ctx* ctx, int64_t count) : c(ctx), n(std::max<int64_t>(count, 1)) {
+  chunk = std::max<int64_t>(int64_t(1) << 17, (n + 7) / 8);
+  if (n > HOST_STAGE_MAX) {
+    own.resize(size_t(n));
+    h = own.data();
+    return;
+  }
+  if (n > c->h_stage_cap) {
+    const int64_t cap = std::min(HOST_STAGE_MAX, std::max(n + n / 4, int64_t(1) << 17));
+    if (c->h_stage) cudaFreeHost(c->h_stage);
+    c->h_stage = nullptr;
+    c->h_stage_cap = 0;
+    cuda_check(cudaMallocHost(reinterpret_cast<void**>(&c->h_stage), size_t(cap) * sizeof(double)),
+               "cudaMallocHost(staging)");
+    c->h_stage_cap = cap;
+  }
+  for (cudaEvent_t& e : c->stage_ev)
+    if (!e) cuda_check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "staging event");
+  h = c->h_stage;
+}
+
+void HostStage::sent(double* dev, int64_t upto) {
+  if (upto < n && upto - at < chunk) return;
+  open = true;
+  if (upto > at)
+    cuda_check(cudaMemcpyAsync(dev + at, h + at, size_t(upto - at) * sizeof(double),
+                               cudaMemcpyHostToDevice, c->stream), "operand upload");
+  at = upto;
+}
+
+void HostStage::fetch(const double* dev) {
+  ready = 0;
+  open = true;
+  if (!own.empty()) {
+    cuda_check(cudaMemcpyAsync(h, dev, size_t(n) * sizeof(double), cudaMemcpyDeviceToHost,
+                               c->stream), "result download");
+    cuda_check(cudaStreamSynchronize(c->stream), "result download");
+    ready = 8;
+    return;
+  }
+  for (int64_t o = 0, i = 0; o < n; o += chunk, ++i) {
+    cuda_check(cudaMemcpyAsync(h + o, dev + o, size_t(std::min(chunk, n - o)) * sizeof(double),
+                               cudaMemcpyDeviceToHost, c->stream), "result download");
+    cuda_check(cudaEventRecord(c->stage_ev[i], c->stream), "staging event");
+  }
+}
+
+void HostStage::need(int64_t upto) {
+  for (; ready < 8 && ready * chunk < std::min(upto, n); ++ready)
+    cuda_check(cudaEventSynchronize(c->stage_ev[ready]), "result download");
+}
+
+void HostStage::finish() {
+  cuda_check(cudaStreamSynchronize(c->stream), "operand transfer");
+  open = false;
+}
+
 namespace {
 inline bool in_range(int64_t off, int64_t last, int64_t n) { return off >= 0 && off + last < n; }
 [[noreturn]] void bad_plan(const char* what) {

@@ -230,14 +230,7 @@ void join_env(dmrg_ctx* c) {
 double krylov_energy(dmrg_ctx* c, const KrylovRun& kr) {
   double e = c->h_scal[lz::EN];
   if (kr.fp64_energy && c->h_scal[lz::KK] > 0) e = c->h_scal[lz::KH] / c->h_scal[lz::KK];
-  if (kr.split) {
-    int flag = 0;
-    std::memcpy(&flag, c->h_scal + 20, sizeof(int));
-    if (flag != 0) {
-      cudaMemsetAsync(c->d_status + STATUS_MMA, 0, sizeof(int), c->stream);
-      fail(DMRG_ERR_TIMEOUT, "split-precision GEMM: a tensor-core MMA completion wait gave up");
-    }
-  }
+  if (kr.split) check_mma_flag(c);
   return e;
 }
 

@@ -409,7 +409,7 @@ class DeviceState:
     def env(self, i, left):
         dims = (C.c_int * 3)()
         check(lib().dmrg_env_get(self.h, i, 1 if left else 0, None, dims), self.ctx.h)
-        out = np.zeros(tuple(dims), order="F")
+        out = np.empty(tuple(dims), order="F")   # written in full by the call
         check(lib().dmrg_env_get(self.h, i, 1 if left else 0,
                                  out.ctypes.data_as(C.POINTER(C.c_double)), dims), self.ctx.h)
         return out
@@ -420,7 +420,7 @@ class DeviceState:
         x = np.asfortranarray(psi2, dtype=float)
         if x.shape != tuple(dims):
             raise ValueError(f"two-site vector has shape {x.shape}, expected {tuple(dims)}")
-        y = np.zeros(tuple(dims), order="F")
+        y = np.empty(tuple(dims), order="F")     # written in full by the call
         check(lib().dmrg_heff_apply(self.h, self.dmpo.h, iL, x.ctypes.data_as(C.POINTER(C.c_double)),
                                     y.ctypes.data_as(C.POINTER(C.c_double)),
                                     _lib.PREC[precision]), self.ctx.h)
@@ -789,13 +789,22 @@ def makeEnv(psi: MPS, mpo: MPO, ctx=None):
     return Env(dev, True), Env(dev, False)
 
 
+def _as_stored(x):
+    """(array of doubles, 1 if its memory is row-major): row- and column-major arrays as they are,
+    others as a column-major copy."""
+    x = np.asarray(x, dtype=float)
+    if x.flags.f_contiguous or not x.flags.c_contiguous:
+        return np.asfortranarray(x), 0
+    return x, 1
+
+
 def _env_step(left, env, dual, psi, W, ctx=None):
     """One dense environment step on the device (``dmrg_env_step``)."""
     ctx = ctx or default_context()
-    A = np.asfortranarray(np.asarray(psi, dtype=float))
-    B = np.asfortranarray(np.asarray(dual, dtype=float)) if dual is not None else A
+    A, a_rows = _as_stored(psi)
+    B, b_rows = (A, a_rows) if dual is None or dual is psi else _as_stored(dual)
     Wf = np.asfortranarray(np.asarray(W, dtype=float))
-    E = np.asfortranarray(np.asarray(env, dtype=float))
+    E, e_rows = _as_stored(env)
     if A.ndim != 3 or B.shape != A.shape or Wf.ndim != 4 or E.ndim != 3:
         raise ValueError("env step: environment [m,w,m], sites [ml,d,mr], MPO [wl,d,d,wr]")
     ml, d, mr = A.shape
@@ -805,11 +814,13 @@ def _env_step(left, env, dual, psi, W, ctx=None):
     want = (ml, wl, ml) if left else (mr, wr, mr)
     if E.shape != want:
         raise ValueError(f"environment has shape {E.shape}, expected {want}")
-    out = np.zeros((mr, wr, mr) if left else (ml, wl, ml), order="F")
+    out = np.empty((mr, wr, mr) if left else (ml, wl, ml), order="F")
     dp = C.POINTER(C.c_double)
-    check(lib().dmrg_env_step(ctx.h, 1 if left else 0, ml, d, mr, wl, wr, E.ctypes.data_as(dp),
-                              B.ctypes.data_as(dp), A.ctypes.data_as(dp), Wf.ctypes.data_as(dp),
-                              out.ctypes.data_as(dp)), ctx.h)
+    check(lib().dmrg_env_step_order(ctx.h, 1 if left else 0, ml, d, mr, wl, wr,
+                                    E.ctypes.data_as(dp), B.ctypes.data_as(dp),
+                                    A.ctypes.data_as(dp), Wf.ctypes.data_as(dp),
+                                    out.ctypes.data_as(dp), e_rows + 2 * a_rows + 4 * b_rows),
+          ctx.h)
     return out
 
 

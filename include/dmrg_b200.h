@@ -215,6 +215,11 @@ DMRG_API int dmrg_rupdate(dmrg_state* st, const dmrg_mpo* mpo, int site);
 DMRG_API int dmrg_env_step(dmrg_ctx* ctx, int left, int ml, int d, int mr, int wl, int wr,
                            const double* env_in, const double* dual, const double* psi,
                            const double* W, double* env_out);
+/* The same with operands that are row-major in memory: row_major is the sum of 1 (env_in),
+ * 2 (psi) and 4 (dual); they are reordered on the device. W and env_out stay column-major. */
+DMRG_API int dmrg_env_step_order(dmrg_ctx* ctx, int left, int ml, int d, int mr, int wl, int wr,
+                                 const double* env_in, const double* dual, const double* psi,
+                                 const double* W, double* env_out, int row_major);
 /* Lenv[i] (left=1) or Renv[i] (left=0) as a dense-equivalent column-major [m, w, m] array
  * (L[bra,w,ket] / R[ket,w,bra]). dims receives the 3 sizes; out may be NULL to query them. */
 DMRG_API int dmrg_env_get(dmrg_state* st, int site, int left, double* out, int* dims);
