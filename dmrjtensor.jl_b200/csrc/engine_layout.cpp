@@ -367,7 +367,7 @@ void MixList::add(int64_t out_off, int ld, int rows, int cols) {
   t.term0 = int(terms.size());
   t.nterm = 0;
   t.tile0 = tiles;
-  t.ntiles = (rows > 0 && cols > 0) ? (cols + 31) / 32 : 0;
+  t.ntiles = (rows > 0 && cols > 0) ? (cols + mix_cols(rows) - 1) / mix_cols(rows) : 0;
   tiles += t.ntiles;
   tasks.push_back(t);
 }
@@ -395,7 +395,7 @@ void CopyList::add(int64_t src_off, int lds, int64_t dst_off, int ldd, int rows,
   t.cols = cols;
   t.trans = trans;
   t.tile0 = tiles;
-  t.ntiles = (cols + 31) / 32;
+  t.ntiles = (cols + mix_cols(rows) - 1) / mix_cols(rows);
   t.scale = scale;
   tiles += t.ntiles;
   tasks.push_back(t);

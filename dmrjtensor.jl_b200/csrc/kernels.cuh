@@ -28,6 +28,14 @@ struct GemmTask {
   double alpha, beta;
 };
 
+// Columns of a mixing or copy tile. A tile costs its block the lookup of the task and of each
+// term before the first element moves, so the launches are bound by latency until every SM holds
+// several tiles, and narrow tiles spread the work: ten blocks of 384 x 384 in tiles of 32 columns
+// 7.4 us, of 16 5.9; the 7 to 49 row blocks of a U(1) chain 6.6 us, of 16 4.8, of 8 3.7. With many
+// tall blocks the lookups add up: the mixing of a cylinder's step 11.1, 10.6 and 12.7 us.
+constexpr int MIX_TALL = 64;      // blocks of at least this many rows: a warp per column
+__host__ __device__ constexpr int mix_cols(int rows) { return rows >= MIX_TALL ? 16 : 8; }
+
 // out block (rows x cols, ld) = sum_t coef_t * in_t (same shape, own ld); sparse MPO mixing.
 struct MixTerm {
   int64_t in_off;
@@ -38,7 +46,7 @@ struct MixTask {
   int64_t out_off;
   int ld, rows, cols;
   int term0, nterm;
-  int tile0;        // first tile (tiles of 32 columns x all rows)
+  int tile0;        // first tile (tiles of mix_cols(rows) columns x all rows)
   int ntiles;
   int pad;
 };

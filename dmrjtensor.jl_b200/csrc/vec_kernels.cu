@@ -10,8 +10,6 @@
 namespace dmrg {
 namespace {
 
-constexpr int MIX_COLS = 32;      // columns per mixing / copy tile
-constexpr int MIX_TALL = 64;      // mixing blocks of at least this many rows: a warp per column
 constexpr int MIX_ROWS_PER_LANE = 4;
 constexpr int RED_BLOCKS = 296;   // 2 x 148 SMs
 constexpr int RED_THREADS = 256;
@@ -65,8 +63,8 @@ __global__ void k_mix(const double* __restrict__ in0, double* __restrict__ out0,
     const double* in = in0 + set * in_stride;
     double* out = out0 + set * out_stride;
     const MixTask tk = tasks[find_task(tasks, ntasks, tile)];
-    const int c0 = (tile - tk.tile0) * MIX_COLS;
-    const int ncol = min(MIX_COLS, tk.cols - c0);
+    const int width = mix_cols(tk.rows), c0 = (tile - tk.tile0) * width;
+    const int ncol = min(width, tk.cols - c0);
     if (tk.rows >= MIX_TALL) {
       // tall blocks: a warp per column, MIX_ROWS_PER_LANE rows per lane (rows lane + 32 j of a
       // 128-row slab), so that every thread has that many independent loads of a term in flight
@@ -117,8 +115,8 @@ __global__ void k_copy(const double* __restrict__ src, double* __restrict__ dst,
   grid_entry();
   for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
     const CopyTask tk = tasks[find_task(tasks, ntasks, tile)];
-    const int c0 = (tile - tk.tile0) * MIX_COLS;
-    const int ncol = min(MIX_COLS, tk.cols - c0);
+    const int width = mix_cols(tk.rows), c0 = (tile - tk.tile0) * width;
+    const int ncol = min(width, tk.cols - c0);
     const int nel = ncol * tk.rows;
     for (int e = threadIdx.x; e < nel; e += blockDim.x) {
       const int r = e % tk.rows, c = c0 + e / tk.rows;
