@@ -6,6 +6,7 @@
 
 #include "kernels.cuh"
 #include "launch.cuh"
+#include "syevt_common.cuh"
 
 namespace dmrg {
 namespace {
@@ -360,6 +361,56 @@ __global__ void k_next_vector(const double* __restrict__ H, double* __restrict__
   }
 }
 
+// Lowest eigenpair of T = tridiag(alpha, beta) of the m active vectors, one warp, when m > 2 (else
+// false): the eigenvalue by multisection, 32 Sturm counts a step, each shrinking the interval 33
+// times (11 steps); its vector by inverse iteration in lane 0, with a first component >= 0; the
+// energy is the vector's Rayleigh quotient. All three are chains of a few dozen dependent
+// operations, where the Jacobi rotations of the whole matrix are 49 rounds of them (m = 8: 30 us
+// as one of a sweep's launches, 6.6 this way).
+__device__ bool lowest_pair(double* s, int kdim) {
+  __shared__ double d[MAXK], e[MAXK], e2[MAXK], z[MAXK], u0[MAXK], u1[MAXK], l[MAXK];
+  __shared__ int piv[MAXK];
+  const int lane = threadIdx.x;
+  const bool on = lane + 1 < kdim && s[lz::BETA + lane] > 0.0;
+  const int m = 1 + __ffs(~__ballot_sync(FULL, on)) - 1;
+  if (m <= 2) return false;
+  const double al = lane < m ? s[lz::ALPHA + lane] : 0.0;
+  const double be = lane + 1 < m ? s[lz::BETA + lane] : 0.0;
+  const double r = be + __shfl_up_sync(FULL, be, 1) * (lane > 0);
+  double lo = lane < m ? al - r : 1e300, hi = lane < m ? al + r : -1e300;
+  if (lane < m) {
+    d[lane] = al;
+    e[lane] = be;
+    e2[lane] = be * be;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    lo = fmin(lo, __shfl_xor_sync(FULL, lo, o));
+    hi = fmax(hi, __shfl_xor_sync(FULL, hi, o));
+  }
+  __syncwarp();
+  const double tn = fmax(fmax(fabs(lo), fabs(hi)), 1e-300);
+  const double tol = 8.9e-16 * tn;
+  double a = lo - 2.2e-16 * tn, b = hi + 2.2e-16 * tn;   // no eigenvalue below a, all below b
+  for (int it = 0; it < 64 && b - a > tol; ++it) {
+    const double w = (b - a) * (1.0 / 33.0);
+    const unsigned below = __ballot_sync(FULL, sturm_below(d, e2, m, a + w * (lane + 1)) > 0);
+    const int g = below ? __ffs(below) - 1 : 32;         // the lowest lies in (x_(g-1), x_g]
+    const double x = a + w * g;
+    if (g < 32) b = a + w * (g + 1);
+    a = x;
+  }
+  if (lane == 0)
+    inverse_iteration(d, e, m, 0.5 * (a + b), z, 1, 0, tn, LUSlot{u0, u1, l, piv, 1});
+  __syncwarp();
+  const double sg = z[0] < 0.0 ? -1.0 : 1.0;
+  const double zi = lane < m ? sg * z[lane] : 0.0, zn = lane + 1 < m ? sg * z[lane + 1] : 0.0;
+  const double en = wsum(al * zi * zi + 2.0 * be * zi * zn);
+  if (lane == 0) s[lz::EN] = en;
+  if (lane < kdim) s[lz::COEF + lane] = zi;
+  return true;
+}
+
 // Ritz step of the Krylov solve, one warp: T = tridiag(alpha, beta) of the m active vectors
 // (m = 1 + number of leading non-zero beta_j, at most kdim), Jacobi rotations until the
 // off-diagonal is at the rounding level of the diagonal, lowest eigenvalue -> s[EN], its
@@ -367,13 +418,15 @@ __global__ void k_next_vector(const double* __restrict__ H, double* __restrict__
 // round-robin order of a tournament), one lane per angle and one lane per element of the row,
 // column and vector updates: m - 1 rounds a sweep instead of m (m - 1) / 2 rotations one after the
 // other, each of which is a chain of square roots and divisions (m = 8: 81 -> 35 us). A
-// 2-vector step is one rotation, written out.
+// 2-vector step is one rotation, written out. Only expo and 2-vector steps get there: the lowest
+// pair of three or more vectors alone is lowest_pair.
 // expo = 0: the lowest Ritz pair (s[EN], s[COEF + j]). expo = 1: s[COEF + j] = (exp(tau T) e_1)_j
 // (krylovTimeEvol, algs/time.jl:182-203: the Krylov vectors are orthonormal, so these are the
 // coefficients of exp(tau H) applied to the normalised start vector), from the eigenpairs of T;
 // when they sum to exactly zero, the first column of I + T instead. s[EN] = lowest eigenvalue.
 __global__ void k_ritz(double* s, int kdim, double tau, int expo) {
   grid_entry();
+  if (!expo && kdim > 2 && lowest_pair(s, kdim)) return;
   __shared__ double A[MAXK * MAXK], V[MAXK * MAXK];
   __shared__ double rc[MAXK / 2], rs[MAXK / 2];
   __shared__ int rp[MAXK / 2], rq[MAXK / 2];
