@@ -1112,7 +1112,10 @@ int dmrg_test_syevt(dmrg_ctx* c, int nmat, const int* n, const int* k, double* A
     DBuf buf;
     dalloc(c, buf, ta + 4 * tw + tu);
     cuda_check(cudaMemcpyAsync(buf.p, A, ta * 8, cudaMemcpyHostToDevice, c->stream), "A");
-    run_trid_eigvals(c, buf.p, buf.n, tasks, 8);
+    TridValues tv;
+    Upload u;
+    put_trid_values(u, tasks, tv);
+    run_trid_values(c, buf.p, buf.n, tv, u.send(c, 8));
     if (mk > 0) run_trid_vectors(c, buf.p, buf.n, tasks, 6);
     cuda_check(cudaMemcpyAsync(w, buf.p + ta, tw * 8, cudaMemcpyDeviceToHost, c->stream), "w");
     cuda_check(cudaMemcpyAsync(U, buf.p + ta + 4 * tw, tu * 8, cudaMemcpyDeviceToHost, c->stream), "U");

@@ -515,8 +515,14 @@ void measure_correlation(dmrg_state* st, int d, const double* Cc, const double* 
 // one launch each), then the kept eigenvectors (tasks with keep > 0; mid-size blocks use c->W
 // as workspace). Offsets are checked against nbase before any launch.
 void set_trid_paths(std::vector<TridTask>& t);
-void run_trid_eigvals(dmrg_ctx* c, double* base, int64_t nbase, const std::vector<TridTask>& t,
-                      int slot);
+struct TridValues {              // the eigenvalue launches' lists, sent with the caller's upload
+  std::vector<TridTask> small, mid;
+  int ns = 0;                    // largest small block
+  int64_t sum = 0;               // mid-size blocks' states
+  size_t o_small = 0, o_mid = 0;
+};
+void put_trid_values(Upload& u, const std::vector<TridTask>& t, TridValues& v);
+void run_trid_values(dmrg_ctx* c, double* base, int64_t nbase, const TridValues& v, char* db);
 void run_trid_vectors(dmrg_ctx* c, double* base, int64_t nbase, std::vector<TridTask> t,
                       int slot);
 int64_t eig_workspace(const std::vector<EigTask>& tasks);

@@ -262,7 +262,7 @@ void single_site_step(dmrg_state* st, const dmrg_params& P, const SiteMode& md, 
   u2.put(gather);
   u2.put(mexp);
   u2.put(gexp);
-  u2.put(rs.grho);
+  put_rho(u2, rs);
   char* db2 = u2.send(c, 1);
   cuda_check(cudaMemsetAsync(c->M.p, 0, size_t(std::max<int64_t>(rs.mtot, 1)) * sizeof(double), s),
              "3S group matrices");

@@ -1,5 +1,6 @@
 // engine_eig.cpp -- batched eigensolve of the density-matrix blocks of one truncation:
-// blocks with n <= 100 go to the one-CTA shared-memory Jacobi, larger ones to the block Jacobi.
+// the tridiagonal path (one CTA per block, or clusters) for all that it may solve, block Jacobi for
+// the rest (with the one-CTA shared-memory Jacobi up to 100 states).
 #include <algorithm>
 
 #include "engine.hpp"
@@ -26,29 +27,28 @@ void set_trid_paths(std::vector<TridTask>& t) {
   for (TridTask& x : t) x.mid = nmax > SYEVT_ROUTE ? 1 : 0;
 }
 
-void run_trid_eigvals(dmrg_ctx* c, double* base, int64_t nbase, const std::vector<TridTask>& t,
-                      int slot) {
-  check_trid(t, nbase, false);
-  std::vector<TridTask> small, mid;
-  int ns = 0;
-  int64_t sum = 0;
+void put_trid_values(Upload& u, const std::vector<TridTask>& t, TridValues& v) {
+  v = TridValues{};
   for (const TridTask& x : t) {
-    if (!x.mid) { small.push_back(x); ns = std::max(ns, x.n); }
-    else { mid.push_back(x); sum += x.n; }
+    if (!x.mid) { v.small.push_back(x); v.ns = std::max(v.ns, x.n); }
+    else { v.mid.push_back(x); v.sum += x.n; }
   }
   // the largest first: not all clusters of a long list are resident at once
-  std::stable_sort(mid.begin(), mid.end(),
+  std::stable_sort(v.mid.begin(), v.mid.end(),
                    [](const TridTask& a, const TridTask& b) { return a.n > b.n; });
-  if (small.empty() && mid.empty()) return;
-  Upload u;
-  const size_t o1 = u.put(small), o2 = u.put(mid);
-  char* db = u.send(c, slot);
-  if (!small.empty())
-    launch_trid_eigvals(c->stream, base, reinterpret_cast<const TridTask*>(db + o1),
-                        int(small.size()), ns);
-  if (!mid.empty())
-    launch_trid_cluster(c->stream, base, reinterpret_cast<const TridTask*>(db + o2),
-                        int(mid.size()), mid[0].n, sum);
+  v.o_small = u.put(v.small);
+  v.o_mid = u.put(v.mid);
+}
+
+void run_trid_values(dmrg_ctx* c, double* base, int64_t nbase, const TridValues& v, char* db) {
+  check_trid(v.small, nbase, false);
+  check_trid(v.mid, nbase, false);
+  if (!v.small.empty())
+    launch_trid_eigvals(c->stream, base, reinterpret_cast<const TridTask*>(db + v.o_small),
+                        int(v.small.size()), v.ns);
+  if (!v.mid.empty())
+    launch_trid_cluster(c->stream, base, reinterpret_cast<const TridTask*>(db + v.o_mid),
+                        int(v.mid.size()), v.mid[0].n, v.sum);
   cuda_check(cudaGetLastError(), "tridiagonal eigenvalues");
 }
 

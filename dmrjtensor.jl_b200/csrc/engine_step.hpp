@@ -120,6 +120,7 @@ struct RhoSolve {
   std::vector<int> tgroup;
   std::vector<int64_t> uoff;   // per group: offset of its eigenvectors (columns) in c->R
   GemmList grho;
+  TridValues tv;
 };
 // Host plan: group offsets (moff, roff, woff), eigen tasks, the rho GEMM list; ensures c->M and
 // c->R. eig_max_n: the largest block.
@@ -128,6 +129,8 @@ void plan_rho(dmrg_ctx* c, std::vector<Group>& G, bool rows, const dmrg_params& 
 // Launches (after the group matrices are in c->M and grho is uploaded at db): rho, eigenvalues,
 // and the asynchronous eigenvalue download into c->h_lam.
 void launch_rho(dmrg_ctx* c, RhoSolve& rs, char* db);
+// Its lists, into the upload whose device base launch_rho gets.
+void put_rho(Upload& u, RhoSolve& rs);
 // After the synchronisation: eigenvalues of group g (descending).
 std::vector<std::vector<double>> rho_values(dmrg_ctx* c, const std::vector<Group>& G,
                                             const RhoSolve& rs);

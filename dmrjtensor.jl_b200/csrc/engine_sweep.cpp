@@ -131,10 +131,11 @@ KrylovRun krylov_solve(dmrg_state* st, const dmrg_params& P, const HeffPlan& hp,
     tm.end(tv, 3);
     heff(K1, H);
     tv = tm.begin();
-    if (!launch_krylov(s, KRY_ALPHA, K, H, n, scal, 1, P.betatest))
+    if (!launch_krylov(s, KRY_LAST2, K, H, n, scal, 1, P.betatest)) {
       launch_mdot(s, K1, 0, 1, H, n, c->d_partial, scal + lz::ALPHA + 1);
-    launch_ritz(s, scal, 2, 0.0, false);
-    launch_lincomb(s, K, n, 2, scal + lz::COEF, H, n);
+      launch_ritz(s, scal, 2, 0.0, false);
+      launch_lincomb(s, K, n, 2, scal + lz::COEF, H, n);
+    }
     tm.end(tv, 3);
   } else {
     tv = tm.begin();
@@ -302,9 +303,14 @@ void plan_rho(dmrg_ctx* c, std::vector<Group>& G, bool rows, const dmrg_params& 
   tune_gemm(c, grho);
 }
 
+void put_rho(Upload& u, RhoSolve& rs) {
+  u.put(rs.grho);
+  put_trid_values(u, rs.ttasks, rs.tv);
+}
+
 void launch_rho(dmrg_ctx* c, RhoSolve& rs, char* db) {
   run_gemm(c, rs.grho, db, c->M.p, c->M.n, c->M.p, c->M.n, c->R.p, c->R.n);
-  run_trid_eigvals(c, c->R.p, c->R.n, rs.ttasks, 8);
+  run_trid_values(c, c->R.p, c->R.n, rs.tv, db);
   cuda_check(cudaGetLastError(), "density matrix and eigenvalue launch");
   run_eigs(c, c->R.p, c->R.n, rs.etasks, rs.J0, nullptr);
   // pinned destination: the transfer stays asynchronous and the host waits only in the step's
@@ -445,7 +451,7 @@ void twostep(dmrg_state* st, const dmrg_params& P, int j, int iL, int iR, bool f
       }
   Upload u2;
   u2.put(gather);
-  u2.put(rs.grho);
+  put_rho(u2, rs);
   char* db2 = u2.send(c, 1);
   run_copy(c, gather, db2, psi, n, c->M.p, c->M.n);
   launch_rho(c, rs, db2);

@@ -252,8 +252,10 @@ void launch_pair_dot_rows(cudaStream_t s, const double* X, int64_t x_stride, con
 //   KRY_FIRST      the first half of the 2-vector step           (dot2, lanczos2_orth, next_vector)
 //   KRY_STEP       Lanczos iteration j: alpha_j, two-term recursion, CGS2, next vector K_{j+1}
 //   KRY_ALPHA      alpha_j alone                                 (mdot)
+//   KRY_LAST2      the end of the 2-vector step: alpha_1, the Ritz pair, H = its vector
+//                                                                (mdot, ritz, lincomb)
 constexpr int KRY_MAX = 65536;
-constexpr int KRY_NORMALISE = 0, KRY_FIRST = 1, KRY_STEP = 2, KRY_ALPHA = 3;
+constexpr int KRY_NORMALISE = 0, KRY_FIRST = 1, KRY_STEP = 2, KRY_ALPHA = 3, KRY_LAST2 = 4;
 bool launch_krylov(cudaStream_t s, int mode, double* K, double* H, int64_t n, double* scal, int j,
                    double betatest);
 // y = sum_j c[j] X_j, j < k

@@ -2,7 +2,8 @@
 // vector in registers (up to KRY_MAX elements) and takes every dot product, subtraction and
 // normalisation between two Heff applications, where the general kernels (vec_kernels.cu) need a
 // launch for each: nine for a Lanczos iteration with re-orthogonalisation (45 us of kernels at
-// n = 40,000), three for the first half of the 2-vector step, two for a normalisation.
+// n = 40,000), three for the first half of the 2-vector step and three for its end, two for a
+// normalisation.
 //
 // The dot products are summed in the order of the general kernels: 256-element blocks (a warp's
 // 32 elements by shuffles over 16, 8, 4, 2, 1, the block's eight warps one after the other), then
@@ -112,6 +113,39 @@ __device__ __forceinline__ void dots(Sums& su, int k, F term) {
   su.par ^= 1;
 }
 
+// Lowest eigenpair (c0, c1) of [[a0, b], [b, a1]] by the rotations of the general Ritz kernel, in
+// its arithmetic; b = 0 after a breakdown: the first vector alone.
+__device__ __forceinline__ double ritz2(double a0, double b, double a1, double& c0, double& c1) {
+  c0 = 1.0;
+  c1 = 0.0;
+  if (!(b > 0.0)) return a0;
+  double A00 = a0, A10 = b, A01 = b, A11 = a1, V00 = 1.0, V10 = 0.0, V01 = 0.0, V11 = 1.0;
+  for (int sweep = 0; sweep < 100; ++sweep) {
+    const double off = __dmul_rn(A01, A01);
+    const double dg = __dadd_rn(__dmul_rn(A00, A00), __dmul_rn(A11, A11));
+    if (off < 1e-300 || off <= 1e-32 * dg) break;
+    const double apq = A01;
+    const double theta = (A11 - A00) / (2.0 * apq);
+    const double t = (theta >= 0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
+    const double c = 1.0 / sqrt(t * t + 1.0), sn = t * c;
+    auto rotate = [&](double& p, double& q) {
+      const double ap = p, aq = q;
+      p = fma(c, ap, -__dmul_rn(sn, aq));   // the roundings of the general kernel
+      q = fma(sn, ap, __dmul_rn(c, aq));
+    };
+    rotate(A00, A10);
+    rotate(A01, A11);
+    rotate(A00, A01);
+    rotate(A10, A11);
+    rotate(V00, V01);
+    rotate(V10, V11);
+  }
+  const bool second = A11 < A00;
+  c0 = second ? V01 : V00;
+  c1 = second ? V11 : V10;
+  return second ? A11 : A00;
+}
+
 // One cluster; n <= NQ KST. nd: dot products of the largest set; the last ncache of the Krylov
 // vectors 0..j are held in shared memory (every thread its own elements).
 template <int NQ>
@@ -164,6 +198,24 @@ k_krylov(int mode, double* __restrict__ K, double* __restrict__ H, int64_t n, do
     const double* Kj = K + int64_t(j) * n + i0;
     dots<NQ>(su, 1, [&](int, int q) { return in[q] ? Kj[q * KST] * h[q] : 0.0; });
     if (rank == 0 && tid == 0) s[lz::ALPHA + j] = su.dot[0];
+  } else if (mode == KRY_LAST2) {
+    double k[NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) k[q] = in[q] ? K[n + i0 + q * KST] : 0.0;
+    const double a0 = s[lz::ALPHA], b = s[lz::BETA];
+    dots<NQ>(su, 1, [&](int, int q) { return k[q] * h[q]; });
+    const double a1 = su.dot[0];
+    double c0, c1;
+    const double en = ritz2(a0, b, a1, c0, c1);
+#pragma unroll
+    for (int q = 0; q < NQ; ++q)
+      if (in[q]) H[i0 + q * KST] = fma(c1, k[q], __dmul_rn(c0, K[i0 + q * KST]));
+    if (rank == 0 && tid == 0) {
+      s[lz::ALPHA + 1] = a1;
+      s[lz::EN] = en;
+      s[lz::COEF] = c0;
+      s[lz::COEF + 1] = c1;
+    }
   } else {
     double b2;
     if (mode == KRY_FIRST) {
