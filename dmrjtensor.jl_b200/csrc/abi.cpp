@@ -1075,53 +1075,62 @@ int dmrg_tdvp(dmrg_state* st, const dmrg_mpo* mpo, const dmrg_params* p, double 
   });
 }
 
+static void test_syevt(dmrg_ctx* c, bool fixed, int nmat, const int* n, const int* k, double* A,
+                       double* w, double* U) {
+  if (nmat <= 0 || !n || !k || !A || !w || !U) fail(DMRG_ERR_ARG, "bad syevt arguments");
+  set_device(c);
+  int64_t ta = 0, tw = 0, tu = 0;
+  int mn = 0, mk = 0;
+  for (int i = 0; i < nmat; ++i) {
+    if (n[i] <= 0 || n[i] > (fixed ? SYEVT_RESOLVE_NMAX : SYEVT_MID_NMAX) || k[i] < 0 || k[i] > n[i])
+      fail(DMRG_ERR_SHAPE, "bad size");
+    ta += int64_t(n[i]) * n[i];
+    tw += n[i];
+    tu += int64_t(n[i]) * k[i];
+    mn = std::max(mn, n[i]);
+    mk = std::max(mk, k[i]);
+  }
+  std::vector<TridTask> tasks;
+  int64_t oa = 0, ow = ta, ows = ta + tw, ou = ta + 4 * tw;
+  for (int i = 0; i < nmat; ++i) {
+    TridTask t{};
+    t.a_off = oa;
+    t.w_off = ow;
+    t.ws_off = ows;
+    t.u_off = ou;
+    t.n = n[i];
+    t.keep = k[i];
+    tasks.push_back(t);
+    oa += int64_t(n[i]) * n[i];
+    ow += n[i];
+    ows += 3 * n[i];
+    ou += int64_t(n[i]) * k[i];
+  }
+  set_trid_paths(tasks, fixed);
+  DBuf buf;
+  dalloc(c, buf, ta + 4 * tw + tu);
+  cuda_check(cudaMemcpyAsync(buf.p, A, ta * 8, cudaMemcpyHostToDevice, c->stream), "A");
+  TridValues tv;
+  Upload u;
+  put_trid_values(u, tasks, tv);
+  run_trid_values(c, buf.p, buf.n, tv, u.send(c, 8));
+  if (mk > 0) run_trid_vectors(c, buf.p, buf.n, tasks, 6);
+  cuda_check(cudaMemcpyAsync(w, buf.p + ta, tw * 8, cudaMemcpyDeviceToHost, c->stream), "w");
+  cuda_check(cudaMemcpyAsync(U, buf.p + ta + 4 * tw, tu * 8, cudaMemcpyDeviceToHost, c->stream), "U");
+  cuda_check(cudaStreamSynchronize(c->stream), "syevt sync");
+  dfree(c, buf);
+}
+
 int dmrg_test_syevt(dmrg_ctx* c, int nmat, const int* n, const int* k, double* A, double* w,
                     double* U) {
   if (!c) return DMRG_ERR_ARG;
-  return guarded(c, [&] {
-    if (nmat <= 0 || !n || !k || !A || !w || !U) fail(DMRG_ERR_ARG, "bad syevt arguments");
-    set_device(c);
-    int64_t ta = 0, tw = 0, tu = 0;
-    int mn = 0, mk = 0;
-    for (int i = 0; i < nmat; ++i) {
-      if (n[i] <= 0 || n[i] > SYEVT_MID_NMAX || k[i] < 0 || k[i] > n[i])
-        fail(DMRG_ERR_SHAPE, "bad size");
-      ta += int64_t(n[i]) * n[i];
-      tw += n[i];
-      tu += int64_t(n[i]) * k[i];
-      mn = std::max(mn, n[i]);
-      mk = std::max(mk, k[i]);
-    }
-    std::vector<TridTask> tasks;
-    int64_t oa = 0, ow = ta, ows = ta + tw, ou = ta + 4 * tw;
-    for (int i = 0; i < nmat; ++i) {
-      TridTask t{};
-      t.a_off = oa;
-      t.w_off = ow;
-      t.ws_off = ows;
-      t.u_off = ou;
-      t.n = n[i];
-      t.keep = k[i];
-      tasks.push_back(t);
-      oa += int64_t(n[i]) * n[i];
-      ow += n[i];
-      ows += 3 * n[i];
-      ou += int64_t(n[i]) * k[i];
-    }
-    set_trid_paths(tasks);
-    DBuf buf;
-    dalloc(c, buf, ta + 4 * tw + tu);
-    cuda_check(cudaMemcpyAsync(buf.p, A, ta * 8, cudaMemcpyHostToDevice, c->stream), "A");
-    TridValues tv;
-    Upload u;
-    put_trid_values(u, tasks, tv);
-    run_trid_values(c, buf.p, buf.n, tv, u.send(c, 8));
-    if (mk > 0) run_trid_vectors(c, buf.p, buf.n, tasks, 6);
-    cuda_check(cudaMemcpyAsync(w, buf.p + ta, tw * 8, cudaMemcpyDeviceToHost, c->stream), "w");
-    cuda_check(cudaMemcpyAsync(U, buf.p + ta + 4 * tw, tu * 8, cudaMemcpyDeviceToHost, c->stream), "U");
-    cuda_check(cudaStreamSynchronize(c->stream), "syevt sync");
-    dfree(c, buf);
-  });
+  return guarded(c, [&] { test_syevt(c, false, nmat, n, k, A, w, U); });
+}
+
+int dmrg_test_syevt_fixed(dmrg_ctx* c, int nmat, const int* n, const int* k, double* A, double* w,
+                          double* U) {
+  if (!c) return DMRG_ERR_ARG;
+  return guarded(c, [&] { test_syevt(c, true, nmat, n, k, A, w, U); });
 }
 
 }  // extern "C"

@@ -511,15 +511,37 @@ void measure_correlation(dmrg_state* st, int d, const double* Cc, const double* 
                          const double* F, double* rho, double* flops, double* norm = nullptr);
 
 // ---- eigensolves (engine_eig.cpp)
-// Tridiagonal-path eigenvalues of every task (n <= SYEVT_MID_NMAX; small and mid-size blocks in
-// one launch each), then the kept eigenvectors (tasks with keep > 0; mid-size blocks use c->W
-// as workspace). Offsets are checked against nbase before any launch.
-void set_trid_paths(std::vector<TridTask>& t);
+// Solves whose sums keep one order for good: their density-matrix blocks take the one-CTA kernels
+// (block Jacobi above SYEVT_RESOLVE_NMAX states) and their Ritz step the cyclic rotations. Another
+// order rotates kept vectors of nearly equal weight among themselves, which is as right, but some
+// solves multiply any such difference by so much that a program which compares runs would see their
+// results change by far more than rounding. How far the records and (in 32 bits) the correlations
+// after one or two sweeps from a random state move at most between the clusters' order and this one,
+// which is as far as an input changed by 1e-15 moves them in either:
+//   split precision, whose products round at 2^-24 or so in a way that depends on the basis:
+//     2 vectors             1.4e-4 (of 1,093 sweeps three above 2e-5)
+//     4 and 8 vectors       1.3e-2 (of 158 sweeps thirteen above 2e-5)
+//   FP64:
+//     2 vectors             records 1.5e-11, correlations 2.5e-9 (62 sweeps)
+//     4 vectors             7.5e-12, 1.1e-8 (113)
+//     8, up to 24 sites     4.2e-10, 4.9e-8 (400)
+//     8, 25 to 100 sites    2.4e-5, 3.3e-3 (200, one in ten above 1e-9)
+//     TDVP, up to 8         3.3e-11, 2.0e-9 (51)
+// The others take the clusters, which are faster from 40 states on: 0.6 against 4.6 ms for the values
+// of a block of 345 states; a half-filled Hubbard sweep of 32 sites and 400 states takes 65 ms with
+// them and 218 ms in this order.
+constexpr int FIXED_KRYLOV = 4, FIXED_SITES = 24;
+bool fixed_order(const dmrg_params& P, int L, bool tdvp);
+// The family of kernels that solves each block of a step (TridTask::path).
+void set_trid_paths(std::vector<TridTask>& t, bool fixed);
+// Tridiagonal-path eigenvalues of every task, then the kept eigenvectors (tasks with keep > 0; the
+// two families of larger blocks use c->W as workspace). Offsets are checked against nbase before any
+// launch.
 struct TridValues {              // the eigenvalue launches' lists, sent with the caller's upload
-  std::vector<TridTask> small, mid;
-  int ns = 0;                    // largest small block
-  int64_t sum = 0;               // mid-size blocks' states
-  size_t o_small = 0, o_mid = 0;
+  std::vector<TridTask> t[3];    // by path
+  int nmax[3] = {0, 0, 0};       // largest block
+  int64_t sum = 0;               // TRID_CLUSTER: the blocks' states
+  size_t off[3] = {0, 0, 0};
 };
 void put_trid_values(Upload& u, const std::vector<TridTask>& t, TridValues& v);
 void run_trid_values(dmrg_ctx* c, double* base, int64_t nbase, const TridValues& v, char* db);

@@ -131,7 +131,7 @@ void single_site_step(dmrg_state* st, const dmrg_params& P, const SiteMode& md, 
           it->second.np += Br.dim[kbp];
         }
     for (auto& kv : gm) G.push_back(kv.second);
-    plan_rho(c, G, true, P, rs, &so.eig_max_n);
+    plan_rho(c, G, true, P, fixed_order(P, st->L, md.tdvp), rs, &so.eig_max_n);
     for (const Group& g : G) {
       const bool orig = !g.cols.empty() && g.cols[0].s < 0;
       for (const Piece& r : g.rows) {
@@ -205,7 +205,7 @@ void single_site_step(dmrg_state* st, const dmrg_params& P, const SiteMode& md, 
           it->second.n += Bl.dim[ka];
         }
     for (auto& kv : gm) G.push_back(kv.second);
-    plan_rho(c, G, false, P, rs, &so.eig_max_n);
+    plan_rho(c, G, false, P, fixed_order(P, st->L, md.tdvp), rs, &so.eig_max_n);
     for (const Group& g : G) {
       if (g.rows.empty() || g.rows[0].s >= 0) continue;
       const int ka = g.rows[0].sec;

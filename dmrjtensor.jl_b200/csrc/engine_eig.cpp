@@ -8,10 +8,11 @@
 namespace dmrg {
 
 namespace {
+constexpr int TRID_NMAX[3] = {SYEVT_NMAX, SYEVT_MID_NMAX, SYEVT_RESOLVE_NMAX};   // by path
 void check_trid(const std::vector<TridTask>& ts, int64_t nbase, bool vectors) {
   for (const TridTask& t : ts) {
     const int64_t nn = int64_t(t.n) * t.n;
-    if (t.n <= 0 || t.n > (t.mid ? SYEVT_MID_NMAX : SYEVT_NMAX) || t.a_off < 0 || t.a_off + nn > nbase ||
+    if (t.n <= 0 || t.n > TRID_NMAX[t.path] || t.a_off < 0 || t.a_off + nn > nbase ||
         t.w_off < 0 || t.w_off + t.n > nbase || t.ws_off < 0 || t.ws_off + 3 * t.n > nbase)
       fail(DMRG_ERR_ARG, "internal plan check failed: tridiagonal eigensolver task");
     if (vectors && (t.keep < 0 || t.keep > t.n || t.u_off < 0 ||
@@ -19,70 +20,91 @@ void check_trid(const std::vector<TridTask>& ts, int64_t nbase, bool vectors) {
       fail(DMRG_ERR_ARG, "internal plan check failed: tridiagonal eigenvector task");
   }
 }
+const TridTask* at(const char* db, size_t off) {
+  return reinterpret_cast<const TridTask*>(db + off);
+}
 }  // namespace
 
-void set_trid_paths(std::vector<TridTask>& t) {
+bool fixed_order(const dmrg_params& P, int L, bool tdvp) {
+  return split_form(P.precision) != 0 || (!tdvp && P.krylov > FIXED_KRYLOV && L > FIXED_SITES);
+}
+
+void set_trid_paths(std::vector<TridTask>& t, bool fixed) {
   int nmax = 0;
   for (const TridTask& x : t) nmax = std::max(nmax, x.n);
-  for (TridTask& x : t) x.mid = nmax > SYEVT_ROUTE ? 1 : 0;
+  for (TridTask& x : t)
+    x.path = fixed ? (x.n <= SYEVT_NMAX ? TRID_SMALL : TRID_BLOCK)
+                   : (nmax > SYEVT_ROUTE ? TRID_CLUSTER : TRID_SMALL);
 }
 
 void put_trid_values(Upload& u, const std::vector<TridTask>& t, TridValues& v) {
   v = TridValues{};
   for (const TridTask& x : t) {
-    if (!x.mid) { v.small.push_back(x); v.ns = std::max(v.ns, x.n); }
-    else { v.mid.push_back(x); v.sum += x.n; }
+    v.t[x.path].push_back(x);
+    v.nmax[x.path] = std::max(v.nmax[x.path], x.n);
+    if (x.path == TRID_CLUSTER) v.sum += x.n;
   }
   // the largest first: not all clusters of a long list are resident at once
-  std::stable_sort(v.mid.begin(), v.mid.end(),
+  std::stable_sort(v.t[TRID_CLUSTER].begin(), v.t[TRID_CLUSTER].end(),
                    [](const TridTask& a, const TridTask& b) { return a.n > b.n; });
-  v.o_small = u.put(v.small);
-  v.o_mid = u.put(v.mid);
+  for (int p = 0; p < 3; ++p) v.off[p] = u.put(v.t[p]);
 }
 
 void run_trid_values(dmrg_ctx* c, double* base, int64_t nbase, const TridValues& v, char* db) {
-  check_trid(v.small, nbase, false);
-  check_trid(v.mid, nbase, false);
-  if (!v.small.empty())
-    launch_trid_eigvals(c->stream, base, reinterpret_cast<const TridTask*>(db + v.o_small),
-                        int(v.small.size()), v.ns);
-  if (!v.mid.empty())
-    launch_trid_cluster(c->stream, base, reinterpret_cast<const TridTask*>(db + v.o_mid),
-                        int(v.mid.size()), v.mid[0].n, v.sum);
+  for (int p = 0; p < 3; ++p) {
+    const int n = int(v.t[p].size());
+    if (n == 0) continue;
+    check_trid(v.t[p], nbase, false);
+    const TridTask* tasks = at(db, v.off[p]);
+    if (p == TRID_SMALL) launch_trid_eigvals(c->stream, base, tasks, n, v.nmax[p]);
+    else if (p == TRID_BLOCK) launch_trid_block_eigvals(c->stream, base, tasks, n, v.nmax[p]);
+    else launch_trid_cluster(c->stream, base, tasks, n, v.nmax[p], v.sum);
+  }
   cuda_check(cudaGetLastError(), "tridiagonal eigenvalues");
 }
 
 void run_trid_vectors(dmrg_ctx* c, double* base, int64_t nbase, std::vector<TridTask> t,
                       int slot) {
   check_trid(t, nbase, true);
-  std::vector<TridTask> small, mid;
-  int ns = 0, ks = 0, nm = 0, km = 0;
+  // one launch per path; TRID_BLOCK in two: the blocks whose Gram matrix fits in shared memory
+  // beside their vectors, and the rest (which keep the whole L1 for their global-memory Gram)
+  std::vector<TridTask> list[4];
+  int nmax[4] = {0, 0, 0, 0}, kmax[4] = {0, 0, 0, 0}, nblock = 0;
+  for (const TridTask& x : t)
+    if (x.keep > 0 && x.path == TRID_BLOCK) nblock = std::max(nblock, x.n);
+  const int kg = nblock > 0 ? syevt_block_gram_limit(nblock) : 0;
   int64_t xw = 0;
   for (TridTask x : t) {
     if (x.keep <= 0) continue;
-    if (!x.mid) {
-      small.push_back(x);
-      ns = std::max(ns, x.n);
-      ks = std::max(ks, x.keep);
-    } else {
+    if (x.path != TRID_SMALL) {
       x.x_off = xw;
-      xw += syevt_mid_workspace(x.n, x.keep);
-      mid.push_back(x);
-      nm = std::max(nm, x.n);
-      km = std::max(km, x.keep);
+      xw += x.path == TRID_BLOCK ? syevt_block_workspace(x.n, x.keep)
+                                 : syevt_mid_workspace(x.n, x.keep);
     }
+    const int l = x.path == TRID_BLOCK && x.keep > kg ? 3 : x.path;
+    list[l].push_back(x);
+    nmax[l] = std::max(nmax[l], x.n);
+    kmax[l] = std::max(kmax[l], x.keep);
   }
-  if (small.empty() && mid.empty()) return;
-  if (xw > 0) ensure(c, c->W, xw);
   Upload u;
-  const size_t o1 = u.put(small), o2 = u.put(mid);
+  size_t off[4];
+  bool any = false;
+  for (int l = 0; l < 4; ++l) {
+    off[l] = u.put(list[l]);
+    any |= !list[l].empty();
+  }
+  if (!any) return;
+  if (xw > 0) ensure(c, c->W, xw);
   char* db = u.send(c, slot);
-  if (!small.empty())
-    launch_trid_vectors(c->stream, base, reinterpret_cast<const TridTask*>(db + o1),
-                        int(small.size()), ns, ks);
-  if (!mid.empty())
-    launch_trid_mid_vectors(c->stream, base, reinterpret_cast<const TridTask*>(db + o2),
-                            int(mid.size()), nm, km, c->W.p);
+  for (int l = 0; l < 4; ++l) {
+    const int n = int(list[l].size());
+    if (n == 0) continue;
+    const TridTask* tasks = at(db, off[l]);
+    if (l == TRID_SMALL) launch_trid_vectors(c->stream, base, tasks, n, nmax[l], kmax[l]);
+    else if (l == TRID_CLUSTER)
+      launch_trid_mid_vectors(c->stream, base, tasks, n, nmax[l], kmax[l], c->W.p);
+    else launch_trid_block_vectors(c->stream, base, tasks, n, nmax[l], kmax[l], c->W.p);
+  }
   cuda_check(cudaGetLastError(), "tridiagonal eigenvectors");
 }
 

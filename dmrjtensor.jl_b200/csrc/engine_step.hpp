@@ -123,9 +123,9 @@ struct RhoSolve {
   TridValues tv;
 };
 // Host plan: group offsets (moff, roff, woff), eigen tasks, the rho GEMM list; ensures c->M and
-// c->R. eig_max_n: the largest block.
-void plan_rho(dmrg_ctx* c, std::vector<Group>& G, bool rows, const dmrg_params& P, RhoSolve& rs,
-              int* eig_max_n);
+// c->R. fixed: fixed_order(...); eig_max_n: the largest block.
+void plan_rho(dmrg_ctx* c, std::vector<Group>& G, bool rows, const dmrg_params& P, bool fixed,
+              RhoSolve& rs, int* eig_max_n);
 // Launches (after the group matrices are in c->M and grho is uploaded at db): rho, eigenvalues,
 // and the asynchronous eigenvalue download into c->h_lam.
 void launch_rho(dmrg_ctx* c, RhoSolve& rs, char* db);

@@ -133,7 +133,7 @@ KrylovRun krylov_solve(dmrg_state* st, const dmrg_params& P, const HeffPlan& hp,
     tv = tm.begin();
     if (!launch_krylov(s, KRY_LAST2, K, H, n, scal, 1, P.betatest)) {
       launch_mdot(s, K1, 0, 1, H, n, c->d_partial, scal + lz::ALPHA + 1);
-      launch_ritz(s, scal, 2, 0.0, false);
+      launch_ritz(s, scal, 2, 0.0, false, true);
       launch_lincomb(s, K, n, 2, scal + lz::COEF, H, n);
     }
     tm.end(tv, 3);
@@ -164,7 +164,7 @@ KrylovRun krylov_solve(dmrg_state* st, const dmrg_params& P, const HeffPlan& hp,
       tm.end(tv, 3);
     }
     tv = tm.begin();
-    launch_ritz(s, scal, kdim, tau, expo);
+    launch_ritz(s, scal, kdim, tau, expo, fixed_order(P, st->L, expo));
     launch_lincomb(s, K, n, kdim, scal + lz::COEF, H, n);
     tm.end(tv, 3);
   }
@@ -235,8 +235,8 @@ double krylov_energy(dmrg_ctx* c, const KrylovRun& kr) {
   return e;
 }
 
-void plan_rho(dmrg_ctx* c, std::vector<Group>& G, bool rows, const dmrg_params& P, RhoSolve& rs,
-              int* eig_max_n) {
+void plan_rho(dmrg_ctx* c, std::vector<Group>& G, bool rows, const dmrg_params& P, bool fixed,
+              RhoSolve& rs, int* eig_max_n) {
   // side = dimension of the density matrix that is diagonalised (rows of M, or its columns)
   rs.rows = rows;
   rs.mtot = rs.rtot = rs.wtot = 0;
@@ -254,8 +254,8 @@ void plan_rho(dmrg_ctx* c, std::vector<Group>& G, bool rows, const dmrg_params& 
   // of its own row and column. Blocks above SYEVT_RESOLVE_NMAX therefore take the tridiagonal path
   // only where the cutoff keeps the cut far above that: with cutoff 0, where the sign of the last
   // weights decides, a dense L = 20 sweep at m = 384 kept 252 states instead of 384.
-  const int trid_max = P.cutoff >= 1e-11 && P.minm <= SYEVT_NMAX ? SYEVT_MID_NMAX
-                                                                 : SYEVT_RESOLVE_NMAX;
+  const int trid_max = !fixed && P.cutoff >= 1e-11 && P.minm <= SYEVT_NMAX ? SYEVT_MID_NMAX
+                                                                           : SYEVT_RESOLVE_NMAX;
   rs.etasks.clear();
   rs.ttasks.clear();
   rs.tgroup.clear();
@@ -285,7 +285,7 @@ void plan_rho(dmrg_ctx* c, std::vector<Group>& G, bool rows, const dmrg_params& 
       rs.uoff[gi] = g.roff;      // block Jacobi returns the eigenvectors in place
     }
   }
-  set_trid_paths(rs.ttasks);
+  set_trid_paths(rs.ttasks, fixed);
   const int64_t ews = eig_workspace(rs.etasks);
   ensure(c, c->M, std::max<int64_t>(rs.mtot, 1));
   ensure(c, c->R, std::max<int64_t>(rs.J0 + ews, 1));
@@ -436,7 +436,7 @@ void twostep(dmrg_state* st, const dmrg_params& P, int j, int iL, int iR, bool f
     for (const Piece& p : G[g].cols) coloff[p.sec * d2 + p.s] = p.off;
   }
   RhoSolve rs;
-  plan_rho(c, G, j > 0, P, rs, &so.eig_max_n);
+  plan_rho(c, G, j > 0, P, fixed_order(P, st->L, mode.tdvp), rs, &so.eig_max_n);
   CopyList gather;
   for (int ka = 0; ka < tl.nl; ++ka)
     for (int s1 = 0; s1 < d1; ++s1)

@@ -74,34 +74,46 @@ struct EigTask {
   int n, pad;
 };
 
-// Tridiagonal eigensolver for density-matrix blocks: one CTA per block for n <= SYEVT_NMAX
-// (syevt.cu), clusters for n <= SYEVT_MID_NMAX (syevt_cluster.cu and syevt_mid.cu; that line is
-// where the smaller kernels' shared memory ends: at n = 1024 with 512 vectors 7.5 ms against about
-// 90 ms of block Jacobi sweeps).
+// Tridiagonal eigensolver for density-matrix blocks. Three families (TridTask::path, chosen by
+// set_trid_paths): one CTA per block with the matrix in shared memory, n <= SYEVT_NMAX (syevt.cu);
+// one CTA per block with the matrix in global memory, n <= SYEVT_RESOLVE_NMAX (syevt_block.cu);
+// clusters and many CTAs, n <= SYEVT_MID_NMAX (syevt_cluster.cu and syevt_mid.cu; that line is where
+// their shared memory ends: at n = 1024 with 512 vectors 7.5 ms against about 90 ms of block Jacobi
+// sweeps).
 constexpr int SYEVT_NMAX = 112;
 constexpr int SYEVT_MID_NMAX = 2048;
-constexpr int SYEVT_RESOLVE_NMAX = 512;   // its limit where weights at the rounding level matter
+constexpr int SYEVT_RESOLVE_NMAX = 512;   // limit of the path where weights at the rounding level matter
+constexpr int TRID_SMALL = 0, TRID_CLUSTER = 1, TRID_BLOCK = 2;
 struct TridTask {
   int64_t a_off;   // n x n matrix (column-major, ld n); reflectors are stored in its lower part
   int64_t w_off;   // n eigenvalues, descending
   int64_t ws_off;  // 3n workspace: d, e, tau
   int64_t u_off;   // n x keep eigenvectors (launch 2)
   int n, keep;
-  int64_t x_off;   // mid-size launches: workspace offset (syevt_mid_workspace(n, keep) doubles)
-  int mid = 0;     // the block takes the mid-size kernels (set_trid_paths)
+  int64_t x_off;   // vector launches of the larger families: workspace offset (trid_workspace)
+  int path = TRID_SMALL;
   int pad = 0;
 };
-// The blocks of one step run side by side, so they take one path where they can: the mid-size
-// kernels for all of them once the largest has more than SYEVT_ROUTE states. One CTA per block is
+// The blocks of one step run side by side, so they take one family where they can: the clusters
+// for all of them once the largest has more than SYEVT_ROUTE states. One CTA per block is
 // as fast up to there (values and vectors, largest block 48 states: 85 against 80 us), above it the
-// clusters win (85 states: 185 against 135 us), and both paths one after the other would cost
-// their sum.
+// clusters win (85 states: 185 against 135 us), and both one after the other would cost their sum.
 constexpr int SYEVT_ROUTE = 40;
 size_t syevt_smem_vals(int n);
 size_t syevt_smem_vecs(int n, int k);
 void launch_trid_eigvals(cudaStream_t s, double* base, const TridTask* tasks, int ntasks, int max_n);
 void launch_trid_vectors(cudaStream_t s, double* base, const TridTask* tasks, int ntasks,
                          int max_n, int max_k);
+// TRID_BLOCK. The workspace of a task's vectors in doubles; the largest kept count whose Gram
+// matrix the vector kernel holds in shared memory for blocks up to max_n (tasks above it take the
+// global-memory form; launch them separately).
+int64_t syevt_block_workspace(int n, int k);
+int syevt_block_gram_limit(int max_n);
+void launch_trid_block_eigvals(cudaStream_t s, double* base, const TridTask* tasks, int ntasks,
+                               int max_n);
+void launch_trid_block_vectors(cudaStream_t s, double* base, const TridTask* tasks, int ntasks,
+                               int max_n, int max_k, double* xws);
+// TRID_CLUSTER. The workspace of a task's vectors in doubles.
 int64_t syevt_mid_workspace(int n, int k);
 // Tridiagonalisation by thread-block clusters and all eigenvalues (syevt_cluster.cu); sum_n: the
 // blocks' sizes added up.
@@ -235,8 +247,9 @@ void launch_lanczos2_orth(cudaStream_t s, double* K, double* H, int64_t n, doubl
 void launch_next_vector(cudaStream_t s, const double* H, double* Kn, int64_t n, double* scal,
                         int j, double betatest);
 // lowest Ritz pair of the Krylov tridiagonal: s[EN], s[COEF + j]; with expo the coefficients of
-// exp(tau T) e_1 instead (s[EN] still the lowest eigenvalue)
-void launch_ritz(cudaStream_t s, double* scal, int kdim, double tau, bool expo);
+// exp(tau T) e_1 instead (s[EN] still the lowest eigenvalue). cyclic: by Jacobi rotations in the
+// fixed serial order whatever kdim (fixed_order solves)
+void launch_ritz(cudaStream_t s, double* scal, int kdim, double tau, bool expo, bool cyclic);
 // out[0] = sum over the pair tasks (total elements `total`; deterministic order)
 void launch_pair_dot(cudaStream_t s, const double* X, const double* Y, const PairTask* tasks,
                      int ntasks, int64_t total, double* partial, double* out);

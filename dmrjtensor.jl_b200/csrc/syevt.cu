@@ -15,7 +15,7 @@
 // The host then truncates globally and asks for the top-k vectors of each block.
 // Launch 2 (k_trid_vectors):
 //   * eigenvectors of T by inverse iteration on (T - lambda I) with partial-pivoting LU, one
-//     thread per vector (two iterations from a fixed pseudo-random start; factors in shared
+//     thread per vector (three iterations from a fixed pseudo-random start; factors in shared
 //     memory). Vectors of (nearly) equal eigenvalues come out as independent vectors of their
 //     common eigenspace; kept eigenvalues below 1e-13 ||T|| (numerically zero) start from the
 //     pseudo-random vector alone (an orthonormal completion after the next step);
@@ -302,7 +302,7 @@ k_trid_eigvals(double* __restrict__ base, const TridTask* __restrict__ tasks) {
 
 // Shared-memory layout of k_trid_vectors (doubles first, then ints).
 __host__ __device__ size_t vec_union_doubles(int n, int k, int nslot) {
-  size_t u = size_t(3) * nslot * n;
+  size_t u = size_t(4) * nslot * n;
   if (size_t(k) * k > u) u = size_t(k) * k;
   if (size_t(n) * n > u) u = size_t(n) * n;
   return u;
@@ -363,9 +363,9 @@ k_trid_vectors(double* __restrict__ base, const TridTask* __restrict__ tasks, in
     const int j = b0 + tid;
     if (tid < nslot && j < kk) {
       LUSlot f{Un + tid, Un + int64_t(nslot) * n + tid, Un + int64_t(2) * nslot * n + tid,
-               piv + tid, nslot};
-      if (W[j] > 1e-13 * tn) inverse_iteration(d, e, n, W[j], Z + j, ldz, j, tn, f);
-      else for (int r = 0; r < n; ++r) Z[r * ldz + j] = prand(r, j);
+               Un + int64_t(3) * nslot * n + tid, piv + tid, nslot};
+      for (int r = 0; r < n; ++r) Z[r * ldz + j] = prand(r, j);
+      if (W[j] > 1e-13 * tn) inverse_iteration(d, e, n, W[j], Z, ldz, j, tn, f);
     }
     __syncthreads();
   }

@@ -27,7 +27,7 @@
 #include "cluster.cuh"
 #include "kernels.cuh"
 #include "launch.cuh"
-#include "syevt_common.cuh"
+#include "trid_solve.cuh"
 
 namespace dmrg {
 namespace {
@@ -563,7 +563,7 @@ k_trid_sturm(double* __restrict__ base, const TridTask* __restrict__ tasks) {
     if (!done) {
       const double xl = a + wd * frac, xh = a + wd * (double(P) * frac);
       if (wd <= tol || !(a < xl && xl < xh && xh < b)) done = true;   // converged / no progress
-      else below = sturm_below(d, e2, n, a + wd * (double(h + 1) * frac)) > target;
+      else below = sturm_lagged(d, e2, n, a + wd * (double(h + 1) * frac)) > target;
     }
     const unsigned bal = __ballot_sync(FULL, below);
     if (!done) {

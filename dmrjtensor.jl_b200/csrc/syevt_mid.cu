@@ -20,7 +20,7 @@
 
 #include "kernels.cuh"
 #include "launch.cuh"
-#include "syevt_common.cuh"
+#include "trid_solve.cuh"
 
 namespace dmrg {
 namespace {
@@ -64,10 +64,10 @@ k_mid_invit(double* __restrict__ base, const TridTask* __restrict__ tasks,
   double* z = F + 3 * nl;
   if (lane < lanes && j < kk) {
     const double tn = fmax(fmax(fabs(W[0]), fabs(W[n - 1])), 1e-300);   // descending
-    LUSlot f{F + lane, F + nl + lane, F + 2 * nl + lane, reinterpret_cast<int*>(F + 4 * nl) + lane,
+    LeanSlot f{F + lane, F + nl + lane, F + 2 * nl + lane, reinterpret_cast<int*>(F + 4 * nl) + lane,
              lanes};
     // kept eigenvalues that are numerically zero keep the pseudo-random vector alone
-    if (W[j] > 1e-13 * tn) inverse_iteration(d, e, n, W[j], z + lane, lanes, j, tn, f);
+    if (W[j] > 1e-13 * tn) lean_inverse_iteration(d, e, n, W[j], z + lane, lanes, j, tn, f);
     else for (int r = 0; r < n; ++r) z[r * lanes + lane] = prand(r, j);
   }
   __syncwarp();

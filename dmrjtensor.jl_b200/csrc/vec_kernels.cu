@@ -6,7 +6,7 @@
 
 #include "kernels.cuh"
 #include "launch.cuh"
-#include "syevt_common.cuh"
+#include "trid_solve.cuh"
 
 namespace dmrg {
 namespace {
@@ -394,14 +394,14 @@ __device__ bool lowest_pair(double* s, int kdim) {
   double a = lo - 2.2e-16 * tn, b = hi + 2.2e-16 * tn;   // no eigenvalue below a, all below b
   for (int it = 0; it < 64 && b - a > tol; ++it) {
     const double w = (b - a) * (1.0 / 33.0);
-    const unsigned below = __ballot_sync(FULL, sturm_below(d, e2, m, a + w * (lane + 1)) > 0);
+    const unsigned below = __ballot_sync(FULL, sturm_lagged(d, e2, m, a + w * (lane + 1)) > 0);
     const int g = below ? __ffs(below) - 1 : 32;         // the lowest lies in (x_(g-1), x_g]
     const double x = a + w * g;
     if (g < 32) b = a + w * (g + 1);
     a = x;
   }
   if (lane == 0)
-    inverse_iteration(d, e, m, 0.5 * (a + b), z, 1, 0, tn, LUSlot{u0, u1, l, piv, 1});
+    lean_inverse_iteration(d, e, m, 0.5 * (a + b), z, 1, 0, tn, LeanSlot{u0, u1, l, piv, 1});
   __syncwarp();
   const double sg = z[0] < 0.0 ? -1.0 : 1.0;
   const double zi = lane < m ? sg * z[lane] : 0.0, zn = lane + 1 < m ? sg * z[lane + 1] : 0.0;
@@ -411,25 +411,9 @@ __device__ bool lowest_pair(double* s, int kdim) {
   return true;
 }
 
-// Ritz step of the Krylov solve, one warp: T = tridiag(alpha, beta) of the m active vectors
-// (m = 1 + number of leading non-zero beta_j, at most kdim), Jacobi rotations until the
-// off-diagonal is at the rounding level of the diagonal, lowest eigenvalue -> s[EN], its
-// eigenvector -> s[COEF + j] (0 for j >= m). The rotations of a round are disjoint pairs (the
-// round-robin order of a tournament), one lane per angle and one lane per element of the row,
-// column and vector updates: m - 1 rounds a sweep instead of m (m - 1) / 2 rotations one after the
-// other, each of which is a chain of square roots and divisions (m = 8: 81 -> 35 us). A
-// 2-vector step is one rotation, written out. Only expo and 2-vector steps get there: the lowest
-// pair of three or more vectors alone is lowest_pair.
-// expo = 0: the lowest Ritz pair (s[EN], s[COEF + j]). expo = 1: s[COEF + j] = (exp(tau T) e_1)_j
-// (krylovTimeEvol, algs/time.jl:182-203: the Krylov vectors are orthonormal, so these are the
-// coefficients of exp(tau H) applied to the normalised start vector), from the eigenpairs of T;
-// when they sum to exactly zero, the first column of I + T instead. s[EN] = lowest eigenvalue.
-__global__ void k_ritz(double* s, int kdim, double tau, int expo) {
-  grid_entry();
-  if (!expo && kdim > 2 && lowest_pair(s, kdim)) return;
-  __shared__ double A[MAXK * MAXK], V[MAXK * MAXK];
-  __shared__ double rc[MAXK / 2], rs[MAXK / 2];
-  __shared__ int rp[MAXK / 2], rq[MAXK / 2];
+// The projected matrix T = tridiag(alpha, beta) of the m active Krylov vectors into A, the unit
+// matrix into V (one warp); returns m = 1 + number of leading non-zero beta_j, at most kdim.
+__device__ __forceinline__ int ritz_matrix(const double* s, double* A, double* V, int kdim) {
   const int lane = threadIdx.x;
   int m = 1;
   while (m < kdim && s[lz::BETA + m - 1] > 0.0) ++m;
@@ -442,6 +426,100 @@ __global__ void k_ritz(double* s, int kdim, double tau, int expo) {
     A[e] = v;
     V[e] = (r == c) ? 1.0 : 0.0;
   }
+  return m;
+}
+
+// The results of a diagonalised T (A: its eigenvalues, V: its eigenvectors).
+// expo = 0: the lowest Ritz pair (s[EN], s[COEF + j]). expo = 1: s[COEF + j] = (exp(tau T) e_1)_j
+// (krylovTimeEvol, algs/time.jl:182-203: the Krylov vectors are orthonormal, so these are the
+// coefficients of exp(tau H) applied to the normalised start vector), from the eigenpairs of T;
+// when they sum to exactly zero, the first column of I + T instead. s[EN] = lowest eigenvalue.
+__device__ __forceinline__ void ritz_result(double* s, const double* A, const double* V, int m,
+                                            int kdim, double tau, int expo) {
+  const int lane = threadIdx.x;
+  int o = 0;
+  for (int k = 1; k < m; ++k)
+    if (A[k + k * m] < A[o + o * m]) o = k;   // lowest; ties keep the lower index
+  if (lane == 0) s[lz::EN] = A[o + o * m];
+  if (!expo) {
+    for (int k = lane; k < kdim; k += 32) s[lz::COEF + k] = (k < m) ? V[k + o * m] : 0.0;
+    return;
+  }
+  // c_k = sum_j V[k,j] exp(tau lambda_j) V[0,j]; every lane forms the sum of all c_k itself (the
+  // same fixed order in each lane) for the zero test
+  double tot = 0.0, mine = 0.0;
+  for (int k = 0; k < m; ++k) {
+    double ck = 0.0;
+    for (int jj = 0; jj < m; ++jj) ck += V[k + jj * m] * exp(tau * A[jj + jj * m]) * V[jj * m];
+    tot += ck;
+    if (k == lane) mine = ck;
+  }
+  if (tot == 0.0) {   // (I + T) e_1
+    mine = lane == 0 ? 1.0 + s[lz::ALPHA] : (lane == 1 && m > 1 ? s[lz::BETA] : 0.0);
+  }
+  for (int k = lane; k < kdim; k += 32) s[lz::COEF + k] = (k < m) ? mine : 0.0;
+}
+
+// Ritz step of the Krylov solve, one warp: T = tridiag(alpha, beta) of the m active vectors
+// (ritz_matrix), cyclic Jacobi (serial rotation
+// order; lanes own the rows/columns of one rotation) until the off-diagonal is at the rounding
+// level of the diagonal, lowest eigenvalue -> s[EN], its eigenvector -> s[COEF + j] (0 for j >= m).
+// For two vectors, where it is one rotation, and for fixed_order solves whatever kdim (m = 8: 81 us a
+// launch; k_ritz needs 6.6 or 35).
+__global__ void k_ritz_cyclic(double* s, int kdim, double tau, int expo) {
+  grid_entry();
+  __shared__ double A[MAXK * MAXK], V[MAXK * MAXK];
+  const int lane = threadIdx.x;
+  const int m = ritz_matrix(s, A, V, kdim);
+  __syncwarp();
+  for (int sweep = 0; sweep < 100; ++sweep) {
+    double off = 0.0, dg = 0.0;
+    for (int p = 0; p < m; ++p) {
+      dg += A[p + p * m] * A[p + p * m];
+      for (int q = p + 1; q < m; ++q) off += A[p + q * m] * A[p + q * m];
+    }
+    if (off < 1e-300 || off <= 1e-32 * dg) break;   // off-diagonal at the rounding level
+    for (int p = 0; p < m; ++p)
+      for (int q = p + 1; q < m; ++q) {
+        const double apq = A[p + q * m];
+        if (fabs(apq) < 1e-300) continue;
+        const double theta = (A[q + q * m] - A[p + p * m]) / (2.0 * apq);
+        const double t = (theta >= 0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
+        const double c = 1.0 / sqrt(t * t + 1.0), sn = t * c;
+        __syncwarp();
+        if (lane < m) {   // rows p, q
+          const double ap = A[p + lane * m], aq = A[q + lane * m];
+          A[p + lane * m] = c * ap - sn * aq;
+          A[q + lane * m] = sn * ap + c * aq;
+        }
+        __syncwarp();
+        if (lane < m) {   // columns p, q
+          const double ap = A[lane + p * m], aq = A[lane + q * m];
+          A[lane + p * m] = c * ap - sn * aq;
+          A[lane + q * m] = sn * ap + c * aq;
+          const double vp = V[lane + p * m], vq = V[lane + q * m];
+          V[lane + p * m] = c * vp - sn * vq;
+          V[lane + q * m] = sn * vp + c * vq;
+        }
+        __syncwarp();
+      }
+  }
+  ritz_result(s, A, V, m, kdim, tau, expo);
+}
+
+// The same for three or more vectors in the other solves: the lowest pair by lowest_pair; with expo
+// the rotations of a round are disjoint pairs (the round-robin order of a tournament), one lane per
+// angle and one lane per element of the row, column and vector updates: m - 1 rounds a sweep instead
+// of m (m - 1) / 2 rotations one after the other, each of which is a chain of square roots and
+// divisions (m = 8: 81 -> 35 us).
+__global__ void k_ritz(double* s, int kdim, double tau, int expo) {
+  grid_entry();
+  if (!expo && kdim > 2 && lowest_pair(s, kdim)) return;
+  __shared__ double A[MAXK * MAXK], V[MAXK * MAXK];
+  __shared__ double rc[MAXK / 2], rs[MAXK / 2];
+  __shared__ int rp[MAXK / 2], rq[MAXK / 2];
+  const int lane = threadIdx.x;
+  const int m = ritz_matrix(s, A, V, kdim);
   __syncwarp();
   // this lane's elements e = lane, lane + 32, ... of a row or column update: pair e / m, index e % m
   const int x0 = lane / m, i0 = lane - x0 * m, xs = 32 / m, is = 32 - xs * m;
@@ -456,30 +534,6 @@ __global__ void k_ritz(double* s, int kdim, double tau, int expo) {
     off = warp_sum(off);
     dg = warp_sum(dg);
     if (off < 1e-300 || off <= 1e-32 * dg) break;   // off-diagonal at the rounding level
-    if (m == 2) {
-      const int p = 0, q = 1;
-      const double apq = A[p + q * m];
-      const double theta = (A[q + q * m] - A[p + p * m]) / (2.0 * apq);
-      const double t = (theta >= 0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
-      const double c = 1.0 / sqrt(t * t + 1.0), sn = t * c;
-      __syncwarp();
-      if (lane < m) {   // rows p, q
-        const double ap = A[p + lane * m], aq = A[q + lane * m];
-        A[p + lane * m] = c * ap - sn * aq;
-        A[q + lane * m] = sn * ap + c * aq;
-      }
-      __syncwarp();
-      if (lane < m) {   // columns p, q
-        const double ap = A[lane + p * m], aq = A[lane + q * m];
-        A[lane + p * m] = c * ap - sn * aq;
-        A[lane + q * m] = sn * ap + c * aq;
-        const double vp = V[lane + p * m], vq = V[lane + q * m];
-        V[lane + p * m] = c * vp - sn * vq;
-        V[lane + q * m] = sn * vp + c * vq;
-      }
-      __syncwarp();
-      continue;
-    }
     for (int round = 0; round < mm - 1; ++round) {
       if (lane < mm / 2) {
         // pair of this lane: index mm - 1 stays, the others move one place a round
@@ -528,27 +582,7 @@ __global__ void k_ritz(double* s, int kdim, double tau, int expo) {
       __syncwarp();
     }
   }
-  int o = 0;
-  for (int k = 1; k < m; ++k)
-    if (A[k + k * m] < A[o + o * m]) o = k;   // lowest; ties keep the lower index
-  if (lane == 0) s[lz::EN] = A[o + o * m];
-  if (!expo) {
-    for (int k = lane; k < kdim; k += 32) s[lz::COEF + k] = (k < m) ? V[k + o * m] : 0.0;
-    return;
-  }
-  // c_k = sum_j V[k,j] exp(tau lambda_j) V[0,j]; every lane forms the sum of all c_k itself (the
-  // same fixed order in each lane) for the zero test
-  double tot = 0.0, mine = 0.0;
-  for (int k = 0; k < m; ++k) {
-    double ck = 0.0;
-    for (int jj = 0; jj < m; ++jj) ck += V[k + jj * m] * exp(tau * A[jj + jj * m]) * V[jj * m];
-    tot += ck;
-    if (k == lane) mine = ck;
-  }
-  if (tot == 0.0) {   // (I + T) e_1
-    mine = lane == 0 ? 1.0 + s[lz::ALPHA] : (lane == 1 && m > 1 ? s[lz::BETA] : 0.0);
-  }
-  for (int k = lane; k < kdim; k += 32) s[lz::COEF + k] = (k < m) ? mine : 0.0;
+  ritz_result(s, A, V, m, kdim, tau, expo);
 }
 
 // y = sum_j c[j] * X_j (y not read), j < k, c in device memory
@@ -677,8 +711,8 @@ void launch_next_vector(cudaStream_t s, const double* H, double* Kn, int64_t n, 
   count_launch();
 }
 
-void launch_ritz(cudaStream_t s, double* scal, int kdim, double tau, bool expo) {
-  launch_k(k_ritz, 1, 32, 0, s, scal, kdim, tau, expo ? 1 : 0);
+void launch_ritz(cudaStream_t s, double* scal, int kdim, double tau, bool expo, bool cyclic) {
+  launch_k(cyclic || kdim <= 2 ? k_ritz_cyclic : k_ritz, 1, 32, 0, s, scal, kdim, tau, expo ? 1 : 0);
   count_launch();
 }
 

@@ -337,11 +337,15 @@ DMRG_API int dmrg_test_gemm(dmrg_ctx* ctx, int transA, int transB, int M, int N,
  * (columns) overwrite A. */
 DMRG_API int dmrg_test_eigh(dmrg_ctx* ctx, int nmat, const int* n, double* A, double* w);
 
-/* Tridiagonal-path eigensolver (n[i] <= 2048; blocks above 112 take the mid-size kernels): all
- * eigenvalues (descending, packed in w) and the
+/* Tridiagonal-path eigensolver of the FP64 solves (n[i] <= 2048; all blocks take the clusters once
+ * the largest has more than 40 states): all eigenvalues (descending, packed in w) and the
  * eigenvectors of the k[i] largest (packed n[i] x k[i] column-major in U). A is overwritten. */
 DMRG_API int dmrg_test_syevt(dmrg_ctx* ctx, int nmat, const int* n, const int* k, double* A,
                              double* w, double* U);
+/* The same by the kernels of the solves whose sums keep one order (split-precision solves, and
+ * sweeps of more than four Krylov vectors on long chains; n[i] <= 512, one CTA per block). */
+DMRG_API int dmrg_test_syevt_fixed(dmrg_ctx* ctx, int nmat, const int* n, const int* k, double* A,
+                                   double* w, double* U);
 
 /* Device time of the two-site Heff at (iL, iL+1) in the given precision: `reps` applications to
  * a device-resident vector timed with CUDA events on the context's stream (no host copies).
