@@ -1075,8 +1075,10 @@ int dmrg_tdvp(dmrg_state* st, const dmrg_mpo* mpo, const dmrg_params* p, double 
   });
 }
 
-static void test_syevt(dmrg_ctx* c, bool fixed, int nmat, const int* n, const int* k, double* A,
+enum class Trid { solve, fixed, dirty };
+static void test_syevt(dmrg_ctx* c, Trid how, int nmat, const int* n, const int* k, double* A,
                        double* w, double* U) {
+  const bool fixed = how == Trid::fixed;
   if (nmat <= 0 || !n || !k || !A || !w || !U) fail(DMRG_ERR_ARG, "bad syevt arguments");
   set_device(c);
   int64_t ta = 0, tw = 0, tu = 0;
@@ -1113,8 +1115,28 @@ static void test_syevt(dmrg_ctx* c, bool fixed, int nmat, const int* n, const in
   TridValues tv;
   Upload u;
   put_trid_values(u, tasks, tv);
-  run_trid_values(c, buf.p, buf.n, tv, u.send(c, 8));
-  if (mk > 0) run_trid_vectors(c, buf.p, buf.n, tasks, 6);
+  char* db = u.send(c, 8);
+  if (how == Trid::dirty) launch_dirty_smem(c->stream);
+  run_trid_values(c, buf.p, buf.n, tv, db);
+  if (mk > 0 && how == Trid::dirty && mn > SYEVT_ROUTE) {
+    int64_t xw = 0;
+    for (TridTask& t : tasks) {
+      t.x_off = xw;
+      xw += syevt_mid_workspace(t.n, t.keep);
+    }
+    ensure(c, c->W, xw);
+    Upload v;
+    v.put(tasks);
+    const TridTask* dt = reinterpret_cast<const TridTask*>(v.send(c, 6));
+    launch_dirty_smem(c->stream);
+    launch_trid_mid_inner(c->stream, buf.p, dt, nmat, mn, mk, c->W.p);
+    launch_dirty_smem(c->stream);
+    launch_trid_mid_back(c->stream, buf.p, dt, nmat, mn, mk, c->W.p);
+    cuda_check(cudaGetLastError(), "tridiagonal eigenvectors");
+  } else if (mk > 0) {
+    if (how == Trid::dirty) launch_dirty_smem(c->stream);
+    run_trid_vectors(c, buf.p, buf.n, tasks, 6);
+  }
   cuda_check(cudaMemcpyAsync(w, buf.p + ta, tw * 8, cudaMemcpyDeviceToHost, c->stream), "w");
   cuda_check(cudaMemcpyAsync(U, buf.p + ta + 4 * tw, tu * 8, cudaMemcpyDeviceToHost, c->stream), "U");
   cuda_check(cudaStreamSynchronize(c->stream), "syevt sync");
@@ -1124,13 +1146,19 @@ static void test_syevt(dmrg_ctx* c, bool fixed, int nmat, const int* n, const in
 int dmrg_test_syevt(dmrg_ctx* c, int nmat, const int* n, const int* k, double* A, double* w,
                     double* U) {
   if (!c) return DMRG_ERR_ARG;
-  return guarded(c, [&] { test_syevt(c, false, nmat, n, k, A, w, U); });
+  return guarded(c, [&] { test_syevt(c, Trid::solve, nmat, n, k, A, w, U); });
 }
 
 int dmrg_test_syevt_fixed(dmrg_ctx* c, int nmat, const int* n, const int* k, double* A, double* w,
                           double* U) {
   if (!c) return DMRG_ERR_ARG;
-  return guarded(c, [&] { test_syevt(c, true, nmat, n, k, A, w, U); });
+  return guarded(c, [&] { test_syevt(c, Trid::fixed, nmat, n, k, A, w, U); });
+}
+
+int dmrg_test_syevt_dirty(dmrg_ctx* c, int nmat, const int* n, const int* k, double* A, double* w,
+                          double* U) {
+  if (!c) return DMRG_ERR_ARG;
+  return guarded(c, [&] { test_syevt(c, Trid::dirty, nmat, n, k, A, w, U); });
 }
 
 }  // extern "C"

@@ -122,9 +122,14 @@ int64_t syevt_mid_workspace(int n, int k);
 bool trid_gave_up(double w);
 void launch_trid_cluster(cudaStream_t s, double* base, const TridTask* tasks, int ntasks,
                          int max_n, int64_t sum_n);
-// xws: workspace base of the tasks' x_off
+// xws: workspace base of the tasks' x_off. The vectors of the tridiagonal matrices into the
+// workspace (inner), then the eigenvectors of the blocks from them (back).
 void launch_trid_mid_vectors(cudaStream_t s, double* base, const TridTask* tasks, int ntasks,
                              int max_n, int max_k, double* xws);
+void launch_trid_mid_inner(cudaStream_t s, double* base, const TridTask* tasks, int ntasks,
+                           int max_n, int max_k, double* xws);
+void launch_trid_mid_back(cudaStream_t s, double* base, const TridTask* tasks, int ntasks,
+                          int max_n, int max_k, const double* xws);
 
 // Tiles of the FP64 GEMM: 32 x 32, or 32 x 16 for lists too short to give every SM three of them.
 constexpr int GEMM_BM = 32, GEMM_BN = 32, GEMM_BN_SMALL = 16;
@@ -213,6 +218,8 @@ void launch_msub(cudaStream_t s, const double* X, int64_t ldx, int k, const doub
                  double* y, int64_t n);
 void launch_scale(cudaStream_t s, double* x, int64_t n, double a);
 void launch_zero(cudaStream_t s, double* x, int64_t n);
+// Leaves NaN in the shared memory of every SM (tests: what a kernel reads must have been written).
+void launch_dirty_smem(cudaStream_t s);
 // Descriptor bytes [src, src + bytes) to the device address dst (16-byte aligned) as one launch
 // whose parameter block carries them; false (nothing launched) above UPLOAD_PARAM_MAX bytes.
 constexpr int UPLOAD_PARAM_MAX = 32704;

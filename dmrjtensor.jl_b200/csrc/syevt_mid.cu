@@ -551,6 +551,8 @@ k_mid_back(double* __restrict__ base, const TridTask* __restrict__ tasks,
         if (k >= 1)
           asm volatile("cp.async.ca.shared.global [%0], [%1], 8;"
                        :: "r"(da + 8 * LD), "l"(V + int64_t(k - 1) * n + i));
+        else
+          st[LD + i] = 0.0;                      // no partner: tb = 0 alone would let a NaN through
       }
     }
     asm volatile("cp.async.commit_group;");
@@ -637,6 +639,12 @@ int64_t syevt_mid_workspace(int n, int k) { return mid_vec_workspace(n, k); }
 
 void launch_trid_mid_vectors(cudaStream_t s, double* base, const TridTask* tasks, int ntasks,
                              int max_n, int max_k, double* xws) {
+  launch_trid_mid_inner(s, base, tasks, ntasks, max_n, max_k, xws);
+  launch_trid_mid_back(s, base, tasks, ntasks, max_n, max_k, xws);
+}
+
+void launch_trid_mid_inner(cudaStream_t s, double* base, const TridTask* tasks, int ntasks,
+                           int max_n, int max_k, double* xws) {
   if (ntasks <= 0) return;
   int lanes = 8;                           // 152 KB at n = 512
   while (lanes > 1 && invit_smem(max_n, lanes) > MID_SMEM_LIMIT) lanes /= 2;
@@ -658,6 +666,12 @@ void launch_trid_mid_vectors(cudaStream_t s, double* base, const TridTask* tasks
   const size_t sm = std::max(mid_vec_smem_k(std::min(max_k, kg), true), mid_vec_smem_k(max_k, false));
   raise_smem_limit(reinterpret_cast<const void*>(k_mid_cholqr), sm);
   launch_k(k_mid_cholqr, ntasks, MT, sm, s, base, tasks, xws, kg);
+  count_launch(9);
+}
+
+void launch_trid_mid_back(cudaStream_t s, double* base, const TridTask* tasks, int ntasks,
+                          int max_n, int max_k, const double* xws) {
+  if (ntasks <= 0) return;
   auto back = [&](auto launch) { launch(s, base, tasks, ntasks, max_n, max_k, xws); };
   if (max_n <= 128) back(launch_back<4, 2>);
   else if (max_n <= 160) back(launch_back<5, 2>);
@@ -666,7 +680,7 @@ void launch_trid_mid_vectors(cudaStream_t s, double* base, const TridTask* tasks
   else if (max_n <= 512) back(launch_back<16, 2>);
   else if (max_n <= 1024) back(launch_back<32, 2>);
   else back(launch_back<64, 1>);
-  count_launch(10);
+  count_launch();
 }
 
 }  // namespace dmrg

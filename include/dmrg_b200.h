@@ -346,6 +346,9 @@ DMRG_API int dmrg_test_syevt(dmrg_ctx* ctx, int nmat, const int* n, const int* k
  * sweeps of more than four Krylov vectors on long chains; n[i] <= 512, one CTA per block). */
 DMRG_API int dmrg_test_syevt_fixed(dmrg_ctx* ctx, int nmat, const int* n, const int* k, double* A,
                                    double* w, double* U);
+/* dmrg_test_syevt with NaN left in the shared memory of every SM before each stage. */
+DMRG_API int dmrg_test_syevt_dirty(dmrg_ctx* ctx, int nmat, const int* n, const int* k, double* A,
+                                   double* w, double* U);
 
 /* Device time of the two-site Heff at (iL, iL+1) in the given precision: `reps` applications to
  * a device-resident vector timed with CUDA events on the context's stream (no host copies).
