@@ -232,6 +232,10 @@ double krylov_energy(dmrg_ctx* c, const KrylovRun& kr) {
   double e = c->h_scal[lz::EN];
   if (kr.fp64_energy && c->h_scal[lz::KK] > 0) e = c->h_scal[lz::KH] / c->h_scal[lz::KK];
   if (kr.split) check_mma_flag(c);
+  // every element of the vector enters it, so a NaN anywhere in the state shows here
+  if (!std::isfinite(e))
+    fail(DMRG_ERR_STATE, "bond step: the energy is not finite (a NaN or an infinity in the state, "
+                         "the operator or the environments)");
   return e;
 }
 
@@ -337,6 +341,8 @@ std::vector<std::vector<double>> rho_values(dmrg_ctx* c, const std::vector<Group
     vals[g].assign(c->h_lam + G[g].woff, c->h_lam + G[g].woff + side);
     if (side > 0 && trid_gave_up(vals[g][0]))
       fail(DMRG_ERR_TIMEOUT, "density-matrix eigensolver: a wait inside a cluster gave up");
+    for (double v : vals[g])
+      if (!std::isfinite(v)) fail(DMRG_ERR_STATE, "bond step: a density-matrix weight is not finite");
   }
   return vals;
 }

@@ -527,6 +527,7 @@ k_trid_sturm(double* __restrict__ base, const TridTask* __restrict__ tasks) {
     return;
   }
   double lo = 1e300, hi = -1e300;          // Gershgorin interval
+  bool fin = true;
   for (int i = tid; i < n; i += CT) {
     const double di = ws[i], ei = i + 1 < n ? ws[n + i] : 0.0, ep = i > 0 ? ws[n + i - 1] : 0.0;
     d[i] = di;
@@ -534,6 +535,7 @@ k_trid_sturm(double* __restrict__ base, const TridTask* __restrict__ tasks) {
     const double r = fabs(ei) + fabs(ep);
     lo = fmin(lo, di - r);
     hi = fmax(hi, di + r);
+    fin &= isfinite(di) && isfinite(ei);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -541,7 +543,11 @@ k_trid_sturm(double* __restrict__ base, const TridTask* __restrict__ tasks) {
     hi = fmax(hi, __shfl_xor_sync(FULL, hi, o));
   }
   if (lane == 0) { s_lo[warp] = lo; s_hi[warp] = hi; }
-  __syncthreads();
+  if (!__syncthreads_and(fin)) {           // no eigenvalue of a NaN or an infinity is a number
+    const int ei = int(blockIdx.x) * (CT / P) + tid / P;
+    if (tid % P == 0 && ei < n) base[tk.w_off + ei] = __longlong_as_double(0x7ff8000000000000LL);
+    return;
+  }
 #pragma unroll
   for (int q = 0; q < CWARPS; ++q) {
     lo = fmin(lo, s_lo[q]);

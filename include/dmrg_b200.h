@@ -54,7 +54,8 @@ enum dmrg_status {
   DMRG_ERR_BUDGET = 5,   /* request exceeds the context's HBM budget */
   DMRG_ERR_TIMEOUT = 6,  /* a bounded device wait gave up */
   DMRG_ERR_CUDA = 7,     /* CUDA runtime error */
-  DMRG_ERR_STATE = 8,    /* object not in a usable state (e.g. environments not built) */
+  DMRG_ERR_STATE = 8,    /* object not in a usable state (e.g. environments not built, or a NaN or an
+                            infinity in the state or operator of a solve) */
   DMRG_ERR_NOCUDA = 9    /* no CUDA device */
 };
 
