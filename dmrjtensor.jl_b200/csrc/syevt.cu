@@ -84,7 +84,7 @@ k_trid_eigvals(double* __restrict__ base, const TridTask* __restrict__ tasks) {
   double* e = d + n;            // n
   double* e2 = e + n;           // n
   double* tau = e2 + n;         // n
-  __shared__ double s_lo, s_hi;
+  __shared__ double s_lo, s_hi, s_scale, s_back;
   __shared__ double kw[TE_THREADS / 32];   // per-warp shares of K
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
   double* Ag = base + tk.a_off;
@@ -232,7 +232,6 @@ k_trid_eigvals(double* __restrict__ base, const TridTask* __restrict__ tasks) {
     tau[n - 1] = 0.0;
   }
   __syncthreads();
-  for (int i = tid; i < n; i += blockDim.x) e2[i] = e[i] * e[i];
   for (int x = tid; x < n * n; x += blockDim.x) Ag[x] = A[x];
   double* ws = base + tk.ws_off;          // d | e | tau
   for (int i = tid; i < n; i += blockDim.x) {
@@ -253,10 +252,19 @@ k_trid_eigvals(double* __restrict__ base, const TridTask* __restrict__ tasks) {
       hi = fmax(hi, __shfl_xor_sync(FULL, hi, o));
     }
     if (lane == 0) {
+      s_scale = unit_scale(fmax(fabs(lo), fabs(hi)), s_back);
+      lo *= s_scale;
+      hi *= s_scale;
       const double pad = 2.2e-16 * fmax(fabs(lo), fabs(hi)) + 1e-300;
       s_lo = lo - pad;
       s_hi = hi + pad;
     }
+  }
+  __syncthreads();
+  for (int i = tid; i < n; i += blockDim.x) {   // the counts run on T with a norm in [1, 2)
+    const double ei = e[i] * s_scale;
+    d[i] *= s_scale;
+    e2[i] = ei * ei;
   }
   __syncthreads();
   // multisection: a group of P lanes per eigenvalue (P = 2, 3, 4 or 8 as n allows with 256
@@ -297,7 +305,7 @@ k_trid_eigvals(double* __restrict__ base, const TridTask* __restrict__ tasks) {
       }
     }
   }
-  if (h == 0 && ei < n) base[tk.w_off + ei] = 0.5 * (a + b);
+  if (h == 0 && ei < n) base[tk.w_off + ei] = 0.5 * (a + b) * s_back;
 }
 
 // Shared-memory layout of k_trid_vectors (doubles first, then ints).

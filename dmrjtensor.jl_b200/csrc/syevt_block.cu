@@ -85,7 +85,7 @@ k_trid_block_vals(double* __restrict__ base, const TridTask* __restrict__ tasks,
   double* tau = e2 + n;                    // n
   double* S = tau + n;                     // packed trailing block, mp (mp + 1) / 2
   __shared__ double kw[NW];
-  __shared__ double s_lo, s_hi;
+  __shared__ double s_lo, s_hi, s_scale, s_back;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   double* Ag = base + tk.a_off;
   double* B = Ag + n + 1;                  // trailing block of step 0, A[1:, 1:]
@@ -377,7 +377,6 @@ k_trid_block_vals(double* __restrict__ base, const TridTask* __restrict__ tasks,
     }
   }
   __syncthreads();
-  for (int i = tid; i < n; i += MT) e2[i] = e[i] * e[i];
   double* ws = base + tk.ws_off;          // d | e | tau
   for (int i = tid; i < n; i += MT) {
     ws[i] = d[i];
@@ -397,10 +396,19 @@ k_trid_block_vals(double* __restrict__ base, const TridTask* __restrict__ tasks,
       hi = fmax(hi, __shfl_xor_sync(FULL, hi, o));
     }
     if (lane == 0) {
+      s_scale = unit_scale(fmax(fabs(lo), fabs(hi)), s_back);
+      lo *= s_scale;
+      hi *= s_scale;
       const double pad = 2.2e-16 * fmax(fabs(lo), fabs(hi)) + 1e-300;
       s_lo = lo - pad;
       s_hi = hi + pad;
     }
+  }
+  __syncthreads();
+  for (int i = tid; i < n; i += MT) {   // the counts run on T with a norm in [1, 2)
+    const double ei = e[i] * s_scale;
+    d[i] *= s_scale;
+    e2[i] = ei * ei;
   }
   __syncthreads();
   // trisection, MT/2 eigenvalues per round: threads 2i, 2i+1 count at the interval's two
@@ -431,7 +439,7 @@ k_trid_block_vals(double* __restrict__ base, const TridTask* __restrict__ tasks,
         else a = x1;
       }
     }
-    if (h == 0 && ei < n) base[tk.w_off + ei] = 0.5 * (a + b);
+    if (h == 0 && ei < n) base[tk.w_off + ei] = 0.5 * (a + b) * s_back;
   }
 }
 

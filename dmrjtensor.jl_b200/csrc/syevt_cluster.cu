@@ -531,7 +531,7 @@ k_trid_sturm(double* __restrict__ base, const TridTask* __restrict__ tasks) {
   for (int i = tid; i < n; i += CT) {
     const double di = ws[i], ei = i + 1 < n ? ws[n + i] : 0.0, ep = i > 0 ? ws[n + i - 1] : 0.0;
     d[i] = di;
-    e2[i] = ei * ei;
+    e2[i] = ei;
     const double r = fabs(ei) + fabs(ep);
     lo = fmin(lo, di - r);
     hi = fmax(hi, di + r);
@@ -553,6 +553,16 @@ k_trid_sturm(double* __restrict__ base, const TridTask* __restrict__ tasks) {
     lo = fmin(lo, s_lo[q]);
     hi = fmax(hi, s_hi[q]);
   }
+  double back;                             // the counts run on T with a norm in [1, 2)
+  const double scale = unit_scale(fmax(fabs(lo), fabs(hi)), back);
+  lo *= scale;
+  hi *= scale;
+  for (int i = tid; i < n; i += CT) {
+    const double ei = e2[i] * scale;
+    d[i] *= scale;
+    e2[i] = ei * ei;
+  }
+  __syncthreads();
   const double pad = 2.2e-16 * fmax(fabs(lo), fabs(hi)) + 1e-300;
   lo -= pad;
   hi += pad;
@@ -584,7 +594,7 @@ k_trid_sturm(double* __restrict__ base, const TridTask* __restrict__ tasks) {
       }
     }
   }
-  if (h == 0 && ei < n) base[tk.w_off + ei] = 0.5 * (a + b);
+  if (h == 0 && ei < n) base[tk.w_off + ei] = 0.5 * (a + b) * back;
 }
 
 }  // namespace

@@ -16,6 +16,13 @@ __device__ __forceinline__ double wsum(double v) {
   return v;
 }
 
+// The power of two that brings a norm into [1, 2) (exact to multiply by), and its inverse.
+__device__ __forceinline__ double unit_scale(double norm, double& back) {
+  const int f = min((__double2hiint(norm) >> 20) & 0x7ff, 2045);   // 0: zero and subnormal numbers
+  back = __hiloint2double(max(f, 1) << 20, 0);
+  return __hiloint2double((2046 - max(f, 1)) << 20, 0);
+}
+
 // Scales a pair by the power of two that brings the larger magnitude into [1, 2): exact, keeps
 // the signs, and needs only exponent-field arithmetic.
 __device__ __forceinline__ void rescale_pair(double& D, double& Dm1) {
@@ -34,7 +41,7 @@ __device__ __forceinline__ void rescale_pair(double& D, double& Dm1) {
 // t_j = -e_{j-1}^2 D_{j-2}: each step is one FMA for D_j and one product t_{j+1} from D_{j-1}, two
 // independent operations, so only the FMA is on the dependent chain. Groups of 8 steps load
 // first, count signs after the group (an exact zero minor counts with the sign opposite to its
-// predecessor), then rescale the pair by a power of two.
+// predecessor), then rescale the pair by a power of two; T has to come with a norm near 1 (unit_scale).
 __device__ int sturm_below(const double* __restrict__ d, const double* __restrict__ e2, int n,
                            double x) {
   double D = d[0] - x;

@@ -14,9 +14,10 @@ namespace {
 // independent operations, so only the FMA is on the dependent chain. Signs are counted on the high
 // words (an isolated exact zero gives the same count with either sign). After every 8 steps the
 // pair is rescaled by the power of two that brought its larger magnitude after the fourth of them
-// into [1, 2): the factor is ready before the chain needs it, and 12 steps stay far from
-// overflow and underflow. With the small blocks' kernel (85, 70 and 40 rows in one launch) the
-// lagged rescaling and the bit counts took 108 to 100 us.
+// into [1, 2): the factor is ready before the chain needs it. The pair goes 12 steps without a
+// rescaling, each of which may multiply it by the norm of T, so T has to come with a norm near 1
+// (unit_scale): at 1e-26 the pair would underflow and never recover. With blocks of 85, 70 and 40
+// rows in one launch the lagged rescaling and the bit counts took 108 to 100 us.
 __device__ int sturm_lagged(const double* __restrict__ d, const double* __restrict__ e2, int n,
                            double x) {
   double D = d[0] - x;

@@ -374,19 +374,25 @@ __device__ bool lowest_pair(double* s, int kdim) {
   const bool on = lane + 1 < kdim && s[lz::BETA + lane] > 0.0;
   const int m = 1 + __ffs(~__ballot_sync(FULL, on)) - 1;
   if (m <= 2) return false;
-  const double al = lane < m ? s[lz::ALPHA + lane] : 0.0;
-  const double be = lane + 1 < m ? s[lz::BETA + lane] : 0.0;
+  double al = lane < m ? s[lz::ALPHA + lane] : 0.0;
+  double be = lane + 1 < m ? s[lz::BETA + lane] : 0.0;
   const double r = be + __shfl_up_sync(FULL, be, 1) * (lane > 0);
   double lo = lane < m ? al - r : 1e300, hi = lane < m ? al + r : -1e300;
-  if (lane < m) {
-    d[lane] = al;
-    e[lane] = be;
-    e2[lane] = be * be;
-  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     lo = fmin(lo, __shfl_xor_sync(FULL, lo, o));
     hi = fmax(hi, __shfl_xor_sync(FULL, hi, o));
+  }
+  double back;                             // everything on T with a norm in [1, 2)
+  const double scale = unit_scale(fmax(fabs(lo), fabs(hi)), back);
+  al *= scale;
+  be *= scale;
+  lo *= scale;
+  hi *= scale;
+  if (lane < m) {
+    d[lane] = al;
+    e[lane] = be;
+    e2[lane] = be * be;
   }
   __syncwarp();
   const double tn = fmax(fmax(fabs(lo), fabs(hi)), 1e-300);
@@ -406,7 +412,7 @@ __device__ bool lowest_pair(double* s, int kdim) {
   const double sg = z[0] < 0.0 ? -1.0 : 1.0;
   const double zi = lane < m ? sg * z[lane] : 0.0, zn = lane + 1 < m ? sg * z[lane + 1] : 0.0;
   const double en = wsum(al * zi * zi + 2.0 * be * zi * zn);
-  if (lane == 0) s[lz::EN] = en;
+  if (lane == 0) s[lz::EN] = en * back;
   if (lane < kdim) s[lz::COEF + lane] = zi;
   return true;
 }
