@@ -135,6 +135,8 @@ SIGNATURES = {
     "dmrg_test_gemm": (C.c_int, [_P, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, _DP, C.c_int,
                                  _DP, C.c_int, _DP, C.c_int]),
     "dmrg_test_eigh": (C.c_int, [_P, C.c_int, _IP, _DP, _DP]),
+    "dmrg_test_krylov": (C.c_int, [_P, C.c_int, C.c_int, C.c_int64, C.c_int, C.c_double, _DP, _DP,
+                                   _DP]),
     "dmrg_test_syevt": (C.c_int, [_P, C.c_int, _IP, _IP, _DP, _DP, _DP]),
     "dmrg_test_syevt_fixed": (C.c_int, [_P, C.c_int, _IP, _IP, _DP, _DP, _DP]),
     "dmrg_test_syevt_dirty": (C.c_int, [_P, C.c_int, _IP, _IP, _DP, _DP, _DP]),

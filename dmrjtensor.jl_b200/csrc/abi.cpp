@@ -8,7 +8,7 @@
 #include <map>
 #include <numeric>
 
-#include "engine.hpp"
+#include "engine_step.hpp"
 
 using namespace dmrg;
 
@@ -1164,6 +1164,33 @@ int dmrg_test_syevt_dirty(dmrg_ctx* c, int nmat, const int* n, const int* k, dou
 }  // extern "C"
 
 extern "C" {
+
+int dmrg_test_krylov(dmrg_ctx* c, int general, int mode, int64_t n, int j, double betatest,
+                     double* K, double* H, double* scal) {
+  if (!c) return DMRG_ERR_ARG;
+  return guarded(c, [&] {
+    if (n <= 0 || j < 0 || mode < KRY_NORMALISE || mode > KRY_LAST2 || !K || !H || !scal ||
+        j > (mode == KRY_NORMALISE ? lz::NRM : mode == KRY_STEP ? 14 : 15) ||
+        (mode == KRY_LAST2 && j != 1) || (mode == KRY_FIRST && j != 0))
+      fail(DMRG_ERR_ARG, "bad Krylov arguments");
+    set_device(c);
+    const int64_t nk = n * (mode == KRY_NORMALISE ? 1 : j + 2);
+    ensure(c, c->K, nk);
+    ensure(c, c->H, n);
+    auto copy = [&](void* to, const void* from, int64_t m, cudaMemcpyKind kind) {
+      cuda_check(cudaMemcpyAsync(to, from, size_t(m) * 8, kind, c->stream), "Krylov test copy");
+    };
+    copy(c->K.p, K, nk, cudaMemcpyHostToDevice);
+    copy(c->H.p, H, n, cudaMemcpyHostToDevice);
+    copy(c->d_scal, scal, 256, cudaMemcpyHostToDevice);
+    krylov_vectors(c, mode, c->K.p, c->H.p, n, j, betatest, general != 0);
+    cuda_check(cudaGetLastError(), "Krylov vectors");
+    copy(K, c->K.p, nk, cudaMemcpyDeviceToHost);
+    copy(H, c->H.p, n, cudaMemcpyDeviceToHost);
+    copy(scal, c->d_scal, 256, cudaMemcpyDeviceToHost);
+    cuda_check(cudaStreamSynchronize(c->stream), "Krylov test");
+  });
+}
 
 int dmrg_test_gemm(dmrg_ctx* c, int transA, int transB, int M, int N, int K, const double* A,
                    int lda, const double* B, int ldb, double* C, int ldc) {

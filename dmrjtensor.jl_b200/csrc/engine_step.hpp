@@ -105,6 +105,12 @@ struct Group {
   int64_t moff = 0, roff = 0, woff = 0;
 };
 
+// The vector work `mode` (KRY_*) of a Krylov step: one launch for vectors of up to KRY_MAX elements,
+// the general launches above (general: at any size, the same numbers bit for bit). KRY_NORMALISE:
+// j is the scalar slot.
+void krylov_vectors(dmrg_ctx* c, int mode, double* K, double* H, int64_t n, int j,
+                    double betatest, bool general = false);
+
 // x /= |x| (n elements on the device), with <x,x> left in the scalar slot.
 void normalise_vec(dmrg_ctx* c, double* x, int64_t n, int slot);
 

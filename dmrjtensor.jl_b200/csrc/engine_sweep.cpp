@@ -74,10 +74,44 @@ void Timing::flush() {
   used = 0;
 }
 
+void krylov_vectors(dmrg_ctx* c, int mode, double* K, double* H, int64_t n, int j,
+                    double betatest, bool general) {
+  cudaStream_t s = c->stream;
+  double* scal = c->d_scal;
+  if (!general && launch_krylov(s, mode, K, H, n, scal, j, betatest)) return;
+  double* Kj = K + (mode == KRY_NORMALISE ? 0 : j) * n;
+  switch (mode) {
+    case KRY_NORMALISE:
+      launch_mdot(s, K, 0, 1, K, n, c->d_partial, scal + j);
+      launch_scale_rsqrt(s, K, n, scal + j);
+      return;
+    case KRY_FIRST:
+      launch_dot2(s, K, H, n, c->d_partial, scal + lz::KK);
+      launch_lanczos2_orth(s, K, H, n, scal, c->d_partial);   // K /= |K|, H -= a1 K, |H|^2
+      launch_next_vector(s, H, K + n, n, scal, 0, betatest);
+      return;
+    case KRY_LAST2:
+      launch_mdot(s, Kj, 0, 1, H, n, c->d_partial, scal + lz::ALPHA + 1);
+      launch_ritz(s, scal, 2, 0.0, false, true);
+      launch_lincomb(s, K, n, 2, scal + lz::COEF, H, n);
+      return;
+    default:
+      launch_mdot(s, Kj, 0, 1, H, n, c->d_partial, scal + lz::ALPHA + j);
+      if (mode == KRY_ALPHA) return;
+      launch_axpby(s, n, 0.0, scal + lz::ALPHA + j, -1.0, Kj, 1.0, nullptr, 0, H, 0);
+      if (j > 0)
+        launch_axpby(s, n, 0.0, scal + lz::BETA + j - 1, -1.0, Kj - n, 1.0, nullptr, 0, H, 0);
+      for (int pass = 0; pass < 2; ++pass) {   // full re-orthogonalisation (CGS2)
+        launch_mdot(s, K, n, j + 1, H, n, c->d_partial, scal + lz::CGS);
+        launch_msub(s, K, n, j + 1, scal + lz::CGS, H, n);
+      }
+      launch_mdot(s, H, 0, 1, H, n, c->d_partial, scal + lz::B2 + j);
+      launch_next_vector(s, H, Kj + n, n, scal, j, betatest);
+  }
+}
+
 void normalise_vec(dmrg_ctx* c, double* x, int64_t n, int slot) {
-  if (launch_krylov(c->stream, KRY_NORMALISE, x, nullptr, n, c->d_scal, slot, 0.0)) return;
-  launch_mdot(c->stream, x, 0, 1, x, n, c->d_partial, c->d_scal + slot);
-  launch_scale_rsqrt(c->stream, x, n, c->d_scal + slot);
+  krylov_vectors(c, KRY_NORMALISE, x, nullptr, n, slot, 0.0);
 }
 
 // Krylov solve: see engine_step.hpp. P.graph: everything of the solve after its first Heff
@@ -121,46 +155,21 @@ KrylovRun krylov_solve(dmrg_state* st, const dmrg_params& P, const HeffPlan& hp,
     // simplelanczos (algs/DMRG.jl:57-90): H is applied to AA before its normalisation
     heff(K, H);
     tv = tm.begin();
-    double* K1 = K + n;
-    if (!launch_krylov(s, KRY_FIRST, K, H, n, scal, 0, P.betatest)) {
-      launch_dot2(s, K, H, n, c->d_partial, scal + lz::KK);
-      launch_lanczos2_orth(s, K, H, n, scal, c->d_partial);   // K /= |K|, H -= a1 K, |H|^2
-      launch_next_vector(s, H, K1, n, scal, 0, P.betatest);
-    }
+    krylov_vectors(c, KRY_FIRST, K, H, n, 0, P.betatest);
     cuda_check(cudaGetLastError(), "Krylov vector");
     tm.end(tv, 3);
-    heff(K1, H);
+    heff(K + n, H);
     tv = tm.begin();
-    if (!launch_krylov(s, KRY_LAST2, K, H, n, scal, 1, P.betatest)) {
-      launch_mdot(s, K1, 0, 1, H, n, c->d_partial, scal + lz::ALPHA + 1);
-      launch_ritz(s, scal, 2, 0.0, false, true);
-      launch_lincomb(s, K, n, 2, scal + lz::COEF, H, n);
-    }
+    krylov_vectors(c, KRY_LAST2, K, H, n, 1, P.betatest);
     tm.end(tv, 3);
   } else {
     tv = tm.begin();
     normalise_vec(c, K, n, lz::KK);
     tm.end(tv, 3);
     for (int jj = 0; jj < kdim; ++jj) {
-      double* Kj = K + int64_t(jj) * n;
-      heff(Kj, H);
+      heff(K + int64_t(jj) * n, H);
       tv = tm.begin();
-      const bool last = jj == kdim - 1;
-      if (launch_krylov(s, last ? KRY_ALPHA : KRY_STEP, K, H, n, scal, jj, P.betatest)) {
-        tm.end(tv, 3);
-        continue;
-      }
-      launch_mdot(s, Kj, 0, 1, H, n, c->d_partial, scal + lz::ALPHA + jj);
-      if (last) { tm.end(tv, 3); break; }
-      launch_axpby(s, n, 0.0, scal + lz::ALPHA + jj, -1.0, Kj, 1.0, nullptr, 0, H, 0);
-      if (jj > 0)
-        launch_axpby(s, n, 0.0, scal + lz::BETA + jj - 1, -1.0, Kj - n, 1.0, nullptr, 0, H, 0);
-      for (int pass = 0; pass < 2; ++pass) {   // full re-orthogonalisation (CGS2)
-        launch_mdot(s, K, n, jj + 1, H, n, c->d_partial, scal + lz::CGS);
-        launch_msub(s, K, n, jj + 1, scal + lz::CGS, H, n);
-      }
-      launch_mdot(s, H, 0, 1, H, n, c->d_partial, scal + lz::B2 + jj);
-      launch_next_vector(s, H, K + int64_t(jj + 1) * n, n, scal, jj, P.betatest);
+      krylov_vectors(c, jj == kdim - 1 ? KRY_ALPHA : KRY_STEP, K, H, n, jj, P.betatest);
       tm.end(tv, 3);
     }
     tv = tm.begin();

@@ -338,6 +338,12 @@ DMRG_API int dmrg_test_gemm(dmrg_ctx* ctx, int transA, int transB, int M, int N,
  * (columns) overwrite A. */
 DMRG_API int dmrg_test_eigh(dmrg_ctx* ctx, int nmat, const int* n, double* A, double* w);
 
+/* The vector work of a Krylov step on host data: mode = 0 normalise (j: scalar slot), 1 first half of
+ * the 2-vector step (j = 0), 2 Lanczos iteration j < 15, 3 alpha_j, 4 end of the 2-vector step
+ * (j = 1). general: by the general launches whatever n. K holds j + 2 vectors (mode 0: one) of n
+ * elements, scal the 256 scalars; all three are updated in place. */
+DMRG_API int dmrg_test_krylov(dmrg_ctx* ctx, int general, int mode, int64_t n, int j,
+                              double betatest, double* K, double* H, double* scal);
 /* Tridiagonal-path eigensolver of the FP64 solves (n[i] <= 2048; all blocks take the clusters once
  * the largest has more than 40 states): all eigenvalues (descending, packed in w) and the
  * eigenvectors of the k[i] largest (packed n[i] x k[i] column-major in U). A is overwritten. */
