@@ -796,6 +796,7 @@ int dmrg_env_step_order(dmrg_ctx* c, int left, int ml, int d, int mr, int wl, in
   return guarded(c, [&] {
     if (!env_in || !psi || !W || !env_out) fail(DMRG_ERR_ARG, "env step: null array");
     if (row_major & ~7) fail(DMRG_ERR_ARG, "env step: unknown order bits");
+    if (!dual) row_major = (row_major & 3) | (row_major & 2) << 1;   // psi itself, in its order
     set_device(c);
     env_step_dense(c, left != 0, ml, d, mr, wl, wr, env_in, dual ? dual : psi, psi, W, env_out,
                    row_major);

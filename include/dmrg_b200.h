@@ -217,7 +217,8 @@ DMRG_API int dmrg_env_step(dmrg_ctx* ctx, int left, int ml, int d, int mr, int w
                            const double* env_in, const double* dual, const double* psi,
                            const double* W, double* env_out);
 /* The same with operands that are row-major in memory: row_major is the sum of 1 (env_in),
- * 2 (psi) and 4 (dual); they are reordered on the device. W and env_out stay column-major. */
+ * 2 (psi) and 4 (dual; not looked at where dual is NULL, which stands for psi in psi's order); they
+ * are reordered on the device. W and env_out stay column-major. */
 DMRG_API int dmrg_env_step_order(dmrg_ctx* ctx, int left, int ml, int d, int mr, int wl, int wr,
                                  const double* env_in, const double* dual, const double* psi,
                                  const double* W, double* env_out, int row_major);
