@@ -105,9 +105,6 @@ __host__ __device__ __forceinline__ int trid_lead_steps(int n) {
   return n <= HN ? 0 : (n - HN + 31) / 32 * 32;
 }
 
-template <int N, int MASK>
-__device__ __forceinline__ double wsum_cols(const double (&s)[N], int lane);
-
 // The first trid_lead_steps(n) Householder steps of a block above HN rows: columns dealt cyclically
 // to the CTAs, four per warp and sweep; each sweep applies the previous step's rank-2 update,
 // stores, and multiplies by the new reflector (unscaled, as in k_trid_cluster). One cluster
