@@ -522,11 +522,11 @@ void measure_correlation(dmrg_state* st, int d, const double* Cc, const double* 
 //     2 vectors             1.4e-4 (of 1,093 sweeps three above 2e-5)
 //     4 and 8 vectors       1.3e-2 (of 158 sweeps thirteen above 2e-5)
 //   FP64:
-//     2 vectors             records 1.5e-11, correlations 2.5e-9 (62 sweeps)
-//     4 vectors             7.5e-12, 1.1e-8 (113)
+//     2 vectors             records 2.0e-11, correlations 5.6e-9 (462 sweeps)
+//     4 vectors             9.0e-11, 3.5e-8 (613)
 //     8, up to 24 sites     4.2e-10, 4.9e-8 (400)
 //     8, 25 to 100 sites    2.4e-5, 3.3e-3 (200, one in ten above 1e-9)
-//     TDVP, up to 8         3.3e-11, 2.0e-9 (51)
+//     TDVP, up to 8         6.1e-11, 7.3e-9 (351 calls)
 // The others take the clusters, which are faster from 40 states on: 0.6 against 4.6 ms for the values
 // of a block of 345 states; a half-filled Hubbard sweep of 32 sites and 400 states takes 65 ms with
 // them and 218 ms in this order.

@@ -266,7 +266,9 @@ void plan_rho(dmrg_ctx* c, std::vector<Group>& G, bool rows, const dmrg_params& 
   // The tridiagonal path knows a weight to ~n x 1e-17 of the largest, block Jacobi to the rounding
   // of its own row and column. Blocks above SYEVT_RESOLVE_NMAX therefore take the tridiagonal path
   // only where the cutoff keeps the cut far above that: with cutoff 0, where the sign of the last
-  // weights decides, a dense L = 20 sweep at m = 384 kept 252 states instead of 384.
+  // weights decides, a dense L = 20 sweep at m = 384 kept 252 states instead of 384. minm likewise
+  // keeps weights below the cutoff, down to that level; up to SYEVT_NMAX states it does not reach
+  // there as a rule, since a bond that has a block above SYEVT_RESOLVE_NMAX keeps more by its cutoff.
   const int trid_max = !fixed && P.cutoff >= 1e-11 && P.minm <= SYEVT_NMAX ? SYEVT_MID_NMAX
                                                                            : SYEVT_RESOLVE_NMAX;
   rs.etasks.clear();

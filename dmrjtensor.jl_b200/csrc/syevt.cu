@@ -1,7 +1,9 @@
-// syevt.cu -- density-matrix eigensolver for blocks up to SYEVT_NMAX: Householder
-// tridiagonalisation, multisection, inverse iteration, re-orthogonalisation, back-transformation.
-// One CTA per block; every phase is laid out for latency (few block barriers, no dependent
-// shared- or local-memory loads on the arithmetic chains), since the blocks are small.
+// syevt.cu -- density-matrix eigensolver for blocks up to SYEVT_NMAX, one CTA per block: for steps
+// without a block above SYEVT_ROUTE states, and for all such blocks of the solves whose sums keep one
+// order (fixed_order). Householder tridiagonalisation, multisection, inverse iteration,
+// re-orthogonalisation, back-transformation; every phase is laid out for latency (few block
+// barriers, no dependent shared- or local-memory loads on the arithmetic chains), since the blocks
+// are small.
 //
 // Launch 1 (k_trid_eigvals), matrix in shared memory:
 //   * A = Q T Q^T by n-2 Householder reflectors (lower form, LAPACK dsytd2 order). Per step two

@@ -1,7 +1,8 @@
-// syevt_common.cuh -- device helpers shared by the density-matrix eigensolvers (syevt.cu for
-// blocks up to SYEVT_NMAX, syevt_mid.cu for blocks up to SYEVT_MID_NMAX): warp and block sums,
-// the division-free Sturm count of the symmetric tridiagonal matrix, the reproducible start
-// vectors and the inverse iteration of one eigenvector.
+// syevt_common.cuh -- device helpers of the density-matrix eigensolvers: warp and block sums, the
+// division-free Sturm count of the symmetric tridiagonal matrix, the reproducible start vectors and
+// the inverse iteration of one eigenvector, in the forms of the one-CTA kernels (syevt.cu,
+// syevt_block.cu). The many-CTA kernels share the sums and start vectors; their own solvers are in
+// trid_solve.cuh.
 #pragma once
 #include "kernels.cuh"
 

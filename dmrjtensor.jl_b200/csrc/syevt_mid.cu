@@ -1,6 +1,7 @@
 // syevt_mid.cu -- eigenvectors of the density-matrix blocks of a step whose largest has more than
-// SYEVT_ROUTE (up to SYEVT_MID_NMAX) states (their tridiagonal matrices and eigenvalues come from syevt_cluster.cu). Every part runs on many
-// CTAs; one CTA per block for all of it took 1.6 + 0.54 ms at n = 345 with 200 kept vectors.
+// SYEVT_ROUTE (up to SYEVT_MID_NMAX) states (their tridiagonal matrices and eigenvalues come from
+// syevt_cluster.cu). Every part runs on many CTAs; one CTA per block for all of it took 1.6 + 0.54 ms
+// at n = 345 with 200 kept vectors.
 //   * k_mid_invit: inverse iteration, one thread per kept vector, a few vectors per CTA so that
 //     their LU factors and the vectors stay in shared memory (with 32 vectors per CTA and the
 //     factors in global memory 290 us at n = 345). Bound by the latency of the recurrences.
