@@ -466,10 +466,9 @@ __device__ __forceinline__ void ritz_result(double* s, const double* A, const do
   for (int k = lane; k < kdim; k += 32) s[lz::COEF + k] = (k < m) ? mine : 0.0;
 }
 
-// Ritz step of the Krylov solve, one warp: T = tridiag(alpha, beta) of the m active vectors
-// (ritz_matrix), cyclic Jacobi (serial rotation
-// order; lanes own the rows/columns of one rotation) until the off-diagonal is at the rounding
-// level of the diagonal, lowest eigenvalue -> s[EN], its eigenvector -> s[COEF + j] (0 for j >= m).
+// Ritz step of the Krylov solve, one warp: cyclic Jacobi on T (serial rotation order; lanes own the
+// rows/columns of one rotation) until the off-diagonal is at the rounding level of the diagonal, lowest
+// eigenvalue -> s[EN], its eigenvector -> s[COEF + j] (0 for j >= m).
 // For two vectors, where it is one rotation, and for fixed_order solves whatever kdim (m = 8: 81 us a
 // launch; k_ritz needs 6.6 or 35).
 __global__ void k_ritz_cyclic(double* s, int kdim, double tau, int expo) {
